@@ -25,7 +25,6 @@ __device__ __forceinline__ cplx cfma_conj(cplx a, cplx b, cplx c) {
 __device__ __forceinline__ cplx cfnma(cplx a, cplx b, cplx c) {
     return mk(fma(-a.x, b.x, fma(a.y, b.y, c.x)), fma(-a.x, b.y, fma(-a.y, b.x, c.y)));
 }
-__device__ __forceinline__ double norm2_acc(cplx v, double s) { return fma(v.x, v.x, fma(v.y, v.y, s)); }
 
 // Sum of part[0..np) in a fixed order, identical in every block; the result is valid in all threads.
 __device__ __forceinline__ cplx block_reduce_parts(const cplx* part, int np, cplx* sh) {
@@ -53,87 +52,228 @@ __device__ __forceinline__ void block_store_partial(cplx v, cplx* sh, cplx* out)
     if (threadIdx.x == 0) out[blockIdx.x] = sh[0];
 }
 
-// Δg = g - gold ; Δf = fx - fxold (in place in fxold) ; partial of <Qb, Δf> (or |Δf|² when Qb is null).
+// Storage of the vectors.  Without symmetry groups every vector has one value per state element.
+// With them, every iterate is a complex combination of class-symmetric vectors, so all members of a
+// class that carry the same conjugation hold the same value up to their sign: the vectors keep one
+// value per (class, conjugation) pair, the "keys" (key = 2·class + conj), and inner products weight a
+// key by its number of members.  That is the full-vector arithmetic, elementwise the same operations,
+// on 1/8 to 1/16 of the elements (Hubbard 8x8, nK3 = (8, 12): 1.87 M elements, 0.19 M keys).
+
+// code of a state element (class * 4 + op) -> its key and sign
+__device__ __forceinline__ uint32_t key_of(uint32_t code) { return ((code >> 2) << 1) | ((code >> 1) & 1u); }
+__device__ __forceinline__ cplx signed_(cplx v, uint32_t neg) {
+    return neg ? mk(neg_exact(v.x), neg_exact(v.y)) : v;
+}
+// first member and number of members of each key (src preset to 0xffffffff, w to 0)
+__global__ void __launch_bounds__(RT) k_aa_keys(const uint32_t* code, uint32_t* src, double* w, size_t n) {
+    for (size_t j = blockIdx.x * (size_t)RT + threadIdx.x; j < n; j += (size_t)gridDim.x * RT) {
+        const uint32_t k = key_of(code[j]);
+        atomicMin(&src[k], (uint32_t)j);
+        atomicAdd(&w[k], 1.0);
+    }
+}
+// number of elements of x that differ from their key's value (a NaN differs)
+__global__ void __launch_bounds__(RT) k_aa_check(const cplx* x, const uint32_t* code, const uint32_t* src,
+                                                 unsigned int* count, size_t n) {
+    unsigned int bad = 0;
+    for (size_t j = blockIdx.x * (size_t)RT + threadIdx.x; j < n; j += (size_t)gridDim.x * RT) {
+        const uint32_t c = code[j], s = src[key_of(c)];
+        const cplx a = signed_(x[j], c & 1u), b = signed_(x[s], code[s] & 1u);
+        if (!(a.x == b.x && a.y == b.y)) ++bad;
+    }
+    if (bad) atomicAdd(count, bad);
+}
+// value of key k of the full vector x (0 for a key without members)
+__device__ __forceinline__ cplx key_value(const cplx* x, const uint32_t* code, const uint32_t* src, size_t k) {
+    const uint32_t s = src[k];
+    return s == 0xffffffffu ? mk(0.0, 0.0) : signed_(x[s], code[s] & 1u);
+}
+__global__ void __launch_bounds__(RT) k_aa_gather(cplx* xr, const cplx* x, const uint32_t* code, const uint32_t* src,
+                                                  size_t nr) {
+    for (size_t k = blockIdx.x * (size_t)RT + threadIdx.x; k < nr; k += (size_t)gridDim.x * RT)
+        xr[k] = key_value(x, code, src, k);
+}
+__global__ void __launch_bounds__(RT) k_aa_expand(cplx* x, const cplx* xr, const uint32_t* code, size_t n) {
+    for (size_t j = blockIdx.x * (size_t)RT + threadIdx.x; j < n; j += (size_t)gridDim.x * RT) {
+        const uint32_t c = code[j];
+        st16(x + j, signed_(ld16(xr + key_of(c)), c & 1u));
+    }
+}
+// fx = y - x ; g = x + beta fx ; block maxima of |fx|² (y full, x one value per key)
+__global__ void __launch_bounds__(RT) k_aa_residual(const cplx* y, const cplx* xr, const uint32_t* code,
+                                                    const uint32_t* src, cplx* fx, cplx* g, double beta, double* pmax,
+                                                    size_t nr) {
+    __shared__ double red[RT];
+    double mx = 0.0;
+    for (size_t k = blockIdx.x * (size_t)RT + threadIdx.x; k < nr; k += (size_t)gridDim.x * RT) {
+        const cplx x = xr[k], f = key_value(y, code, src, k) - x;
+        fx[k] = f;
+        g[k] = x + f * beta;
+        mx = fmax(mx, f.x * f.x + f.y * f.y);
+    }
+    red[threadIdx.x] = mx;
+    __syncthreads();
+    for (int o = RT / 2; o > 0; o >>= 1) {
+        if ((int)threadIdx.x < o) red[threadIdx.x] = fmax(red[threadIdx.x], red[threadIdx.x + o]);
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) pmax[blockIdx.x] = red[0];
+}
+
+// What bounds the step: at full length the FP64 pipe (about 200 FP64 instructions per element at
+// m = 8: 1.0 ms at 1.87 M elements); at one value per key the launches.  So a pass does all the work
+// that its vectors allow: the Givens rotations of a column deletion, Δg and Δf and the first
+// projection run in one pass, every Gram-Schmidt pass also takes the partial of <Q_i, f> (no separate
+// pass of dot products), and γ and the next deletion's rotations come from one single-block kernel.
+// A step beside the map at m = 8 on GB300, on full vectors with separate passes -> now: Hubbard 8x8,
+// nK3 = (8, 12): 1.03 -> 0.22 ms; Hubbard 8x8, nK3 = (20, 40), 49 M elements: 22 -> 1.9 ms; SIAM,
+// nK3 = (16, 16), 0.1 M elements: 0.26 -> 0.19 ms.
+
+// Column rotations (nrot > 0: the nrot = m - 1 rotations of a deletion, applied to Q in order), then
+// Δg = g - gold ; Δf = fx - fxold (in place in fxold) ; partial of <Q_0, Δf>, or of |Δf|² when Q has no
+// column left (k = 0).
 __global__ void __launch_bounds__(RT) k_aa_diff(cplx* dg, const cplx* g, const cplx* gold, cplx* df, const cplx* fx,
-                                                const cplx* Qb, cplx* part_out, size_t n) {
+                                                AAVecsW Q, int k, int nrot, const cplx* rot, const double* wgt,
+                                                cplx* part_out, size_t n) {
     __shared__ cplx sh[RT];
+    __shared__ cplx rs[2 * AA_MAX];
+    for (int i = threadIdx.x; i < 2 * nrot; i += RT) rs[i] = rot[i];
+    __syncthreads();
     cplx s = mk(0.0, 0.0);
-    for (size_t i = blockIdx.x * (size_t)RT + threadIdx.x; i < n; i += (size_t)gridDim.x * RT) {
-        dg[i] = g[i] - gold[i];
-        const cplx v = fx[i] - df[i];
-        df[i] = v;
-        if (Qb) s = cfma_conj(Qb[i], v, s);
-        else s.x = norm2_acc(v, s.x);
+    for (size_t t = blockIdx.x * (size_t)RT + threadIdx.x; t < n; t += (size_t)gridDim.x * RT) {
+        cplx q0 = mk(0.0, 0.0);
+        if (nrot > 0) {
+            cplx a = Q.v[0][t];
+            for (int i = 1; i <= nrot; ++i) {
+                const double c = rs[2 * (i - 1)].x;
+                const cplx sn = rs[2 * (i - 1) + 1];
+                const cplx b = Q.v[i][t];
+                // Q_{i-1} = c a + conj(s) b ; a = -s a + c b
+                const cplx r = mk(fma(a.x, c, fma(sn.x, b.x, sn.y * b.y)), fma(a.y, c, fma(sn.x, b.y, -sn.y * b.x)));
+                Q.v[i - 1][t] = r;
+                if (i == 1) q0 = r;
+                // (the last column of a deletion is overwritten by the new one: not formed)
+                if (i < nrot) a = mk(fma(b.x, c, fma(-sn.x, a.x, sn.y * a.y)), fma(b.y, c, fma(-sn.x, a.y, -sn.y * a.x)));
+            }
+        } else if (k > 0) {
+            q0 = Q.v[0][t];
+        }
+        dg[t] = g[t] - gold[t];
+        const cplx v = fx[t] - df[t];
+        df[t] = v;
+        const cplx wv = wgt ? v * wgt[t] : v;
+        if (k > 0) s = cfma_conj(q0, wv, s);
+        else s.x = fma(v.x, wv.x, fma(v.y, wv.y, s.x));
     }
     block_store_partial(s, sh, part_out);
 }
 
 // One modified Gram-Schmidt step: r = Σ part_in (= <Qa, Δf>), R entry = r, Δf -= r Qa; then the
-// partial of the next projection <Qb, Δf> (or |Δf|² when Qb is null).
+// partials of the next projection <Qb, Δf> (or |Δf|² when Qb is null) and of <Qa, fx>.
 __global__ void __launch_bounds__(RT) k_aa_mgs(cplx* df, const cplx* Qa, const cplx* part_in, int np, cplx* Rentry,
-                                               const cplx* Qb, cplx* part_out, size_t n) {
+                                               const cplx* Qb, const cplx* fx, const double* wgt, cplx* part_out,
+                                               cplx* pdot, size_t n) {
     __shared__ cplx sh[RT];
     const cplx r = block_reduce_parts(part_in, np, sh);
     if (blockIdx.x == 0 && threadIdx.x == 0) *Rentry = r;
-    cplx s = mk(0.0, 0.0);
+    cplx s = mk(0.0, 0.0), q = mk(0.0, 0.0);
     for (size_t i = blockIdx.x * (size_t)RT + threadIdx.x; i < n; i += (size_t)gridDim.x * RT) {
-        const cplx v = cfnma(r, Qa[i], df[i]);
+        const cplx a = Qa[i];
+        const cplx v = cfnma(r, a, df[i]);
         df[i] = v;
-        if (Qb) s = cfma_conj(Qb[i], v, s);
-        else s.x = norm2_acc(v, s.x);
+        cplx wv = v, wf = fx[i];
+        if (wgt) { const double w = wgt[i]; wv = wv * w; wf = wf * w; }
+        q = cfma_conj(a, wf, q);
+        if (Qb) s = cfma_conj(Qb[i], wv, s);
+        else s.x = fma(v.x, wv.x, fma(v.y, wv.y, s.x));
     }
     block_store_partial(s, sh, part_out);
+    __syncthreads();
+    block_store_partial(q, sh, pdot);
 }
 
-// ‖Δf‖ = sqrt(Σ part_in), R(k,k) = ‖Δf‖, Q_k = Δf / ‖Δf‖.
+// ‖Δf‖ = sqrt(Σ part_in), R(k,k) = ‖Δf‖, Q_k = Δf / ‖Δf‖, partial of <Q_k, fx>.
 __global__ void __launch_bounds__(RT) k_aa_qnew(cplx* Qk, const cplx* df, const cplx* part_in, int np, cplx* Rkk,
-                                                size_t n) {
+                                                const cplx* fx, const double* wgt, cplx* pdot, size_t n) {
     __shared__ cplx sh[RT];
     const double nr = sqrt(fmax(0.0, block_reduce_parts(part_in, np, sh).x));
     if (blockIdx.x == 0 && threadIdx.x == 0) *Rkk = mk(nr, 0.0);
     const double inv = 1.0 / nr;  // one division per block, not two per element
+    cplx q = mk(0.0, 0.0);
     for (size_t i = blockIdx.x * (size_t)RT + threadIdx.x; i < n; i += (size_t)gridDim.x * RT) {
-        const cplx v = df[i];
-        Qk[i] = mk(v.x * inv, v.y * inv);
+        const cplx v = df[i], u = mk(v.x * inv, v.y * inv);
+        Qk[i] = u;
+        cplx wf = fx[i];
+        if (wgt) wf = wf * wgt[i];
+        q = cfma_conj(u, wf, q);
     }
+    block_store_partial(q, sh, pdot);
 }
 
-// Partials of <Q_i, fx> for the AA_CHUNK vectors of chunk blockIdx.y: part[(i) * np + blockIdx.x].
-constexpr int AA_CHUNK = 8;
-__global__ void __launch_bounds__(RT) k_aa_multidot(AAVecs Q, int nv, const cplx* fx, cplx* part, int np, size_t n) {
-    __shared__ cplx sh[RT];
-    const int i0 = blockIdx.y * AA_CHUNK;
-    const int cnt = min(AA_CHUNK, nv - i0);
-    cplx s[AA_CHUNK];
-#pragma unroll
-    for (int j = 0; j < AA_CHUNK; ++j) s[j] = mk(0.0, 0.0);
-    for (size_t i = blockIdx.x * (size_t)RT + threadIdx.x; i < n; i += (size_t)gridDim.x * RT) {
-        const cplx f = fx[i];
-#pragma unroll
-        for (int j = 0; j < AA_CHUNK; ++j)
-            if (j < cnt) s[j] = cfma_conj(Q.v[i0 + j][i], f, s[j]);
+__device__ __forceinline__ double cabs_(cplx a) { return hypot(a.x, a.y); }
+// Deletion of the first column of the m x m QR factor by Givens rotations (NLsolve qrdelete!):
+// rotation i = 1..m-1 acts on rows (i-1, i) of R; the parameters go to rot[2(i-1)] = (c, -) and
+// rot[2(i-1)+1] = s; then the columns shift left by one.  One warp, a column of R per lane: the rotations
+// are a serial chain, the columns are not (one thread took 66 us at m = 8).
+__device__ __forceinline__ void givens_delete(cplx* R, int m, cplx* rot) {
+    const int lane = threadIdx.x & 31;
+    auto Rr = [&](int i, int j) -> cplx& { return R[i + (size_t)m * j]; };
+    for (int i = 1; i < m; ++i) {
+        const cplx f = Rr(i - 1, i), g = Rr(i, i);
+        const double af = cabs_(f), ag = cabs_(g);
+        double c;
+        cplx sn;
+        if (ag == 0.0) { c = 1.0; sn = mk(0.0, 0.0); }
+        else if (af == 0.0) { c = 0.0; sn = mk(g.x / ag, -g.y / ag); }
+        else {
+            const double rr = hypot(af, ag);
+            c = af / rr;
+            const cplx fa = mk(f.x / af, f.y / af);
+            sn = fa * conjg(g);
+            sn = mk(sn.x / rr, sn.y / rr);
+        }
+        __syncwarp();
+        for (int j = lane; j < m; j += 32) {
+            const cplx a = Rr(i - 1, j), b = Rr(i, j);
+            Rr(i - 1, j) = a * c + sn * b;
+            Rr(i, j) = (-conjg(sn)) * a + b * c;
+        }
+        if (lane == 0) {
+            rot[2 * (i - 1)] = mk(c, 0.0);
+            rot[2 * (i - 1) + 1] = sn;
+        }
+        __syncwarp();
     }
-    for (int j = 0; j < cnt; ++j) block_store_partial(s[j], sh, part + (size_t)(i0 + j) * np);
+    for (int j = 0; j < m - 1; ++j) {
+        for (int i = lane; i < m - 1; i += 32) Rr(i, j) = Rr(i, j + 1);
+        __syncwarp();
+    }
 }
+__global__ void k_aa_givens(cplx* R, int m, cplx* rot) { givens_delete(R, m, rot); }
 
-// γ = R⁻¹ (Σ_blocks part): one block; each column of partials is reduced exactly like the
-// Gram-Schmidt coefficients, then thread 0 back-substitutes.  R is column-major m x m.
-__global__ void __launch_bounds__(RT) k_aa_gamma(const cplx* part, int np, const cplx* R, int m, int meff, cplx* gam) {
-    __shared__ cplx sh[RT];
+// γ = R⁻¹ (Σ_blocks part): one block; a warp per column of partials, then one warp back-substitutes
+// (a row of R per lane).  R is column-major m x m.  del: the rotations of the next step's column
+// deletion follow in the same launch (R is not read by the update in between).
+__global__ void __launch_bounds__(RT) k_aa_gamma(const cplx* part, int stride, int np, cplx* R, int m, int meff,
+                                                 cplx* gam, int del, cplx* rot) {
     __shared__ cplx g[AA_MAX];
-    for (int i = 0; i < meff; ++i) {
-        const cplx s = block_reduce_parts(part + (size_t)i * np, np, sh);
-        if (threadIdx.x == 0) g[i] = s;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (int i = warp; i < meff; i += RT / 32) {
+        cplx s = mk(0.0, 0.0);
+        for (int b = lane; b < np; b += 32) s += part[(size_t)i * stride + b];
+        s = warp_sum(s);
+        if (lane == 0) g[i] = s;
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int i = meff - 1; i >= 0; --i) {
-            cplx v = g[i];
-            for (int j = i + 1; j < meff; ++j) v -= R[i + (size_t)m * j] * g[j];
-            g[i] = cdiv(v, R[i + (size_t)m * i]);
-        }
-        for (int i = 0; i < meff; ++i) gam[i] = g[i];
+    if (warp != 0) return;
+    for (int i = meff - 1; i >= 0; --i) {
+        const cplx x = cdiv(g[i], R[i + (size_t)m * i]);
+        __syncwarp();
+        if (lane == 0) { g[i] = x; gam[i] = x; }
+        for (int j = lane; j < i; j += 32) g[j] = cfnma(R[j + (size_t)m * i], x, g[j]);
+        __syncwarp();
     }
+    if (del) givens_delete(R, m, rot);
 }
 
 // x = g - Σ_i γ_i Δg_i (i in order) ; fxold = fx ; gold = g.
@@ -152,58 +292,6 @@ __global__ void __launch_bounds__(RT) k_aa_update(cplx* x, const cplx* g, AAVecs
     }
 }
 
-// Deletion of the first column of the m x m QR factor by Givens rotations (NLsolve qrdelete!):
-// rotation i = 1..m-1 acts on rows (i-1, i) of R; the parameters go to rot[i-1] = (c, s, -);
-// then the columns shift left by one.  One thread: m² work on a handful of numbers.
-__device__ __forceinline__ double cabs_(cplx a) { return hypot(a.x, a.y); }
-__global__ void k_aa_givens(cplx* R, int m, cplx* rot) {
-    if (blockIdx.x != 0 || threadIdx.x != 0) return;
-    auto Rr = [&](int i, int j) -> cplx& { return R[i + (size_t)m * j]; };
-    for (int i = 1; i < m; ++i) {
-        const cplx f = Rr(i - 1, i), g = Rr(i, i);
-        const double af = cabs_(f), ag = cabs_(g);
-        double c;
-        cplx sn;
-        if (ag == 0.0) { c = 1.0; sn = mk(0.0, 0.0); }
-        else if (af == 0.0) { c = 0.0; sn = mk(g.x / ag, -g.y / ag); }
-        else {
-            const double rr = hypot(af, ag);
-            c = af / rr;
-            const cplx fa = mk(f.x / af, f.y / af);
-            sn = fa * conjg(g);
-            sn = mk(sn.x / rr, sn.y / rr);
-        }
-        for (int j = 0; j < m; ++j) {
-            const cplx a = Rr(i - 1, j), b = Rr(i, j);
-            Rr(i - 1, j) = a * c + sn * b;
-            Rr(i, j) = (-conjg(sn)) * a + b * c;
-        }
-        rot[2 * (i - 1)] = mk(c, 0.0);
-        rot[2 * (i - 1) + 1] = sn;
-    }
-    for (int j = 0; j < m - 1; ++j)
-        for (int i = 0; i < m - 1; ++i) Rr(i, j) = Rr(i, j + 1);
-}
-
-// The m-1 rotations applied to the columns of Q, in order, at each element.
-__global__ void __launch_bounds__(RT) k_aa_qrot(AAVecsW Q, int m, const cplx* rot, size_t n) {
-    __shared__ cplx rs[2 * AA_MAX];
-    for (int i = threadIdx.x; i < 2 * (m - 1); i += RT) rs[i] = rot[i];
-    __syncthreads();
-    for (size_t t = blockIdx.x * (size_t)RT + threadIdx.x; t < n; t += (size_t)gridDim.x * RT) {
-        cplx a = Q.v[0][t];
-        for (int i = 1; i < m; ++i) {
-            const double c = rs[2 * (i - 1)].x;
-            const cplx sn = rs[2 * (i - 1) + 1];
-            const cplx b = Q.v[i][t];
-            // Q_{i-1} = c a + conj(s) b ; a = -s a + c b
-            Q.v[i - 1][t] = mk(fma(a.x, c, fma(sn.x, b.x, sn.y * b.y)), fma(a.y, c, fma(sn.x, b.y, -sn.y * b.x)));
-            a = mk(fma(b.x, c, fma(-sn.x, a.x, sn.y * a.y)), fma(b.y, c, fma(-sn.x, a.y, -sn.y * a.x)));
-        }
-        Q.v[m - 1][t] = a;
-    }
-}
-
 }  // namespace
 
 #define AA_CHECK()                                   \
@@ -212,27 +300,45 @@ __global__ void __launch_bounds__(RT) k_aa_qrot(AAVecsW Q, int m, const cplx* ro
         if (e__ != cudaSuccess) return e__;          \
     } while (0)
 
+cudaError_t launch_aa_keys(cudaStream_t s, int nblk, const uint32_t* code, uint32_t* src, double* w, size_t n) {
+    k_aa_keys<<<nblk, RT, 0, s>>>(code, src, w, n);
+    AA_CHECK(); return cudaSuccess;
+}
+cudaError_t launch_aa_check(cudaStream_t s, int nblk, const cplx* x, const uint32_t* code, const uint32_t* src,
+                            unsigned int* count, size_t n) {
+    k_aa_check<<<nblk, RT, 0, s>>>(x, code, src, count, n);
+    AA_CHECK(); return cudaSuccess;
+}
+cudaError_t launch_aa_gather(cudaStream_t s, int nblk, cplx* xr, const cplx* x, const uint32_t* code,
+                             const uint32_t* src, size_t nr) {
+    k_aa_gather<<<nblk, RT, 0, s>>>(xr, x, code, src, nr);
+    AA_CHECK(); return cudaSuccess;
+}
+cudaError_t launch_aa_expand(cudaStream_t s, cplx* x, const cplx* xr, const uint32_t* code, size_t n) {
+    const size_t nb = (n + RT - 1) / RT;
+    k_aa_expand<<<(unsigned)(nb < 4864 ? nb : 4864), RT, 0, s>>>(x, xr, code, n);  // 32 CTAs per SM of 152
+    AA_CHECK(); return cudaSuccess;
+}
+cudaError_t launch_aa_residual(cudaStream_t s, int nblk, const cplx* y, const cplx* xr, const uint32_t* code,
+                               const uint32_t* src, cplx* fx, cplx* g, double beta, double* pmax, size_t nr) {
+    k_aa_residual<<<nblk, RT, 0, s>>>(y, xr, code, src, fx, g, beta, pmax, nr);
+    AA_CHECK(); return cudaSuccess;
+}
 cudaError_t launch_aa_diff(cudaStream_t s, int nblk, cplx* dg, const cplx* g, const cplx* gold, cplx* df,
-                           const cplx* fx, const cplx* Qb, cplx* part_out, size_t n) {
-    k_aa_diff<<<nblk, RT, 0, s>>>(dg, g, gold, df, fx, Qb, part_out, n);
+                           const cplx* fx, const AAVecsW& Q, int k, int nrot, const cplx* rot, const double* wgt,
+                           cplx* part_out, size_t n) {
+    if (k < 0 || k >= AA_MAX || nrot < 0 || nrot >= AA_MAX) return cudaErrorInvalidValue;
+    k_aa_diff<<<nblk, RT, 0, s>>>(dg, g, gold, df, fx, Q, k, nrot, rot, wgt, part_out, n);
     AA_CHECK(); return cudaSuccess;
 }
 cudaError_t launch_aa_mgs(cudaStream_t s, int nblk, cplx* df, const cplx* Qa, const cplx* part_in, cplx* Rentry,
-                          const cplx* Qb, cplx* part_out, size_t n) {
-    k_aa_mgs<<<nblk, RT, 0, s>>>(df, Qa, part_in, nblk, Rentry, Qb, part_out, n);
+                          const cplx* Qb, const cplx* fx, const double* wgt, cplx* part_out, cplx* pdot, size_t n) {
+    k_aa_mgs<<<nblk, RT, 0, s>>>(df, Qa, part_in, nblk, Rentry, Qb, fx, wgt, part_out, pdot, n);
     AA_CHECK(); return cudaSuccess;
 }
 cudaError_t launch_aa_qnew(cudaStream_t s, int nblk, cplx* Qk, const cplx* df, const cplx* part_in, cplx* Rkk,
-                           size_t n) {
-    k_aa_qnew<<<nblk, RT, 0, s>>>(Qk, df, part_in, nblk, Rkk, n);
-    AA_CHECK(); return cudaSuccess;
-}
-cudaError_t launch_aa_gamma(cudaStream_t s, int nblk, const AAVecs& Q, int meff, const cplx* fx, cplx* part,
-                            const cplx* R, int m, cplx* gam, size_t n) {
-    if (meff < 1 || meff > AA_MAX) return cudaErrorInvalidValue;
-    k_aa_multidot<<<dim3(nblk, (meff + AA_CHUNK - 1) / AA_CHUNK), RT, 0, s>>>(Q, meff, fx, part, nblk, n);
-    AA_CHECK();
-    k_aa_gamma<<<1, RT, 0, s>>>(part, nblk, R, m, meff, gam);
+                           const cplx* fx, const double* wgt, cplx* pdot, size_t n) {
+    k_aa_qnew<<<nblk, RT, 0, s>>>(Qk, df, part_in, nblk, Rkk, fx, wgt, pdot, n);
     AA_CHECK(); return cudaSuccess;
 }
 cudaError_t launch_aa_update(cudaStream_t s, int nblk, cplx* x, const cplx* g, const AAVecs& dG, const cplx* gam,
@@ -246,16 +352,10 @@ cudaError_t launch_aa_givens(cudaStream_t s, cplx* R, int m, cplx* rot) {
     k_aa_givens<<<1, 32, 0, s>>>(R, m, rot);
     AA_CHECK(); return cudaSuccess;
 }
-cudaError_t launch_aa_gamma_solve(cudaStream_t s, const cplx* part, int np, const cplx* R, int m, int meff, cplx* gam) {
-    if (meff < 1 || meff > AA_MAX) return cudaErrorInvalidValue;
-    k_aa_gamma<<<1, RT, 0, s>>>(part, np, R, m, meff, gam);
-    AA_CHECK(); return cudaSuccess;
-}
-cudaError_t launch_aa_delete(cudaStream_t s, int nblk, cplx* R, int m, cplx* rot, const AAVecsW& Q, size_t n) {
-    if (m < 2 || m > AA_MAX) return cudaErrorInvalidValue;
-    k_aa_givens<<<1, 32, 0, s>>>(R, m, rot);
-    AA_CHECK();
-    k_aa_qrot<<<nblk, RT, 0, s>>>(Q, m, rot, n);
+cudaError_t launch_aa_gamma(cudaStream_t s, const cplx* part, int stride, int np, cplx* R, int m, int meff, cplx* gam,
+                            int del, cplx* rot) {
+    if (meff < 1 || meff > AA_MAX || (del && (m < 2 || meff != m))) return cudaErrorInvalidValue;
+    k_aa_gamma<<<1, RT, 0, s>>>(part, stride, np, R, m, meff, gam, del, rot);
     AA_CHECK(); return cudaSuccess;
 }
 

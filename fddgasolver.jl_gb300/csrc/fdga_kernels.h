@@ -300,19 +300,26 @@ cudaError_t launch_residual(cudaStream_t s, const cplx* y, const cplx* x, cplx* 
                             int nblk, size_t n);
 cudaError_t launch_sub(cudaStream_t s, cplx* out, const cplx* a, const cplx* b, size_t n);
 cudaError_t launch_gather_sub(cudaStream_t s, cplx* out, const cplx* y, const cplx* x, const uint32_t* perm, size_t n);
+cudaError_t launch_aa_keys(cudaStream_t s, int nblk, const uint32_t* code, uint32_t* src, double* w, size_t n);
+cudaError_t launch_aa_check(cudaStream_t s, int nblk, const cplx* x, const uint32_t* code, const uint32_t* src,
+                            unsigned int* count, size_t n);
+cudaError_t launch_aa_gather(cudaStream_t s, int nblk, cplx* xr, const cplx* x, const uint32_t* code,
+                             const uint32_t* src, size_t nr);
+cudaError_t launch_aa_expand(cudaStream_t s, cplx* x, const cplx* xr, const uint32_t* code, size_t n);
+cudaError_t launch_aa_residual(cudaStream_t s, int nblk, const cplx* y, const cplx* xr, const uint32_t* code,
+                               const uint32_t* src, cplx* fx, cplx* g, double beta, double* pmax, size_t nr);
 cudaError_t launch_aa_diff(cudaStream_t s, int nblk, cplx* dg, const cplx* g, const cplx* gold, cplx* df,
-                           const cplx* fx, const cplx* Qb, cplx* part_out, size_t n);
+                           const cplx* fx, const AAVecsW& Q, int k, int nrot, const cplx* rot, const double* wgt,
+                           cplx* part_out, size_t n);
 cudaError_t launch_aa_mgs(cudaStream_t s, int nblk, cplx* df, const cplx* Qa, const cplx* part_in, cplx* Rentry,
-                          const cplx* Qb, cplx* part_out, size_t n);
+                          const cplx* Qb, const cplx* fx, const double* wgt, cplx* part_out, cplx* pdot, size_t n);
 cudaError_t launch_aa_qnew(cudaStream_t s, int nblk, cplx* Qk, const cplx* df, const cplx* part_in, cplx* Rkk,
-                           size_t n);
-cudaError_t launch_aa_gamma(cudaStream_t s, int nblk, const AAVecs& Q, int meff, const cplx* fx, cplx* part,
-                            const cplx* R, int m, cplx* gam, size_t n);
+                           const cplx* fx, const double* wgt, cplx* pdot, size_t n);
 cudaError_t launch_aa_update(cudaStream_t s, int nblk, cplx* x, const cplx* g, const AAVecs& dG, const cplx* gam,
                              int meff, const cplx* fx, cplx* fxold, cplx* gold, size_t n);
-cudaError_t launch_aa_delete(cudaStream_t s, int nblk, cplx* R, int m, cplx* rot, const AAVecsW& Q, size_t n);
 cudaError_t launch_aa_givens(cudaStream_t s, cplx* R, int m, cplx* rot);
-cudaError_t launch_aa_gamma_solve(cudaStream_t s, const cplx* part, int np, const cplx* R, int m, int meff, cplx* gam);
+cudaError_t launch_aa_gamma(cudaStream_t s, const cplx* part, int stride, int np, cplx* R, int m, int meff, cplx* gam,
+                            int del, cplx* rot);
 // FP32-history Anderson (mixed-precision inner solves)
 cudaError_t launch_ma_residual(cudaStream_t s, int nblk, const cplx* y, const cplx* c, const cplx* x, cplxf* f32,
                                cplx* g, double beta, double* pmax, size_t n);

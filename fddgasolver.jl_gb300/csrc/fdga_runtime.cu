@@ -126,6 +126,12 @@ struct fdga_handle {
                 evR = nullptr;
     // Anderson
     std::vector<cplx*> aa_buf;
+    size_t aa_len = 0;                  // values per vector of aa_buf
+    uint32_t* ak_src = nullptr;         // keys of the state (fdga_anderson.cu): first member, number of members
+    double* ak_w = nullptr;
+    unsigned int* ak_bad = nullptr;
+    int ak_version = -1;
+    double* part_host = nullptr;        // page-locked copy of d_part
     double* d_part = nullptr;
     cplx *aa_R = nullptr, *aa_rot = nullptr, *aa_gam = nullptr, *aa_part = nullptr;  // device QR state
     std::vector<cplx*> kr64;       // Newton-Krylov / linear response, compact (one value per class) FP64
@@ -205,6 +211,11 @@ int dalloc(fdga_handle* h, T** p, size_t n) {
     if (e != cudaSuccess) return fail(h, FDGA_ERR_OOM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
     h->allocs.push_back((void*)*p);
     return cudaMemsetAsync(*p, 0, n * sizeof(T), h->st) == cudaSuccess ? FDGA_OK : FDGA_ERR_CUDA;
+}
+void dfree(fdga_handle* h, void* p) {
+    auto it = std::find(h->allocs.begin(), h->allocs.end(), p);
+    if (it != h->allocs.end()) h->allocs.erase(it);
+    cudaFree(p);
 }
 #define AL(ptr, n)                                           \
     do {                                                     \
@@ -1583,12 +1594,14 @@ int run_iteration(fdga_handle* h, int strategy, bool update_sigma, bool hartree)
 }
 
 double reduce_max(fdga_handle* h, int nblk, int& status) {
-    std::vector<double> part(nblk);
-    cudaError_t e = cudaMemcpyAsync(part.data(), h->d_part, nblk * sizeof(double), cudaMemcpyDeviceToHost, h->st);
+    cudaError_t e = cudaSuccess;
+    if (!h->part_host) e = cudaHostAlloc((void**)&h->part_host, NBLK_RED * sizeof(double), cudaHostAllocDefault);
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(h->part_host, h->d_part, nblk * sizeof(double), cudaMemcpyDeviceToHost, h->st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(h->st);
     if (e != cudaSuccess) { status = cuda_fail(h, e, "reduce_max"); return 0.0; }
     double m = 0.0;  // the partials are squared magnitudes
-    for (double v : part) m = std::max(m, v);
+    for (int i = 0; i < nblk; ++i) m = std::max(m, h->part_host[i]);
     status = FDGA_OK;
     return std::sqrt(m);
 }
@@ -1838,6 +1851,7 @@ void fdga_destroy(fdga_handle* h) {
     drop_graphs(h);
     if (h->flush_buf) cudaFree(h->flush_buf);
     if (h->kr_st_host) cudaFreeHost(h->kr_st_host);
+    if (h->part_host) cudaFreeHost(h->part_host);
     for (void* p : h->allocs) cudaFree(p);
     for (auto& e : h->ev) if (e) cudaEventDestroy(e);
     for (cudaEvent_t e : {h->evfork, h->evA, h->evB, h->evC, h->evD, h->evE, h->evR}) if (e) cudaEventDestroy(e);
@@ -2157,20 +2171,30 @@ struct SolveHooks {
     std::function<int()> before, after;
 };
 
+int ensure_compact(fdga_handle* h);
+
+// Keys of the state for the Anderson vectors (fdga_anderson.cu), rebuilt when the groups change.
+int ensure_keys(fdga_handle* h) {
+    if (int r = ensure_compact(h)) return r;
+    if (h->ak_src && h->ak_version == h->kc_version) return FDGA_OK;
+    if (!h->ak_src) {  // two keys per class; one without members has weight 0
+        AL(h->ak_src, 2 * h->nc);
+        AL(h->ak_w, 2 * h->nc);
+        AL(h->ak_bad, 1);
+    }
+    CK(cudaMemsetAsync(h->ak_src, 0xff, 2 * h->nc * sizeof(uint32_t), h->st));
+    CK(cudaMemsetAsync(h->ak_w, 0, 2 * h->nc * sizeof(double), h->st));
+    CK(launch_aa_keys(h->st, 4 * NBLK_RED, h->kc_code, h->ak_src, h->ak_w, h->nstate));
+    h->ak_version = h->kc_version;
+    return FDGA_OK;
+}
+
 int solve_anderson(fdga_handle* h, int strategy, bool update_sigma, int maxiter, double tol, double beta, int mem,
                    int* iters, double* res, double* trace, const SolveHooks* hk) {
     if (!h) return FDGA_ERR_ARG;
     if (maxiter < 1 || mem < 0 || !(tol >= 0)) return fail(h, FDGA_ERR_ARG, "invalid solver parameters");
     const size_t n = h->nstate;
     const int m = (int)std::min<size_t>((size_t)mem, n);
-    // buffers: fx g fxold gold | dG[m] | Q[m]
-    const size_t need = 4 + 2 * (size_t)m;
-    while (h->aa_buf.size() < need) {
-        cplx* p = nullptr;
-        int r = dalloc(h, &p, n);
-        if (r) return r;
-        h->aa_buf.push_back(p);
-    }
     if (m > AA_MAX) return fail(h, FDGA_ERR_ARG, "Anderson memory exceeds " + std::to_string(AA_MAX));
     if (!h->aa_R) {
         int r = dalloc(h, &h->aa_R, (size_t)AA_MAX * AA_MAX);
@@ -2179,16 +2203,26 @@ int solve_anderson(fdga_handle* h, int strategy, bool update_sigma, int maxiter,
         if (!r) r = dalloc(h, &h->aa_part, (size_t)(AA_MAX + 2) * NBLK_RED);
         if (r) return r;
     }
-    cplx *fx = h->aa_buf[0], *g = h->aa_buf[1], *fxold = h->aa_buf[2], *gold = h->aa_buf[3];
-    std::vector<cplx*> dG(h->aa_buf.begin() + 4, h->aa_buf.begin() + 4 + m);
-    AAVecsW Q{};
-    for (int i = 0; i < m; ++i) Q.v[i] = h->aa_buf[4 + m + i];
-    AAVecs Qc{};
-    for (int i = 0; i < m; ++i) Qc.v[i] = Q.v[i];
+    // One value per key where the symmetry groups are set and both the initial state and its image
+    // hold one value per key (Φ expands its representatives; only Σ0 can break that, and shows in the
+    // first image); else the full vectors.  The two agree to rounding (the order of the sums).
+    bool red = !h->gK1.trivial;
+    if (red) {
+        int r = ensure_keys(h);
+        if (r) return r;
+        CK(cudaMemsetAsync(h->ak_bad, 0, sizeof(unsigned int), h->st));
+        CK(launch_aa_check(h->st, 4 * NBLK_RED, h->xS, h->kc_code, h->ak_src, h->ak_bad, n));
+    }
     cplx* R = h->aa_R;
     cplx* pp[2] = {h->aa_part, h->aa_part + NBLK_RED};  // ping-pong partials of the Gram-Schmidt passes
     cplx* pdot = h->aa_part + 2 * NBLK_RED;              // partials of Qᴴ fx, [AA_MAX][NBLK_RED]
     if (m > 0) CK(cudaMemsetAsync(R, 0, (size_t)m * m * sizeof(cplx), h->st));
+    size_t nr = n;
+    int nblk = NBLK_RED;
+    cplx *xr = nullptr, *fx = nullptr, *g = nullptr, *fxold = nullptr, *gold = nullptr;
+    const double* wgt = nullptr;
+    std::vector<cplx*> dG;
+    AAVecsW Q{};
     int m_eff = 0, it = 0, status = 0;
     double resid = 0.0;
     bool converged = false;
@@ -2198,41 +2232,76 @@ int solve_anderson(fdga_handle* h, int strategy, bool update_sigma, int maxiter,
         r = run_iteration(h, strategy, update_sigma, true);
         if (r) return r;
         if (hk && hk->after && (r = hk->after())) return r;
-        CK(launch_residual(h->st, h->yS, h->xS, fx, g, beta, h->d_part, NBLK_RED, n));
-        resid = reduce_max(h, NBLK_RED, status);
+        if (it == 1) {
+            if (red) {
+                unsigned int bad = 0;
+                CK(launch_aa_check(h->st, 4 * NBLK_RED, h->yS, h->kc_code, h->ak_src, h->ak_bad, n));
+                CK(cudaMemcpyAsync(&bad, h->ak_bad, sizeof(bad), cudaMemcpyDeviceToHost, h->st));
+                CK(cudaStreamSynchronize(h->st));
+                red = bad == 0;
+            }
+            nr = red ? 2 * h->nc : n;
+            nblk = (int)std::min<size_t>(NBLK_RED, (nr + 255) / 256);
+            wgt = red ? h->ak_w : nullptr;
+            // buffers: fx g fxold gold xr | dG[m] | Q[m]
+            if (h->aa_len < nr) {
+                CK(cudaStreamSynchronize(h->st));
+                for (cplx* p : h->aa_buf) dfree(h, p);
+                h->aa_buf.clear();
+                h->aa_len = nr;
+            }
+            while (h->aa_buf.size() < 5 + 2 * (size_t)m) {
+                cplx* p = nullptr;
+                if ((r = dalloc(h, &p, h->aa_len))) return r;
+                h->aa_buf.push_back(p);
+            }
+            fx = h->aa_buf[0]; g = h->aa_buf[1]; fxold = h->aa_buf[2]; gold = h->aa_buf[3];
+            xr = red ? h->aa_buf[4] : h->xS;
+            dG.assign(h->aa_buf.begin() + 5, h->aa_buf.begin() + 5 + m);
+            for (int i = 0; i < m; ++i) Q.v[i] = h->aa_buf[5 + m + i];
+            if (red) CK(launch_aa_gather(h->st, nblk, xr, h->xS, h->kc_code, h->ak_src, nr));
+        }
+        if (red) CK(launch_aa_residual(h->st, nblk, h->yS, xr, h->kc_code, h->ak_src, fx, g, beta, h->d_part, nr));
+        else CK(launch_residual(h->st, h->yS, h->xS, fx, g, beta, h->d_part, nblk, n));
+        resid = reduce_max(h, nblk, status);
         if (status) return status;
         if (!std::isfinite(resid)) return fail(h, FDGA_ERR_NONFINITE, "non-finite residual in solve");
         if (trace) trace[it - 1] = resid;
         if (resid < tol) { converged = true; break; }
         if (m == 0 || it == 1) {
-            CK(cudaMemcpyAsync(h->xS, g, n * sizeof(cplx), cudaMemcpyDeviceToDevice, h->st));
+            CK(cudaMemcpyAsync(xr, g, nr * sizeof(cplx), cudaMemcpyDeviceToDevice, h->st));
+            if (red) CK(launch_aa_expand(h->st, h->xS, xr, h->kc_code, n));
             if (m == 0) continue;
-            CK(cudaMemcpyAsync(fxold, fx, n * sizeof(cplx), cudaMemcpyDeviceToDevice, h->st));
-            CK(cudaMemcpyAsync(gold, g, n * sizeof(cplx), cudaMemcpyDeviceToDevice, h->st));
+            CK(cudaMemcpyAsync(fxold, fx, nr * sizeof(cplx), cudaMemcpyDeviceToDevice, h->st));
+            CK(cudaMemcpyAsync(gold, g, nr * sizeof(cplx), cudaMemcpyDeviceToDevice, h->st));
             continue;
         }
         m_eff += 1;
+        int nrot = 0;
         if (m_eff > m) {
-            // qrdelete!: Givens rotations on R and Q, Δg columns shift by one (pointer rotation)
+            // qrdelete!: Givens rotations on R (formed with the last step's γ) and, below, on Q; the Δg
+            // columns shift by one (pointer rotation)
             std::rotate(dG.begin(), dG.begin() + 1, dG.end());
-            if (m > 1) CK(launch_aa_delete(h->st, NBLK_RED, R, m, h->aa_rot, Q, n));
+            nrot = m - 1;
             m_eff = m;
         }
         const int k = m_eff - 1;
         // qradd!: modified Gram-Schmidt of Δf against Q_0..Q_{k-1}, one pass per column
-        CK(launch_aa_diff(h->st, NBLK_RED, dG[k], g, gold, fxold, fx, k > 0 ? Q.v[0] : nullptr, pp[0], n));
+        CK(launch_aa_diff(h->st, nblk, dG[k], g, gold, fxold, fx, Q, k, nrot, h->aa_rot, wgt, pp[0], nr));
         int cur = 0;
         for (int i = 0; i < k; ++i) {
-            CK(launch_aa_mgs(h->st, NBLK_RED, fxold, Q.v[i], pp[cur], R + i + (size_t)m * k,
-                             i + 1 < k ? Q.v[i + 1] : nullptr, pp[cur ^ 1], n));
+            CK(launch_aa_mgs(h->st, nblk, fxold, Q.v[i], pp[cur], R + i + (size_t)m * k,
+                             i + 1 < k ? Q.v[i + 1] : nullptr, fx, wgt, pp[cur ^ 1], pdot + (size_t)i * NBLK_RED, nr));
             cur ^= 1;
         }
-        CK(launch_aa_qnew(h->st, NBLK_RED, Q.v[k], fxold, pp[cur], R + k + (size_t)m * k, n));
+        CK(launch_aa_qnew(h->st, nblk, Q.v[k], fxold, pp[cur], R + k + (size_t)m * k, fx, wgt,
+                          pdot + (size_t)k * NBLK_RED, nr));
         // γ = R⁻¹ Qᴴ fx ; x = g - Σ γ_i Δg_i ; fxold = fx ; gold = g
-        CK(launch_aa_gamma(h->st, NBLK_RED, Qc, m_eff, fx, pdot, R, m, h->aa_gam, n));
+        CK(launch_aa_gamma(h->st, pdot, NBLK_RED, nblk, R, m, m_eff, h->aa_gam, m > 1 && m_eff == m, h->aa_rot));
         AAVecs dGc{};
         for (int i = 0; i < m_eff; ++i) dGc.v[i] = dG[i];
-        CK(launch_aa_update(h->st, NBLK_RED, h->xS, g, dGc, h->aa_gam, m_eff, fx, fxold, gold, n));
+        CK(launch_aa_update(h->st, nblk, xr, g, dGc, h->aa_gam, m_eff, fx, fxold, gold, nr));
+        if (red) CK(launch_aa_expand(h->st, h->xS, xr, h->kc_code, n));
     }
     if (it > maxiter) it = maxiter;
     // S holds Φ(x) of the last evaluation, as after the reference's solve!
@@ -2346,7 +2415,7 @@ int fdga_solve_mixed(fdga_handle* h, int strategy, int maxiter, double tol, doub
                 }
                 CK(launch_ma_qnew(h->st, NBLK_RED, Q.v[k], df, pp[cur], R + k + (size_t)m * k, n));
                 CK(launch_ma_multidot(h->st, NBLK_RED, Qc, m_eff, f, pdot, n));
-                CK(launch_aa_gamma_solve(h->st, pdot, NBLK_RED, R, m, m_eff, h->aa_gam));
+                CK(launch_aa_gamma(h->st, pdot, NBLK_RED, NBLK_RED, R, m, m_eff, h->aa_gam, 0, nullptr));
                 AAVecs32 dGc{};
                 for (int i = 0; i < m_eff; ++i) dGc.v[i] = dG[i];
                 CK(launch_ma_update(h->st, NBLK_RED, h->xS, g, dGc, h->aa_gam, m_eff, f, df, gold, n));
