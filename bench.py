@@ -254,9 +254,11 @@ def k3_gemm_roofline(S, stages, cfg_name):
                 "hbm_frac": byts / (ms * 1e-3) / 1e9 / hbm, "launch_ms": ms,
                 "share_of_iteration": ms / sum(stages.values()),
                 "stage_ms": {k: round(v, 4) for k, v in stages.items()}}
-    traffic = profile_traffic(f"k_bse_K3_gemm_{cfg_name}.md")
-    tile = 16 if N <= 16 else (24 if N <= 24 else 32)
-    return {"bound": "fp64", "kernel": f"k_bse_K3_gemm<1,{tile},cplx> (fused K3 BSE, FP64)", "achieved": achieved,
+    traffic = profile_traffic(f"k_bse_K3_{'mma' if N <= 32 else 'gemm'}_{cfg_name}.md")
+    # blocks of Nν3 ≤ 32: the warp-level digit-sliced kernel, whose FP64-equivalent rate may pass the FP64 pipe's
+    kernel = ("k_bse_K3_mma<1> (fused K3 BSE, FP64 by digit slicing on mma.sync; FP64-equivalent rate)" if N <= 32
+              else "k_bse_K3_gemm<1,32,cplx> (fused K3 BSE, FP64)")
+    return {"bound": "fp64", "kernel": kernel, "achieved": achieved,
             "peak": fp64_peak, "unit": "TFLOP/s", "frac": achieved / fp64_peak,
             "peak_source": "measured: the library's FP64 FMA calibration kernel on this GPU (fdga_query fp64_gflops)",
             "traffic": traffic, "algorithmic_bytes": byts, "hbm_achieved_gbs": byts / (ms * 1e-3) / 1e9,
@@ -519,8 +521,8 @@ def run_batch(args, rank, world, dist):
         S.set_precision("fp64")
     # the FP64 K3 GEMM work of all members (2 GEMMs x 3 channels x representative blocks x N^3
     # complex products, 3 real FMAs = 6 flops each in the CUDA-core kernel's 3M form) at the measured
-    # FP64 FMA rate: the floor of a batch iteration whose K3 GEMMs run on the FP64 pipe; members with
-    # Nν3 ≥ 32 run them on the tensor cores instead (digit slicing), which this floor does not bound
+    # FP64 FMA rate: the floor of a batch iteration whose K3 GEMMs run on the FP64 pipe; the
+    # members run them on the tensor cores instead (digit slicing), which this floor does not bound
     from fdgasolver.solver import _lib_query
     fp64_rate = _lib_query("fp64_gflops") * 1e9
     gemm_flops = sum(6.0 * S.query("k3_blocks") * 6.0 * S.query("k3_block_dim") ** 3 for S in solvers)

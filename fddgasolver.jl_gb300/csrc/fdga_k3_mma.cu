@@ -1,0 +1,304 @@
+// fdga_k3_mma.cu -- the K3 Bethe-Salpeter contractions of the FP64 map for small blocks (Nν3 ≤ 32) on
+// warp-level tensor-core products, by exact digit slicing (the Ozaki scheme): FP64 results from FP16
+// products.
+//
+// Per (channel, representative (P, Ω) block) the BSE is one complex product C = A·M of Nν3 x Nν3
+// matrices (src/BSEa/BSEa_K3.jl:1-128), M formed elementwise in FP64 from the caches, Π, Π0 and FL.  On
+// the CUDA cores it is bound by the FP64 pipe (1/64 of the FP32 rate); the tcgen05 kernel of
+// fdga_k3_oz.cu has 128-row accumulators, of which a 24 x 24 block fills 24 rows, and a fixed cost per
+// CTA (tensor-memory allocation, the pre-pass of A digits, mbarrier round trips) that a block of three
+// K steps does not carry.  mma.sync.m16n8k16 fits these blocks without waste: one warp owns one 8 x 8
+// complex output tile, whose real and imaginary parts are the two 8-row halves of the MMA's 16 rows.
+//
+// Exact slicing.  Row ν of A and column ν' of M each have a power-of-two bound 2^(F-1022) from the
+// largest exponent field of their entries (integer maxima, no FP64 work).  An entry is rounded to the
+// fixed-point integer Y = v 2^(62+1022-F), |Y| < 2^62 (exact for every entry within 2^9 of its row's or
+// column's largest), taken from the FP64 significand by a shift, and Y is cut into S = 8 balanced
+// base-256 digits: adding 0x80 to every byte makes byte s, less 128, the digit d_s in [-128, 127].  A
+// digit is an FP16 number exactly (0x6400 | byte is 1024 + byte; one packed subtraction of 1152 leaves
+// the digit).  The products of digit pairs (s, t) with s + t = g ≤ 7 share one FP32 accumulator:
+// products are at most 2^14 and at most 8·64 of them meet in one accumulator, so every partial sum is an
+// integer of at most 2^23 and exact.  The pairs with s + t ≥ 8 are dropped; with the rounding of Y they
+// leave below 2^-60 of (row bound)·(column bound) per product term, and the 36 digit products replace the
+// FP64 operations (three real products per complex one, 64 issue slots each).  The epilogue joins the
+// eight integers exactly in two 64-bit integers and one FP64 addition, then applies T and γL as the
+// CUDA-core kernel does.  A row of A or a column of M that holds an infinity or NaN gives NaN in that row
+// or column, as the FP64 sums do.
+//
+// What bounds it: forming M (8 to 14 FP64 operations per entry) and the latency of one pass load ->
+// digits -> MMA -> store; a CTA of NC·NC warps (NC = ⌈Nν3/8⌉) does one block, each warp staging one 8 x 8
+// chunk of M and of A and then one output tile, so that no warp idles in either phase.
+// On GB300, CUDA cores -> this kernel, L_K3 / K3 in us: Hubbard 8x8, nK3 = (8, 12) (675 blocks of
+// 24 x 24) 78 / 98 -> 23 / 37; Hubbard 6x6, nK3 = (7, 11) 50 / 59 -> 19 / 25; 5x5 without groups,
+// nK3 = (5, 7) (675 blocks of 14 x 14) 28 / 34 -> 13 / 16; SIAM, nK3 = (6, 6) 18 / 20 -> 9 / 11.  At
+// Nν3 = 24 the tcgen05 kernel takes 79 / 97.
+#include <algorithm>
+
+#include "fdga_digits.cuh"
+#include "fdga_kernels.h"
+
+namespace fdga {
+
+namespace {
+
+constexpr int S = 8;  // digits per operand
+// bytes between rows of a digit plane: an odd multiple of 16, so that the eight 16-byte rows of an 8 x 8
+// matrix (ldmatrix) and the 4-byte stores of 8 columns x 4 ω pairs fall on distinct banks
+template <int NC> constexpr int PITCH = NC == 1 ? 16 : (NC == 4 ? 80 : 48);
+template <int NC> constexpr int PLANE = 8 * NC * PITCH<NC>;
+// planes [A or M][digit][re, im]
+template <int NC> constexpr int SMEM = 2 * S * 2 * PLANE<NC>;
+
+// v 2^(62+1022-F) rounded to an integer (0 for zero and subnormal v); |v| < 2^(F-1022)
+__device__ __forceinline__ long long fixed62(double v, int F) {
+    const unsigned long long b = (unsigned long long)__double_as_longlong(v);
+    const int ev = (int)((b >> 52) & 0x7ffull);
+    const int rs = F - ev - 9;
+    if (ev == 0 || rs >= 55) return 0;
+    const unsigned long long mant = (b & 0xFFFFFFFFFFFFFull) | (1ull << 52);
+    const long long y = (long long)(rs < 0 ? mant << (-rs) : (rs == 0 ? mant : (mant + (1ull << (rs - 1))) >> rs));
+    return (long long)b < 0 ? -y : y;
+}
+// digit k (from the least significant) of two biased integers as a pair of FP16 numbers
+__device__ __forceinline__ uint32_t digit_pair(unsigned long long a, unsigned long long b, int k) {
+    const uint32_t x = k < 4 ? (uint32_t)a : (uint32_t)(a >> 32), y = k < 4 ? (uint32_t)b : (uint32_t)(b >> 32);
+    const uint32_t i = (uint32_t)(k & 3);
+    const uint32_t u = (__byte_perm(x, y, i | ((4u + i) << 8)) & 0x00ff00ffu) | 0x64006400u;
+    uint32_t r;
+    asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"(u), "r"(0x64806480u));  // 0x6480 = 1152
+    return r;
+}
+constexpr unsigned long long BIAS = 0x8080808080808080ull;
+
+// the digits of two neighbouring ω of one row, both parts, stored to the planes at byte offset o
+template <int NC>
+__device__ __forceinline__ void store_digits(uint8_t* planes, int o, cplx v0, cplx v1, int F) {
+    const unsigned long long r0 = (unsigned long long)fixed62(v0.x, F) + BIAS, i0 = (unsigned long long)fixed62(v0.y, F) + BIAS;
+    const unsigned long long r1 = (unsigned long long)fixed62(v1.x, F) + BIAS, i1 = (unsigned long long)fixed62(v1.y, F) + BIAS;
+#pragma unroll
+    for (int s = 0; s < S; ++s) {
+        uint8_t* p = planes + (2 * s) * PLANE<NC> + o;
+        *reinterpret_cast<uint32_t*>(p) = digit_pair(r0, r1, S - 1 - s);
+        *reinterpret_cast<uint32_t*>(p + PLANE<NC>) = digit_pair(i0, i1, S - 1 - s);
+    }
+}
+
+// MODE 0: L_K3, 1: K3 (and the dA·M part of the tangent), 3: the A·dM part of the tangent
+template <int MODE, int NC>
+__global__ void __launch_bounds__(32 * NC * NC) k_bse_K3_mma(K3Args3 args, Dims d) {
+    extern __shared__ __align__(16) uint8_t sm[];
+    uint8_t* Mp = sm;
+    uint8_t* Ap = sm + 2 * S * PLANE<NC>;
+    __shared__ cplx qf[8 * NC][2];  // the ω factors of M with their signs, as in k_bse_K3_oz
+    __shared__ int fmax_[2][8 * NC];  // largest exponent fields: [0] rows ν of A, [1] columns ν' of M
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int N = d.N3n;
+    const int slot = blockIdx.x / args.nblocks, bi = blockIdx.x % args.nblocks;
+    const int blk = args.blocks ? args.blocks[bi] : bi;
+    const K3Args& a = args.a[slot];
+    const int CH = args.ch[slot];
+    const int m = blk % d.N3O - (d.n3O - 1), P = blk / d.N3O;
+    const size_t base = (size_t)blk * N * N;
+    const double s1 = (CH == CH_A) ? 1.0 : -1.0, s2 = (CH == CH_T) ? -1.0 : 1.0;
+    const bool full = MODE == 3 || (MODE == 1 && (a.flags & K3F_1LOOP) == 0);
+    auto gl_of = [&](const cplx* FLc, const cplx* FLt, const cplx* FLa, size_t i) -> cplx {
+        if (CH == CH_T) {
+            const cplx t = ldg(FLt + i), u = ldg(FLa + i);
+            return cplx{fma(t.x, 2.0, -u.x), fma(t.y, 2.0, -u.y)};
+        }
+        return ldg(FLc + i);
+    };
+    if (tid < 8 * NC) {
+        fmax_[0][tid] = fmax_[1][tid] = 0;
+        cplx q0 = mk(0.0, 0.0), q1 = mk(0.0, 0.0);
+        if (tid < N) {
+            const size_t ip = ixPi(d, P, m, tid - d.n3n);
+            q0 = (MODE != 3 && a.Pi0) ? ldg(a.Pi0 + ip) : mk(0.0, 0.0);
+            if (MODE >= 1) {
+                const cplx pi = ldg(a.Pi + ip);
+                q1 = pi * s1;
+                q0 = (MODE == 3) ? ldg(a.tPi + ip) * s1 : (pi - q0) * s1;
+            }
+        }
+        qf[tid][0] = q0;
+        qf[tid][1] = q1;
+    }
+    // staging: warp = (column chunk, ω chunk); a lane holds one column (row of A) and two neighbouring ω
+    const int cl = 8 * (warp % NC) + (lane & 7), w0 = 8 * (warp / NC) + 2 * (lane >> 3);
+    cplx av[2], x0[2], x1[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const int w = w0 + i;
+        av[i] = x0[i] = x1[i] = mk(0.0, 0.0);
+        if (cl >= N || w >= N) continue;
+        av[i] = ldg(a.A + base + (size_t)cl * N + w);
+        x0[i] = ldg(a.B0 + base + (size_t)w * N + cl);
+        if (full) {
+            // s2 Π = ±s1 Π: the γL terms join the Γ terms before the products
+            const size_t ig = (CH == CH_P) ? base + (size_t)w * N + cl : base + (size_t)cl * N + w;
+            const int ot = cross(CH, m, w - d.n3n);
+            const bool hl = fin(ot, d.n3n);
+            const size_t il = base + (size_t)(ot + d.n3n) * N + cl;
+            cplx g = ldg(a.G + ig);
+            if (hl) {
+                const cplx l = gl_of(a.FLc, a.FLt, a.FLa, il);
+                g = (s1 == s2) ? g + l : g - l;
+            }
+            if (MODE == 3) {  // dM = s1 dΠ (F0 + Γ ± γL) + s1 Π (dΓ ± dγL)
+                x0[i] += g;
+                g = ldg(a.tG + ig);
+                if (hl) {
+                    const cplx l = gl_of(a.tFLc, a.tFLt, a.tFLa, il);
+                    g = (s1 == s2) ? g + l : g - l;
+                }
+            }
+            x1[i] = g;
+        }
+    }
+    __syncthreads();
+    cplx mv[2];
+    int em = 0, ea = 0;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        mv[i] = mk(0.0, 0.0);
+        if (cl < N && w0 + i < N) {
+            const cplx* q = qf[w0 + i];
+            mv[i] = full ? cfma(q[0], x0[i], q[1] * x1[i]) : q[0] * x0[i];
+        }
+        em = max(em, cexpo(mv[i]));
+        ea = max(ea, cexpo(av[i]));
+    }
+#pragma unroll
+    for (int o = 8; o <= 16; o <<= 1) {
+        em = max(em, __shfl_xor_sync(0xffffffffu, em, o));
+        ea = max(ea, __shfl_xor_sync(0xffffffffu, ea, o));
+    }
+    if (lane < 8) {
+        atomicMax(&fmax_[0][cl], ea);
+        atomicMax(&fmax_[1][cl], em);
+    }
+    __syncthreads();
+    const int so = cl * PITCH<NC> + 2 * w0;
+    store_digits<NC>(Ap, so, av[0], av[1], fmax_[0][cl]);
+    store_digits<NC>(Mp, so, mv[0], mv[1], fmax_[1][cl]);
+    __syncthreads();
+    // warp = (ν' chunk j, ν chunk nt): D rows 0-7 = Re, rows 8-15 = Im of the outputs ν' = 8j.., columns ν
+    const int j = warp % NC, nt = warp / NC;
+    float acc[S][4];
+#pragma unroll
+    for (int g = 0; g < S; ++g)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) acc[g][i] = 0.0f;
+    // lane l addresses row l % 8 of matrix l / 8: M re, M im, A re, A im of one digit
+    const uint32_t laddr = (uint32_t)__cvta_generic_to_shared(
+        (lane < 16 ? Mp + (8 * j + (lane & 7)) * PITCH<NC> : Ap + (8 * nt + (lane & 7)) * PITCH<NC>) +
+        ((lane >> 3) & 1) * PLANE<NC>);
+#pragma unroll 1
+    for (int c = 0; c < NC; ++c) {
+        uint32_t mr[S], mi[S], ar[S], ai[S];
+#pragma unroll
+        for (int s = 0; s < S; ++s)
+            asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+                         : "=r"(mr[s]), "=r"(mi[s]), "=r"(ar[s]), "=r"(ai[s])
+                         : "r"(laddr + (uint32_t)(2 * s * PLANE<NC> + 16 * c))
+                         : "memory");
+        // k = (ω chunk; Re A, Im A): rows Re: [Re M, -Im M], rows Im: [Im M, Re M]
+#pragma unroll
+        for (int s = 0; s < S; ++s)
+#pragma unroll
+            for (int t = 0; s + t < S; ++t)
+                asm volatile(
+                    "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
+                    "{%0,%1,%2,%3};"
+                    : "+f"(acc[s + t][0]), "+f"(acc[s + t][1]), "+f"(acc[s + t][2]), "+f"(acc[s + t][3])
+                    : "r"(mr[s]), "r"(mi[s]), "r"(mi[s] ^ 0x80008000u), "r"(mr[s]), "r"(ar[t]), "r"(ai[t]));
+    }
+    // D = 2^(F_A + F_M - 2044 - 124) Σ_g 256^(14-g) acc_g, joined as hi 256^11 + lo 256^7
+    const int col = 8 * j + (lane >> 2);
+    if (col >= N) return;
+    const int FM = fmax_[1][col];
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+        const int nu = 8 * nt + 2 * (lane & 3) + e;
+        if (nu >= N) continue;
+        const int FA = fmax_[0][nu], E = FA + FM - 2168;
+        const size_t io = base + (size_t)nu * N + col;
+        cplx o;
+        if (FA == 0x7ff || FM == 0x7ff) {
+            const double qn = __longlong_as_double(0x7ff8000000000000ll);
+            o = mk(qn, qn);
+        } else {
+            double p[2];
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                long long hi = 0, lo = 0;
+#pragma unroll
+                for (int g = 0; g < S; ++g) {
+                    const long long v = (long long)__float2int_rn(acc[g][2 * q + e]);
+                    if (g < 4) hi = hi * 256 + v;
+                    else lo = lo * 256 + v;
+                }
+                p[q] = i2d_scaled(hi, E + 88) + i2d_scaled(lo, E + 56);
+            }
+            const cplx cv = mk(p[0], p[1]);
+            if (MODE == 0) {
+                o = cv * (d.T * ((CH == CH_A) ? 1.0 : -1.0));
+            } else if (a.flags & K3F_NOEPI) {
+                o = cv * d.T;
+            } else {
+                const cplx g = (MODE == 3) ? gl_of(a.tFLc, a.tFLt, a.tFLa, io) : gl_of(a.FLc, a.FLt, a.FLa, io);
+                o = cplx{fma(cv.x, d.T, g.x), fma(cv.y, d.T, g.y)};
+            }
+            if (a.flags & K3F_ACC) o = a.out[io] + o;
+        }
+        a.out[io] = o;
+    }
+}
+
+template <int MODE, int NC>
+cudaError_t run_mma(cudaStream_t s, const K3Args3& a, int nslots, const Dims& d) {
+    k_bse_K3_mma<MODE, NC><<<(unsigned)(nslots * a.nblocks), 32 * NC * NC, SMEM<NC>, s>>>(a, d);
+    return cudaGetLastError();
+}
+template <int MODE>
+cudaError_t run_mode(cudaStream_t s, const K3Args3& a, int nslots, const Dims& d) {
+    switch ((d.N3n + 7) / 8) {
+        case 1: return run_mma<MODE, 1>(s, a, nslots, d);
+        case 2: return run_mma<MODE, 2>(s, a, nslots, d);
+        case 3: return run_mma<MODE, 3>(s, a, nslots, d);
+        default: return run_mma<MODE, 4>(s, a, nslots, d);
+    }
+}
+
+}  // namespace
+
+bool k3_mma_supported(const Dims& d) { return d.N3n <= 32; }
+
+// raises the shared-memory limit of the four-chunk instantiations (82 KB); the others fit the default
+cudaError_t prepare_bse_K3_mma(const Dims& d) {
+    if (d.N3n <= 24) return cudaSuccess;
+    static SmemRecord set0, set1, set3;
+    cudaError_t e = raise_smem_limit(k_bse_K3_mma<0, 4>, set0, SMEM<4>, 0);
+    if (e == cudaSuccess) e = raise_smem_limit(k_bse_K3_mma<1, 4>, set1, SMEM<4>, 0);
+    if (e == cudaSuccess) e = raise_smem_limit(k_bse_K3_mma<3, 4>, set3, SMEM<4>, 0);
+    return e;
+}
+
+// mode 0 (BSE_L_K3), 1 (BSE_K3), 2 (the tangent dK3 = T (dA·M + A·dM) + dγL, as two launches with their
+// own scales: dA and A need not share a magnitude)
+cudaError_t launch_bse_K3_mma(cudaStream_t s, int mode, const K3Args3& a, int nslots, const Dims& d) {
+    if (!k3_mma_supported(d) || mode < 0 || mode > 2) return cudaErrorInvalidValue;
+    if (mode == 0) return run_mode<0>(s, a, nslots, d);
+    if (mode == 1) return run_mode<1>(s, a, nslots, d);
+    K3Args3 a1 = a, a3 = a;
+    for (int i = 0; i < nslots; ++i) {
+        if (a.a[i].flags & K3F_1LOOP) return cudaErrorInvalidValue;  // no tangent of the one-loop form
+        a1.a[i].A = a.a[i].tA;
+        a1.a[i].flags |= K3F_NOEPI;
+        a3.a[i].flags |= K3F_ACC;
+    }
+    const cudaError_t e = run_mode<1>(s, a1, nslots, d);
+    return e != cudaSuccess ? e : run_mode<3>(s, a3, nslots, d);
+}
+
+}  // namespace fdga

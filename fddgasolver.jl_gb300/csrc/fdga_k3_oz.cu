@@ -39,6 +39,7 @@
 // memory).
 #include <algorithm>
 
+#include "fdga_digits.cuh"
 #include "fdga_kernels.h"
 
 namespace fdga {
@@ -94,10 +95,6 @@ __device__ __forceinline__ void mma_bf16(uint32_t dt, uint64_t a, uint64_t b, ui
         : "r"(dt), "l"(a), "l"(b), "r"(idesc), "r"(acc)
         : "memory");
 }
-// the exponent field of an FP64 value
-__device__ __forceinline__ int efield(double v) {
-    return (int)(((unsigned long long)__double_as_longlong(v) >> 52) & 0x7ffull);
-}
 // |v| in fixed point relative to the bound 2^(F-1022), 56 fractional bits: ⌊|v| 2^(56+1022-F)⌋
 // (0 for zero and subnormal v).  |v| < 2^(F-1022) gives ev ≤ F, so the shift F - ev - 3 is ≥ -3.
 __device__ __forceinline__ unsigned long long fixed56(double v, int F) {
@@ -123,9 +120,6 @@ __device__ __forceinline__ uint32_t bf_pair(uint32_t dlo, uint32_t dhi, uint32_t
 __device__ __forceinline__ uint32_t sbit(double v) {
     return (uint32_t)((unsigned long long)__double_as_longlong(v) >> 63);
 }
-// the larger exponent field of the two parts of a complex number: both |x|, |y| < 2^(E - 1022)
-// (zero and subnormal parts included, with E = 0)
-__device__ __forceinline__ int cexpo(cplx v) { return max(efield(v.x), efield(v.y)); }
 // an FP32 upper bound of |x| from its top 23 significand bits (+1 ulp); 2^-126 below the FP32
 // normal range, +inf above it and for an infinity or NaN
 __device__ __forceinline__ float mag_up(double x) {
@@ -141,20 +135,6 @@ __device__ __forceinline__ void prod_bound(float2 a, float2 b, float2& acc) {
     acc.x = fmaf(a.x, b.x, fmaf(a.y, b.y, acc.x));
     acc.y = fmaf(a.x, b.y, fmaf(a.y, b.x, acc.y));
 }
-// x · 2^e for an integer |x| < 2^53 (exact), built from its bits on the integer pipes; 0 below the
-// normal range
-__device__ __forceinline__ double i2d_scaled(long long x, int e) {
-    if (x == 0) return 0.0;
-    const unsigned long long sg = x < 0 ? (1ull << 63) : 0ull;
-    const unsigned long long u = x < 0 ? (unsigned long long)(-x) : (unsigned long long)x;
-    const int p = 63 - __clzll((long long)u);  // 2^p ≤ u < 2^(p+1), p ≤ 52
-    const int ef = p + e + 1023;
-    if (ef <= 0) return 0.0;
-    if (ef >= 2047) return __longlong_as_double((long long)(sg | 0x7FF0000000000000ull));
-    const unsigned long long mant = (u << (52 - p)) & 0xFFFFFFFFFFFFFull;
-    return __longlong_as_double((long long)(sg | ((unsigned long long)ef << 52) | mant));
-}
-
 // The A digit operands of the blocks r0, r0 + 1, ..: one CTA per block finds F_A, the largest
 // exponent field of the block's entries (both parts; stored in fa_blk for the contraction), then
 // writes, per chunk of 8 ω, S digit operands of the block's N rows in the K-major no-swizzle layout

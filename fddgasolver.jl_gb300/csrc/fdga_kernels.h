@@ -350,6 +350,11 @@ cudaError_t launch_bse_K1_mfrg(cudaStream_t s, const VertP& F, const FLP& FL, co
 cudaError_t launch_bse_K2_mfrg(cudaStream_t s, const VertP& F, const FLP& FL, const BubbleP& B, const ChanWork& cw,
                                const Dims& d);
 cudaError_t launch_scale(cudaStream_t s, cplx* out, const cplx* in, double sc, size_t n);
+// FP64 K3 contractions of small blocks (Nν3 ≤ 32) on warp-level tensor-core products of 8-bit digits
+// (fdga_k3_mma.cu), modes 0, 1 and 2
+bool k3_mma_supported(const Dims& d);
+cudaError_t prepare_bse_K3_mma(const Dims& d);
+cudaError_t launch_bse_K3_mma(cudaStream_t s, int mode, const K3Args3& a, int nslots, const Dims& d);
 // FP64 K3 contractions on the tensor cores by exact BF16 digit slicing (fdga_k3_oz.cu), modes 0, 1
 // and 2 (the tangent); fa_scratch holds nslots x nblocks ints (per-block exponent bounds), adig the
 // A digit operands of adig_blocks blocks (k3_oz_digit_bytes each); ebound = 1 bounds every tile of

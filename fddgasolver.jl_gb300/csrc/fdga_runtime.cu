@@ -610,11 +610,11 @@ cudaError_t launch_k3_tensor_cores(fdga_handle* h, cudaStream_t s, int mode, con
     return launch_bse_K3_tc(s, mode, a3f, 3, h->d, h->d_err);
 }
 
-// The FP64 map's K3 contraction: on the tensor cores by exact BF16 digit slicing when the option is
-// on and the box fits (fdga_k3_oz.cu), else the FP64 CUDA-core GEMM.
-// the FP64 K3 contractions (modes 0, 1 and the tangent's mode 2) on the tensor cores: where the
-// digit-sliced kernel supports the box, and by default from Nν3 = 32 on (below, the CUDA-core
-// kernel is as fast)
+// The FP64 K3 contractions (modes 0, 1 and the tangent's mode 2) by exact digit slicing: on tcgen05
+// (fdga_k3_oz.cu) from Nν3 = 32 on, on warp-level products (fdga_k3_mma.cu) below, where a 128-row
+// accumulator stands mostly empty (Nν3 = 24, Hubbard 8x8: 23 / 37 us against 79 / 97).  The FP64 CUDA-core
+// GEMM runs the rest: Nν3 above 32 that is no multiple of 8 or passes 128, the tangent of the one-loop
+// form, and everything when the option is off.
 bool use_k3_oz(const fdga_handle* h) {
     if (!h->d_err || !h->oz_fa || !h->oz_adig || !k3_oz_supported(h->d)) return false;
     return h->k3_oz == 1 || h->k3_oz == 3 || (h->k3_oz == 2 && h->d.N3n >= 32);
@@ -624,6 +624,7 @@ cudaError_t launch_k3_fp64(fdga_handle* h, cudaStream_t s, int mode, const K3Arg
     for (int i = 0; i < 3; ++i) oneloop |= (a3.a[i].flags & K3F_1LOOP) != 0;
     if (use_k3_oz(h) && (mode <= 1 || !oneloop)) return launch_bse_K3_oz(s, mode, a3, 3, h->d, h->d_err, h->oz_fa, h->oz_adig, h->oz_adig_blocks,
                                                                 h->k3_oz == 3);
+    if (h->k3_oz == 2 && k3_mma_supported(h->d) && (mode <= 1 || !oneloop)) return launch_bse_K3_mma(s, mode, a3, 3, h->d);
     return launch_bse_K3(s, mode, a3, 3, h->d, 0, h->k3_tile[FDGA_FP64][mode < 2 ? mode : 1]);
 }
 
@@ -1908,6 +1909,7 @@ int fdga_finalize(fdga_handle* h) {
         if (int r = ensure_k3_oz(h)) return r;
         CK(prepare_bse_K3_oz());
     }
+    if (k3_mma_supported(d)) CK(prepare_bse_K3_mma(d));
     CK(cudaStreamSynchronize(s));
     h->finalized = true;
     h->c0_dirty = true;
