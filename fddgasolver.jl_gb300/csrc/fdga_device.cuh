@@ -187,6 +187,11 @@ struct VertPT {
     int has0;   // 1: F0 is a Vertex with the channels g0 (box b0) on top of the RefVertex terms
     ChanPT<S> g0[3];
     Box b0;
+    // Table of the irreducible vertex in each channel's representation and BSE spin combination (p and a:
+    // parallel; t: 2 pSp + xSp), Γ_ch(Ω, ν, ω) = the two other channels: with more than one momentum they
+    // enter at their momentum average, so Γ does not depend on P.  [channel][iΩ of the K2 box][iν of the
+    // K2 box][ω + th], ω in [-th, th), th = gamma_half; null: not tabulated (evaluate).
+    const S* tab[3];
 };
 using ChanP = ChanPT<cplx>;
 using VertP = VertPT<cplx>;
@@ -612,6 +617,43 @@ __device__ __forceinline__ S fl_right(const S* FLK2p, const S* FLK2t, const S* F
 }
 
 __device__ __forceinline__ int cross(int ch, int m, int n) { return ch == CH_P ? m - n - 1 : n; }
+
+// half width of the Γ table: Γ(Ω, ν, ω) vanishes for |ω| beyond the K1 windows around ν, -(Ω+ν+1) and
+// Ω-ν-1, and every ω at which a cache or a left BSE reads it lies inside too
+__host__ __device__ __forceinline__ int gamma_half(const Dims& d) { return d.n2O + d.n2n + d.n1 + 2; }
+// row (Ω, ν) of a Γ table, indexed by ω
+template <class S>
+__device__ __forceinline__ const S* gamma_row(const S* tab, const Dims& d, int m, int nu) {
+    const int th = gamma_half(d);
+    return tab + ((size_t)(m + d.n2O - 1) * d.N2n + (nu + d.n2n)) * (2 * th) + th;
+}
+// the part of the K2 vertex difference that is the RefVertex's and the own channel's (k2_vertex_diff
+// less Γ): the correction and K3(Ω,ν,ω), in the spin combination of channel CH
+template <int CH, class S>
+__device__ __forceinline__ S k2_own_diff(const VertPT<S>& F, const Dims& d, int m, int nu, int n, int P, bool in3) {
+    using R = decltype(S::x);
+    S v{0, 0}, r;
+    if constexpr (CH != CH_T) {
+        if (in3) v = k3v(F.g[CH], d, m, nu, n, P);
+        if (!F.noref) {
+            if (CH == CH_A) {
+                if (ref_val(r, F.Ft_x, d, m, n, nu)) v -= r;
+            } else if (ref_val(r, F.Fp_p, d, m, nu, n)) {
+                v += r;
+            }
+        }
+    } else {
+        if (in3) {
+            const S t = k3v(F.g[CH_T], d, m, nu, n, P), a = k3v(F.g[CH_A], d, m, nu, n, P);
+            v = S{fma(t.x, (R)2, -a.x), fma(t.y, (R)2, -a.y)};
+        }
+        if (!F.noref) {  // 2 Ft_p - (-Ft_x)
+            if (ref_val(r, F.Ft_p, d, m, nu, n)) v = S{fma(r.x, (R)2, v.x), fma(r.y, (R)2, v.y)};
+            if (ref_val(r, F.Ft_x, d, m, n, nu)) v += r;
+        }
+    }
+    return v;
+}
 
 // A union of at most 6 closed ω intervals, merged and ordered; used to visit only the bubble
 // frequencies at which a vertex factor differs from its ω-independent value.

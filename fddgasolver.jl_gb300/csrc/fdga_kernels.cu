@@ -525,6 +525,75 @@ __global__ void k_build_cache(VertPT<S> Fin, Caches C, const int* blocks, int nb
 }
 
 // ---------------------------------------------------------------------------------------------
+// Γ table of the nonlocal solver (VertPT::tab): the two other channels at their momentum averages, once
+// per (Ω, ν, ω) for the K2 BSEs and the caches of every P.  Bound by the FP64 pipe (up to 8 complex
+// additions per channel and entry), as the evaluations were that it replaces; those ran once per P.
+// blockIdx.y = position in the list of the Ω that any K2 or K3 work item has.
+// Stage times on GB300 without -> with the table (its launch is in the cache stage), caches / left K2 /
+// K2 in us: Hubbard 8x8, nK3 = (8, 12) 45 / 48 / 112 -> 29 / 29 / 62; 8x8, nK3 = (20, 40) 915 / 386 / 829
+// -> 273 / 151 / 375; 5x5 without groups, nK3 = (5, 7) 23 / 69 / 141 -> 23 / 37 / 68.  The local solver
+// (one momentum) has nothing to share and evaluates in place, as does a Vertex-valued F0, whose own
+// channel depends on P.
+// ---------------------------------------------------------------------------------------------
+template <class S>
+__global__ void __launch_bounds__(256) k_gamma_table(VertPT<S> F, S* tp, S* tt, S* ta, const int* oms, Dims d) {
+    using R = decltype(S::x);
+    const int th = gamma_half(d), NT = 2 * th;
+    const int e = blockIdx.x * 256 + threadIdx.x;
+    if (e >= d.N2n * NT) return;
+    const int iO = oms ? oms[blockIdx.y] : blockIdx.y;
+    const int m = iO - (d.n2O - 1), nu = e / NT - d.n2n, n = e % NT - th;
+    const size_t i = (size_t)iO * d.N2n * NT + e;
+    // (the unused slots of F.noref and has0 do not enter: no F0 flag)
+    tp[i] = vert_pSp(F, d, CH_P, m, nu, n, KAVG, FL_GT | FL_GA);
+    const S a = vert_pSp(F, d, CH_A, m, nu, n, KAVG, FL_GP | FL_GT);
+    const S t = vert_pSp(F, d, CH_T, m, nu, n, KAVG, FL_GP | FL_GA);
+    ta[i] = a;
+    tt[i] = S{fma(t.x, (R)2, -a.x), fma(t.y, (R)2, -a.y)};  // xSp(t) = -pSp(a)
+}
+// K3 caches (see k_build_cache) from the Γ table.  The right caches in reduced form: with F0 and the own
+// channel, F(Ω,ν,ω) - F(Ω,∞,ω) leaves the RefVertex correction, the own K2(ν) and the own K3.
+template <class S>
+__global__ void __launch_bounds__(256) k_build_cache_tab(VertPT<S> F, Caches C, const int* blocks, int nblocks,
+                                                         Dims d) {
+    using R = decltype(S::x);
+    const size_t bs = (size_t)d.N3n * d.N3n;
+    const size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+    if (t >= (size_t)nblocks * bs) return;
+    const int bl = blocks ? blocks[t / bs] : (int)(t / bs);  // block = P * NΩ3 + iΩ
+    const size_t e = t % bs;
+    const size_t i = (size_t)bl * bs + e;
+    const int b = (int)(e % d.N3n) - d.n3n, a = (int)(e / d.N3n) - d.n3n;
+    const int m = bl % d.N3O - (d.n3O - 1), P = bl / d.N3O;
+    const S* rp = gamma_row(F.tab[CH_P], d, m, a);
+    const S gpp = ldv(rp + b), gpx = -ldv(rp + (m - b - 1));
+    const S ga = ldv(gamma_row(F.tab[CH_A], d, m, a) + b), gt = ldv(gamma_row(F.tab[CH_T], d, m, a) + b);
+    auto own = [&](int ch) { return k2v(F.g[ch], d, m, a, P) + k3v(F.g[ch], d, m, a, b, P); };
+    S fp = own(CH_P), fa = own(CH_A), ft = own(CH_T);
+    S f0p{0, 0}, f0a{0, 0}, f0t{0, 0}, r;
+    if (!F.noref) {
+        f0p = ref_call(F.Fp_x, d, m, a, b);
+        f0t = ref_call(F.Ft_p, d, m, a, b);
+        f0a = -ref_call(F.Ft_x, d, m, b, a);
+        if (ref_val(r, F.Fp_p, d, m, a, b)) fp += r;
+        fa += f0a;
+        ft += f0t;
+        f0t = S{fma(f0t.x, (R)2, -f0a.x), fma(f0t.y, (R)2, -f0a.y)};
+    }
+    const S v[10] = {gpx, f0p, f0a, f0t, gpp, ga, gt, fp + gpp, fa + ga,
+                     S{fma(ft.x, (R)2, -fa.x), fma(ft.y, (R)2, -fa.y)} + gt};
+    if (C.f[0]) {
+#pragma unroll
+        for (int k = 0; k < 10; ++k)
+            if (C.f[k]) C.f[k][i] = to_f32(v[k]);
+    } else {
+#pragma unroll
+        for (int k = 0; k < 10; ++k)
+            if (C.c[k]) st16(C.c[k] + i, to_d(v[k]));
+    }
+}
+
+// ---------------------------------------------------------------------------------------------
 // Bubble row sums SΠ(P, Ω) = Σ_ν Π(P, Ω, ν) over the whole bubble mesh; blockIdx.y = array.
 // ---------------------------------------------------------------------------------------------
 __global__ void k_rowsum(const cplx* A0, const cplx* A1, cplx* S0, cplx* S1, int rowlen) {
@@ -794,10 +863,17 @@ __device__ __forceinline__ void bse_L_K2_body(const VertPT<S>& F, const cplx* Pi
         return;
     }
     if (d.local) {
-        for (int n = -d.nPw + lane; n < d.nPw; n += 32) {  // local solver: nPw = nPn
+        // Γ vanishes beyond the K1 windows around ν, -(Ω+ν+1) and Ω-ν-1: the sum over the whole bubble
+        // mesh (nPw = nPn) has terms only within gamma_half
+        const int w = min(d.nPw, gamma_half(d));
+        for (int n = -w + lane; n < w; n += 32) {
             const S Gp = vert_eval(F, d, CH, SP, m, nu, n, P, IRR);
             acc = cfma(Gp, to_c<S>(ldg(Pi0 + ixPi(d, P, m, n))), acc);
         }
+    } else if (F.tab[CH]) {
+        const S* row = gamma_row(F.tab[CH], d, m, nu);
+        for (int n = -d.n2n + lane; n < d.n2n; n += 32)
+            acc = cfma(ldv(row + cross(CH, m, n)), to_c<S>(ldg(Pi0 + ixPi(d, P, m, n))), acc);
     } else {
         for (int n = -d.n2n + lane; n < d.n2n; n += 32) {
             const S Gl = vert_eval(F, d, CH, SP, m, nu, cross(CH, m, n), P, IRR);
@@ -829,7 +905,10 @@ __host__ __device__ __forceinline__ int k2_table_half(const Dims& d) {
     const int W = d.xn2O + d.xn2n + d.xn1 + d.nRn + 2;  // (extents over F and a Vertex-valued F0)
     return W < d.nPw ? W : d.nPw;
 }
-template <int CH, class S, bool TAN>
+// TAB: Γ from the table of the nonlocal solver (F.tab; T.F.tab for the tangent vertex), read along ω, so
+// that a term costs its product and the own K3 only.  The ω range is then the hull of the windows (Γ is
+// zero in their gaps).
+template <int CH, class S, bool TAN, bool TAB>
 __device__ __forceinline__ void bse_K2_row(const VertPT<S>& F, const FLPT<S>& FL, const cplx* Pi, const cplx* Pi0,
                                            const cplx* SX, cplx* out, const int* items, const int* gstart,
                                            int ngroups, int accum, const Dims& d, const TanArgsT<S>& T, S* tab) {
@@ -869,6 +948,28 @@ __device__ __forceinline__ void bse_K2_row(const VertPT<S>& F, const FLPT<S>& FL
         const S c = k2_c<CH>(F, d, m, nu, P);
         S tc{0, 0};
         if constexpr (TAN) tc = k2_c<CH>(T.F, d, m, nu, P);
+        S acc{0, 0};
+        if constexpr (TAB) {
+            const int c2 = -(m + nu + 1), c3 = (CH == CH_P) ? m - nu - 1 : nu, hb = max(d.n2n, d.nRn);
+            const int n0 = max(min(min(-hb, nu - h1), min(c2, c3) - h1), lo);
+            const int n1 = min(max(max(hb - 1, nu + h1), max(c2, c3) + h1), hi);
+            const S* row = gamma_row(F.tab[CH], d, m, nu);
+            const S* trow = TAN ? gamma_row(T.F.tab[CH], d, m, nu) : nullptr;
+            const bool r3 = bin(m, d.n3O) && fin(nu, d.n3n);
+            const int th = gamma_half(d);
+            for (int n = n0 + lane; n <= n1; n += 32) {
+                const bool in3 = r3 && fin(n, d.n3n), inr = fin(n, d.nRn), int_ = fin(n, th);
+                S Fl = int_ ? ldv(row + n) : S{0, 0};
+                if (in3 || inr) Fl += k2_own_diff<CH>(F, d, m, nu, n, P, in3);
+                if constexpr (!TAN) {
+                    acc = cfma(Fl, Xt[n + half], acc);
+                } else {
+                    S tFl = int_ ? ldv(trow + n) : S{0, 0};
+                    if (in3) tFl += k2_own_diff<CH>(T.F, d, m, nu, n, P, true);
+                    acc = cfma(tFl, Xt[n + half], cfma(Fl, tXt[n + half], acc));
+                }
+            }
+        } else {
         Windows win;
         win.add(-d.xn2n, d.xn2n - 1, lo, hi);
         win.add(-d.nRn, d.nRn - 1, lo, hi);
@@ -876,7 +977,6 @@ __device__ __forceinline__ void bse_K2_row(const VertPT<S>& F, const FLPT<S>& FL
         win.add(-(m + nu + 1) - h1, -(m + nu + 1) + h1, lo, hi);
         if (CH == CH_P) win.add(m - nu - 1 - h1, m - nu - 1 + h1, lo, hi);
         win.merge();
-        S acc{0, 0};
         for (int t = lane; t < win.total; t += 32) {
             const int n = win.at(t);
             const int j = n + half;
@@ -888,6 +988,7 @@ __device__ __forceinline__ void bse_K2_row(const VertPT<S>& F, const FLPT<S>& FL
                 k2_vertex_diff2<CH>(F, T.F, d, m, nu, n, P, Fl, tFl);
                 acc = cfma(tFl, Xt[j], cfma(Fl, tXt[j], acc));
             }
+        }
         }
         acc = warp_sum(acc);
         if (lane == 0) {
@@ -1325,7 +1426,7 @@ __global__ void k_bse_L_K2_all(VertPT<S> Fin, BubbleP B, ChanWork cw, Dims d) {
         default:   bse_L_K2_body<CH_A>(F, B.ph0, cw.out[CH_A], cw.items[CH_A], cw.nitems[CH_A], d); break;
     }
 }
-template <class S, bool TAN, bool V0>
+template <class S, bool TAN, bool V0, bool TAB>
 __global__ void __launch_bounds__(512) k_bse_K2_all(VertPT<S> Fin, FLPT<S> FL, BubbleP B, const cplx* SX, ChanWork cw,
                                                     Dims d, TanArgsT<S> Tin) {
     const VertPT<S> F = vert_spec<V0>(Fin);
@@ -1333,9 +1434,9 @@ __global__ void __launch_bounds__(512) k_bse_K2_all(VertPT<S> Fin, FLPT<S> FL, B
     extern __shared__ __align__(16) unsigned char k2_smem[];
     S* tab = reinterpret_cast<S*>(k2_smem);
     switch (blockIdx.y) {
-        case CH_P: bse_K2_row<CH_P, S, TAN>(F, FL, B.pp, B.pp0, SX, cw.out[CH_P], cw.items[CH_P], cw.gstart[CH_P], cw.ngroups[CH_P], cw.acc, d, T, tab); break;
-        case CH_T: bse_K2_row<CH_T, S, TAN>(F, FL, B.ph, B.ph0, SX, cw.out[CH_T], cw.items[CH_T], cw.gstart[CH_T], cw.ngroups[CH_T], cw.acc, d, T, tab); break;
-        default:   bse_K2_row<CH_A, S, TAN>(F, FL, B.ph, B.ph0, SX, cw.out[CH_A], cw.items[CH_A], cw.gstart[CH_A], cw.ngroups[CH_A], cw.acc, d, T, tab); break;
+        case CH_P: bse_K2_row<CH_P, S, TAN, TAB>(F, FL, B.pp, B.pp0, SX, cw.out[CH_P], cw.items[CH_P], cw.gstart[CH_P], cw.ngroups[CH_P], cw.acc, d, T, tab); break;
+        case CH_T: bse_K2_row<CH_T, S, TAN, TAB>(F, FL, B.ph, B.ph0, SX, cw.out[CH_T], cw.items[CH_T], cw.gstart[CH_T], cw.ngroups[CH_T], cw.acc, d, T, tab); break;
+        default:   bse_K2_row<CH_A, S, TAN, TAB>(F, FL, B.ph, B.ph0, SX, cw.out[CH_A], cw.items[CH_A], cw.gstart[CH_A], cw.ngroups[CH_A], cw.acc, d, T, tab); break;
     }
 }
 template <class S, bool TAN, bool V0>
@@ -1778,9 +1879,26 @@ cudaError_t launch_qavg(cudaStream_t s, const ChanArrays& in, const ChanArraysW&
     LAUNCH_CHECK(); return cudaSuccess;
 }
 template <class S>
+static cudaError_t gamma_table_t(cudaStream_t s, const VertPT<S>& F, S* tab, const int* oms, int noms, const Dims& d) {
+    const size_t per = gamma_table_len(d) / 3;
+    const dim3 g(blocks_for((size_t)d.N2n * 2 * gamma_half(d), 256), (unsigned)noms);
+    k_gamma_table<S><<<g, 256, 0, s>>>(F, tab, tab + per, tab + 2 * per, oms, d);
+    LAUNCH_CHECK(); return cudaSuccess;
+}
+cudaError_t launch_gamma_table(cudaStream_t s, const VertP& F, cplx* tab, const int* oms, int noms, const Dims& d) {
+    return gamma_table_t(s, F, tab, oms, noms, d);
+}
+cudaError_t launch_gamma_table(cudaStream_t s, const VertPF& F, cplxf* tab, const int* oms, int noms, const Dims& d) {
+    return gamma_table_t(s, F, tab, oms, noms, d);
+}
+template <class S>
 static cudaError_t build_cache_t(cudaStream_t s, const VertPT<S>& F, const Caches& C, const int* blocks, int nblocks,
                                  const Dims& d) {
     const size_t n = (size_t)nblocks * d.N3n * d.N3n;
+    if (F.tab[0]) {
+        k_build_cache_tab<S><<<blocks_for(n, 256), 256, 0, s>>>(F, C, blocks, nblocks, d);
+        LAUNCH_CHECK(); return cudaSuccess;
+    }
     if (F.has0) k_build_cache<S, true><<<blocks_for(n, 128), 128, 0, s>>>(F, C, blocks, nblocks, d);
     else k_build_cache<S, false><<<blocks_for(n, 128), 128, 0, s>>>(F, C, blocks, nblocks, d);
     LAUNCH_CHECK(); return cudaSuccess;
@@ -1819,8 +1937,8 @@ static unsigned warp_grid(const ChanWork& cw, int nch) {
 }
 // each vertex-evaluating kernel is launched in its V0 = F.has0 instantiation (see vert_spec)
 template <class K>
-static cudaError_t k2_launch_attr(K k_plain, K k_v0, bool v0, size_t smem) {
-    return k2_smem_attr(v0 ? k_v0 : k_plain, smem);
+static cudaError_t k2_launch_attr(K k_plain, K k_v0, K k_tab, bool v0, bool tab, size_t smem) {
+    return k2_smem_attr(tab ? k_tab : (v0 ? k_v0 : k_plain), smem);
 }
 #define FDGA_VERTEX_LAUNCHERS(VT, FT, TT, ST)                                                                       \
     cudaError_t launch_bse_K1_all(cudaStream_t s, const VT& F, const FT& FL, const BubbleP& B, const cplx* SX,    \
@@ -1840,11 +1958,13 @@ static cudaError_t k2_launch_attr(K k_plain, K k_v0, bool v0, size_t smem) {
     cudaError_t launch_bse_K2_all(cudaStream_t s, const VT& F, const FT& FL, const BubbleP& B, const cplx* SX,    \
                                   const ChanWork& cw, const Dims& d) {                                             \
         const size_t smem = k2_row_smem<ST, false>(d);                                                             \
-        cudaError_t e = k2_launch_attr(k_bse_K2_all<ST, false, false>, k_bse_K2_all<ST, false, true>, F.has0, smem); \
+        cudaError_t e = k2_launch_attr(k_bse_K2_all<ST, false, false, false>, k_bse_K2_all<ST, false, true, false>,     \
+                                       k_bse_K2_all<ST, false, false, true>, F.has0, F.tab[0] != nullptr, smem); \
         if (e != cudaSuccess) return e;                                                                             \
         const dim3 g(row_grid(cw, 3), 3);                                                                           \
-        if (F.has0) k_bse_K2_all<ST, false, true><<<g, row_threads(cw, 3), smem, s>>>(F, FL, B, SX, cw, d, TT{});   \
-        else k_bse_K2_all<ST, false, false><<<g, row_threads(cw, 3), smem, s>>>(F, FL, B, SX, cw, d, TT{});         \
+        if (F.tab[0]) k_bse_K2_all<ST, false, false, true><<<g, row_threads(cw, 3), smem, s>>>(F, FL, B, SX, cw, d, TT{}); \
+        else if (F.has0) k_bse_K2_all<ST, false, true, false><<<g, row_threads(cw, 3), smem, s>>>(F, FL, B, SX, cw, d, TT{});    \
+        else k_bse_K2_all<ST, false, false, false><<<g, row_threads(cw, 3), smem, s>>>(F, FL, B, SX, cw, d, TT{});         \
         LAUNCH_CHECK(); return cudaSuccess;                                                                         \
     }                                                                                                               \
     cudaError_t launch_sde_L_all(cudaStream_t s, const VT& F, const BubbleP& B, const cplx* SPpp, const cplx* SPph, \
@@ -1864,11 +1984,13 @@ static cudaError_t k2_launch_attr(K k_plain, K k_v0, bool v0, size_t smem) {
     cudaError_t launch_bse_K2_tan(cudaStream_t s, const VT& F, const FT& FL, const BubbleP& B, const cplx* SX,    \
                                   const TT& T, const ChanWork& cw, const Dims& d) {                                \
         const size_t smem = k2_row_smem<ST, true>(d);                                                              \
-        cudaError_t e = k2_launch_attr(k_bse_K2_all<ST, true, false>, k_bse_K2_all<ST, true, true>, F.has0, smem);  \
+        cudaError_t e = k2_launch_attr(k_bse_K2_all<ST, true, false, false>, k_bse_K2_all<ST, true, true, false>,     \
+                                       k_bse_K2_all<ST, true, false, true>, F.has0, F.tab[0] != nullptr, smem);  \
         if (e != cudaSuccess) return e;                                                                             \
         const dim3 g(row_grid(cw, 3), 3);                                                                           \
-        if (F.has0) k_bse_K2_all<ST, true, true><<<g, row_threads(cw, 3), smem, s>>>(F, FL, B, SX, cw, d, T);       \
-        else k_bse_K2_all<ST, true, false><<<g, row_threads(cw, 3), smem, s>>>(F, FL, B, SX, cw, d, T);             \
+        if (F.tab[0]) k_bse_K2_all<ST, true, false, true><<<g, row_threads(cw, 3), smem, s>>>(F, FL, B, SX, cw, d, T); \
+        else if (F.has0) k_bse_K2_all<ST, true, true, false><<<g, row_threads(cw, 3), smem, s>>>(F, FL, B, SX, cw, d, T);        \
+        else k_bse_K2_all<ST, true, false, false><<<g, row_threads(cw, 3), smem, s>>>(F, FL, B, SX, cw, d, T);             \
         LAUNCH_CHECK(); return cudaSuccess;                                                                         \
     }                                                                                                               \
     cudaError_t launch_sde_L_tan(cudaStream_t s, const VT& F, const BubbleP& B, const cplx* SPpp, const cplx* SPph, \

@@ -221,6 +221,10 @@ cudaError_t launch_sde_L_all(cudaStream_t s, const VertPF& F, const BubbleP& B, 
                              const ChanWork& cw, int use_vertex, double ref_scale, const Dims& d);
 cudaError_t launch_build_cache(cudaStream_t s, const VertPF& F, const Caches& C, const int* blocks, int nblocks,
                                const Dims& d);
+// Γ table of the vertex F (VertPT::tab) at the listed Ω (nullptr: all); gamma_table_len values
+inline size_t gamma_table_len(const Dims& d) { return (size_t)3 * d.N2O * d.N2n * 2 * gamma_half(d); }
+cudaError_t launch_gamma_table(cudaStream_t s, const VertP& F, cplx* tab, const int* oms, int noms, const Dims& d);
+cudaError_t launch_gamma_table(cudaStream_t s, const VertPF& F, cplxf* tab, const int* oms, int noms, const Dims& d);
 // K1 and K2 of the :fdPA_new / :scPA_new strategies (local solver); SPi, SPi0: full-mesh row sums [2][Nq][NΠΩ]
 cudaError_t launch_bse_K1_new(cudaStream_t s, const VertP& F, const BubbleP& B, const cplx* SPi, const cplx* SPi0,
                               const ChanWork& cw, const Dims& d);

@@ -102,6 +102,12 @@ struct fdga_handle {
     size_t flush_bytes = 0;
     unsigned char flush_val = 0;
     int nk3blocks = 0;
+    // Γ table (VertPT::tab; nonlocal solvers with a RefVertex) and its FP32 form, and the Ω (of the K2 box)
+    // that any K2 or K3 work item has (nullptr: all)
+    cplx* gtab = nullptr;
+    cplxf* gtabf = nullptr;
+    int* d_goms = nullptr;
+    int ngoms = 0;
     double* occ = nullptr;
     double n0 = 0.5;
     uint32_t* perm = nullptr;  // reference flatten index -> device index
@@ -158,6 +164,8 @@ struct fdga_handle {
         cplx *x = nullptr, *y = nullptr, *avg = nullptr, *G = nullptr, *GR = nullptr;
         cplx *Pipp = nullptr, *Piph = nullptr, *SPi = nullptr, *SX = nullptr;
         cplx *cache = nullptr;  // 7 caches (Γpx Γpp Γa Γt Fp Fa Ft): the RefVertex caches have no tangent
+        cplx* gtab = nullptr;   // Γ table of the tangent vertex
+        cplxf* gtabf = nullptr;
         cplx *FLK2 = nullptr, *FLK3 = nullptr, *Lpp = nullptr, *Lph = nullptr, *LR = nullptr, *SR = nullptr;
         cplx *SigIn = nullptr, *u2C = nullptr, *u2R = nullptr, *SigU2 = nullptr;
         double* occ = nullptr;
@@ -240,6 +248,7 @@ int ensure_mixed(fdga_handle* h) {
         CK(launch_to_f32(h->st, h->F0v, h->F0vf, 3 * h->n0chan));
         if (h->n0avg) CK(launch_to_f32(h->st, h->F0avg, h->F0avgf, h->n0avg));
     }
+    if (h->gtab) AL(h->gtabf, gamma_table_len(h->d));
     AL(h->d_err, 1);
     if (k3_tc_supported(h->d)) CK(prepare_bse_K3_tc(h->d));
     CK(prepare_bse_K3_tma(h->d));
@@ -553,6 +562,12 @@ VertPT<S> vertex_view_t(const fdga_handle* h, S* st, S* avg, S* const* fref) {
     return F;
 }
 VertP vertex_view(fdga_handle* h, cplx* S) { return vertex_view_t<cplx>(h, S, h->avg, h->Fref); }
+// attaches a Γ table to a vertex view
+template <class S>
+void set_table(const fdga_handle* h, VertPT<S>& F, S* tab) {
+    const size_t per = gamma_table_len(h->d) / 3;
+    for (int c = 0; c < 3; ++c) F.tab[c] = tab ? tab + c * per : nullptr;
+}
 
 const Group& k2group(fdga_handle* h, int ch) { return ch == CH_P ? h->gK2pp : h->gK2ph; }
 // the (P, Ω) rows of the K2 work of channel ch (the K2 BSE kernel runs one CTA per row)
@@ -706,6 +721,12 @@ int enqueue_iteration(fdga_handle* h, int strategy, bool update_sigma, bool hart
     for (int i = 0; i < 10; ++i) {
         C.c[i] = h->cache + (size_t)i * h->n3;
         C.f[i] = mixed ? h->cachef + (size_t)i * h->n3 : nullptr;
+    }
+    if (h->gtab) {
+        if (mixed) LC(launch_gamma_table(s, Ff, h->gtabf, h->d_goms, h->ngoms, d));
+        else LC(launch_gamma_table(s, F, h->gtab, h->d_goms, h->ngoms, d));
+        set_table(h, F, h->gtab);
+        set_table(h, Ff, h->gtabf);
     }
     if (mixed) LC(launch_build_cache(s, Ff, C, h->d_k3blocks, h->nk3blocks, d));
     else LC(launch_build_cache(s, F, C, h->d_k3blocks, h->nk3blocks, d));
@@ -930,10 +951,14 @@ int ensure_tangent(fdga_handle* h) {
         AL(t.SigIn, h->nGk); AL(t.u2C, (size_t)d.Nq * (2 * d.NG - 1)); AL(t.u2R, h->nGk); AL(t.SigU2, h->nGk);
         AL(t.occ, 1);
     }
-    if (!mixed && !t.cache) AL(t.cache, 7 * h->n3);
+    if (!mixed && !t.cache) {
+        AL(t.cache, 7 * h->n3);
+        if (h->gtab) AL(t.gtab, gamma_table_len(d));
+    }
     if (mixed && !t.cachef) {
         int r = ensure_mixed(h);
         if (r) return r;
+        if (h->gtab) AL(t.gtabf, gamma_table_len(d));
         AL(t.cachef, 7 * h->n3);
         AL(t.FLK2f, 3 * h->n2); AL(t.FLK3f, 3 * h->n3);
         AL(t.xSf, 3 * h->nchan); AL(t.ySf, 3 * h->nchan);
@@ -1021,6 +1046,14 @@ int enqueue_tangent(fdga_handle* h, int strategy, bool update_sigma, bool hartre
         C.f[i] = mixed ? h->cachef + (size_t)i * h->n3 : nullptr;
         tC.c[i] = (slot[i] < 0 || mixed) ? nullptr : t.cache + (size_t)slot[i] * h->n3;
         tC.f[i] = (slot[i] < 0 || !mixed) ? nullptr : t.cachef + (size_t)slot[i] * h->n3;
+    }
+    if (h->gtab) {  // (the value table is the value pass's)
+        if (mixed) LC(launch_gamma_table(s, tFf, t.gtabf, h->d_goms, h->ngoms, d));
+        else LC(launch_gamma_table(s, tF, t.gtab, h->d_goms, h->ngoms, d));
+        set_table(h, F, h->gtab);
+        set_table(h, Ff, h->gtabf);
+        set_table(h, tF, t.gtab);
+        set_table(h, tFf, t.gtabf);
     }
     if (mixed) LC(launch_build_cache(s, tFf, tC, h->d_k3blocks, h->nk3blocks, d));
     else LC(launch_build_cache(s, tF, tC, h->d_k3blocks, h->nk3blocks, d));
@@ -1805,6 +1838,8 @@ int fdga_create(const fdga_config* c, fdga_handle** out) {
     ALC(h->LR, 2 * h->n2); ALC(h->SigR, h->nGk);
     ALC(h->raw1, 3 * h->n1); ALC(h->raw2, 3 * h->n2); ALC(h->raw3, 3 * h->n3);
     h->nk3blocks = d.Nq * d.N3O;
+    if (d.Nq > 1 && !h->has0) ALC(h->gtab, gamma_table_len(d));
+    h->ngoms = d.N2O;
     ALC(h->occ, 1);
     ALC(h->perm, h->nstate);
     ALC(h->d_part, NBLK_RED);
@@ -2010,6 +2045,18 @@ int fdga_init_sym_grp(fdga_handle* h) {
         CK(cudaMemcpyAsync(h->d_k3blocks, blocks.data(), blocks.size() * sizeof(int), cudaMemcpyHostToDevice, h->st));
         CK(cudaStreamSynchronize(h->st));
         h->nk3blocks = (int)blocks.size();
+        // the Ω of the Γ table: those of the K2 representatives and of the K3 blocks
+        std::vector<char> om(h->d.N2O, 0);
+        for (int i = 2; i < 4; ++i)
+            for (int r : hg[i].items) om[(r / h->d.N2n) % h->d.N2O] = 1;
+        for (int b : blocks) om[b % h->d.N3O - (h->d.n3O - 1) + h->d.n2O - 1] = 1;
+        std::vector<int> oms;
+        for (int i = 0; i < h->d.N2O; ++i)
+            if (om[i]) oms.push_back(i);
+        if (!h->d_goms) AL(h->d_goms, (size_t)h->d.N2O);
+        CK(cudaMemcpyAsync(h->d_goms, oms.data(), oms.size() * sizeof(int), cudaMemcpyHostToDevice, h->st));
+        CK(cudaStreamSynchronize(h->st));
+        h->ngoms = (int)oms.size();
     }
     drop_graphs(h);
     h->c0_dirty = true;
@@ -2634,6 +2681,7 @@ int mixed_tangent_base_from_fp64(fdga_handle* h) {
     CK(launch_to_f32(s, h->FLK2, h->FLK2f, 3 * h->n2));
     CK(launch_to_f32(s, h->FLK3, h->FLK3f, 3 * h->n3));
     CK(launch_to_f32(s, h->cache, h->cachef, 10 * h->n3));
+    if (h->gtab) CK(launch_to_f32(s, h->gtab, h->gtabf, gamma_table_len(h->d)));
     return FDGA_OK;
 }
 
