@@ -438,6 +438,87 @@ __device__ void adj_K2_body(const VertP& F, const FLP& FL, const cplx* Pi, const
         }
     }
 }
+// The same with the Γ table (nonlocal solver with a RefVertex): one CTA per (P, Ω) row of representatives,
+// one ω per thread.  The cotangents of Π(ω) and FL(ω) are summed over the row's ν in registers and added
+// once; the cotangent of Γ(Ω, ν, ω) goes to one table element, shared by every P, instead of the up to
+// eight elements of the two other channels (k_adj_gamma_table carries the sum there).  The atomics bound
+// the evaluation in place.  Hubbard 8x8, nK3 = (8, 12) on GB300, in place -> with the table: K2 653 -> 56 us;
+// left K2 338 us and caches 311 us -> 25 (caches) + 32 us (k_adj_gamma_table) + the left K2's one atomic per
+// term.
+template <int CH>
+__device__ void adj_K2_row(const VertP& F, const FLP& FL, const cplx* Pi, const cplx* Pi0, const cplx* SX,
+                           const VertBar& Fb, const FLBar& FLb, cplx* tabbar, cplx* Pibar, cplx* SXbar,
+                           const cplx* rawbar, const int* items, const int* gstart, int ngroups, const Dims& d,
+                           cplx* ss, int* sn) {
+    const int g = blockIdx.x;
+    if (g >= ngroups) return;
+    const int i0 = gstart ? gstart[g] : g * d.N2n, i1 = gstart ? gstart[g + 1] : (g + 1) * d.N2n;
+    const int first = items ? items[i0] : i0;
+    const int m = (first / d.N2n) % d.N2O - (d.n2O - 1), P = first / (d.N2n * d.N2O);
+    const size_t is = (size_t)CH * d.Nq * d.NPO + (size_t)P * d.NPO + (m + d.nPO - 1);
+    const int cnt = i1 - i0;
+    for (int j = threadIdx.x; j < cnt; j += blockDim.x) {
+        const int idx = items ? items[i0 + j] : i0 + j;
+        const int nu = idx % d.N2n - d.n2n;
+        const cplx s = rawbar[idx] * (d.T * (CH == CH_T ? -1.0 : 1.0));
+        ss[j] = s;
+        sn[j] = nu;
+        const cplx c = k2_c<CH>(F, d, m, nu, P);
+        aadd(SXbar + is, cmulc(c, s));
+        const cplx cb = cmulc(SX[is], s);
+        if (CH != CH_T) {
+            k2a(Fb.g[CH], d, m, nu, P, cb);
+        } else {
+            k2a(Fb.g[CH_T], d, m, nu, P, cb * 2.0);
+            k2a(Fb.g[CH_A], d, m, nu, P, cb * -1.0);
+        }
+    }
+    __syncthreads();
+    const int half = k2_table_half(d), th = gamma_half(d);
+    for (int n = -half + (int)threadIdx.x; n < half; n += blockDim.x) {
+        const int wt = cross(CH, m, n);
+        const cplx FLr = fl_right(FL.K2[CH_P], FL.K2[CH_T], FL.K2[CH_A], d, CH, m, wt, P);
+        const size_t ip = ixPi(d, P, m, n);
+        const cplx pi = ldg(Pi + ip), pi0 = ldg(Pi0 + ip);
+        const cplx X = cfma(pi, FLr, (pi - pi0) * d.U);
+        cplx Xb = mk(0, 0);
+        const bool int_ = fin(n, th), n3 = bin(m, d.n3O) && fin(n, d.n3n), inr = fin(n, d.nRn);
+        for (int j = 0; j < cnt; ++j) {
+            const int nu = sn[j];
+            int n0, n1;
+            k2_hull<CH>(d, m, nu, n0, n1);
+            if (n < n0 || n > n1) continue;
+            const cplx s = ss[j];
+            const bool in3 = n3 && fin(nu, d.n3n);
+            cplx D = int_ ? ldg(gamma_row(F.tab[CH], d, m, nu) + n) : mk(0, 0);
+            if (in3 || inr) D += k2_own_diff<CH>(F, d, m, nu, n, P, in3);
+            Xb = cfmac(D, s, Xb);
+            const cplx Db = cmulc(X, s);
+            if (int_) aadd(const_cast<cplx*>(gamma_row<cplx>(tabbar, d, m, nu)) + n, Db);
+            if (in3) {
+                if (CH != CH_T) {
+                    k3a(Fb.g[CH], d, m, nu, n, P, Db);
+                } else {
+                    k3a(Fb.g[CH_T], d, m, nu, n, P, Db * 2.0);
+                    k3a(Fb.g[CH_A], d, m, nu, n, P, Db * -1.0);
+                }
+            }
+        }
+        aadd(Pibar + ip, cmulc(FLr + mk(d.U, 0), Xb));
+        fl_right_adj(FLb, d, CH, m, wt, P, cmulc(pi, Xb));
+    }
+}
+__global__ void k_adj_K2_rows(VertP F, FLP FL, BubbleP B, const cplx* SX, VertBar Fb, FLBar FLb, Ptr3 tb, cplx* Pbpp,
+                              cplx* Pbph, cplx* SXbar, const cplx* rawbar, ChanWork cw, size_t n2, Dims d) {
+    extern __shared__ __align__(16) unsigned char sh_rows[];
+    cplx* ss = reinterpret_cast<cplx*>(sh_rows);
+    int* sn = reinterpret_cast<int*>(ss + d.N2n);
+    switch (blockIdx.y) {
+        case CH_P: adj_K2_row<CH_P>(F, FL, B.pp, B.pp0, SX, Fb, FLb, tb.p[CH_P], Pbpp, SXbar, rawbar, cw.items[CH_P], cw.gstart[CH_P], cw.ngroups[CH_P], d, ss, sn); break;
+        case CH_T: adj_K2_row<CH_T>(F, FL, B.ph, B.ph0, SX, Fb, FLb, tb.p[CH_T], Pbph, SXbar, rawbar + n2, cw.items[CH_T], cw.gstart[CH_T], cw.ngroups[CH_T], d, ss, sn); break;
+        default:   adj_K2_row<CH_A>(F, FL, B.ph, B.ph0, SX, Fb, FLb, tb.p[CH_A], Pbph, SXbar, rawbar + 2 * n2, cw.items[CH_A], cw.gstart[CH_A], cw.ngroups[CH_A], d, ss, sn); break;
+    }
+}
 __global__ void k_adj_K1(VertP F, FLP FL, BubbleP B, const cplx* SX, VertBar Fb, FLBar FLb, cplx* Pbpp, cplx* Pbph,
                          cplx* SXbar, const cplx* rawbar, ChanWork cw, size_t n1, Dims d) {
     switch (blockIdx.y) {
@@ -512,6 +593,66 @@ __global__ void k_adj_L_K2(BubbleP B, VertBar Fb, const cplx* rawbar, ChanWork c
     }
 }
 
+// the same into the table's cotangent: warp per item, lanes over ω
+__global__ void k_adj_L_K2_tab(BubbleP B, Ptr3 tb, const cplx* rawbar, ChanWork cw, size_t n2, Dims d) {
+    const int ch = blockIdx.y;
+    const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (w >= cw.nitems[ch]) return;
+    const int idx = cw.items[ch] ? cw.items[ch][w] : w;
+    const int nu = idx % d.N2n - d.n2n;
+    const int m = (idx / d.N2n) % d.N2O - (d.n2O - 1), P = idx / (d.N2n * d.N2O);
+    const cplx s = rawbar[(size_t)ch * n2 + idx] * (d.U * d.T * (ch == CH_T ? -1.0 : 1.0));
+    cplx* row = const_cast<cplx*>(gamma_row<cplx>(tb.p[ch], d, m, nu));
+    const cplx* Pi0 = ch == CH_P ? B.pp0 : B.ph0;
+    for (int n = -d.n2n + lane; n < d.n2n; n += 32)
+        aadd(row + cross(ch, m, n), cmulc(Pi0[ixPi(d, P, m, n)], s));
+}
+// ---- K3 caches from the Γ table (k_build_cache_tab), transposed: warp per (block, ν) row ----
+__global__ void k_adj_cache_tab(VertBar Fb, Ptr3 tb, Caches Cb, const int* blocks, int nblocks, Dims d) {
+    const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (w >= nblocks * d.N3n) return;
+    const int bl = blocks ? blocks[w / d.N3n] : w / d.N3n;
+    const int a = w % d.N3n - d.n3n;
+    const int m = bl % d.N3O - (d.n3O - 1), P = bl / d.N3O;
+    const size_t row = ((size_t)bl * d.N3n + (a + d.n3n)) * d.N3n;
+    cplx* rp = const_cast<cplx*>(gamma_row<cplx>(tb.p[CH_P], d, m, a));
+    cplx* rt = const_cast<cplx*>(gamma_row<cplx>(tb.p[CH_T], d, m, a));
+    cplx* ra = const_cast<cplx*>(gamma_row<cplx>(tb.p[CH_A], d, m, a));
+    cplx sp = mk(0, 0), st = mk(0, 0), sa = mk(0, 0);
+    for (int ib = lane; ib < d.N3n; ib += 32) {
+        const size_t i = row + ib;
+        const int b = ib - d.n3n;
+        const cplx c7 = Cb.c[7][i], c8 = Cb.c[8][i], c9 = Cb.c[9][i];
+        aadd(rp + (m - b - 1), Cb.c[0][i] * -1.0);
+        aadd(rp + b, Cb.c[4][i] + c7);
+        aadd(ra + b, Cb.c[5][i] + c8);
+        aadd(rt + b, Cb.c[6][i] + c9);
+        // the own channel's K2(ν) + K3: fp = u_p + .., fa = u_a + .., 2 ft - fa = 2 u_t - u_a + ..
+        const cplx ua = c8 - c9, ut = c9 * 2.0;
+        const size_t j = ix3(d, P, m, a, b);
+        Fb.g[CH_P].K3[j] += c7; Fb.g[CH_A].K3[j] += ua; Fb.g[CH_T].K3[j] += ut;
+        sp += c7; sa += ua; st += ut;
+    }
+    sp = warp_sum(sp); sa = warp_sum(sa); st = warp_sum(st);
+    if (lane == 0) {
+        const size_t j = ix2(d, P, m, a);
+        Fb.g[CH_P].K2[j] += sp; Fb.g[CH_A].K2[j] += sa; Fb.g[CH_T].K2[j] += st;
+    }
+}
+// ---- Γ table (k_gamma_table), transposed ----
+__global__ void __launch_bounds__(256) k_adj_gamma_table(VertBar Fb, Ptr3 tb, const int* oms, Dims d) {
+    const int th = gamma_half(d), NT = 2 * th;
+    const int e = blockIdx.x * 256 + threadIdx.x;
+    if (e >= d.N2n * NT) return;
+    const int iO = oms ? oms[blockIdx.y] : blockIdx.y;
+    const int m = iO - (d.n2O - 1), nu = e / NT - d.n2n, n = e % NT - th;
+    const size_t i = (size_t)iO * d.N2n * NT + e;
+    const cplx p = ld16(tb.p[CH_P] + i), t = ld16(tb.p[CH_T] + i), a = ld16(tb.p[CH_A] + i) - t;
+    if (p.x != 0.0 || p.y != 0.0) pSp_adj(Fb, d, CH_P, m, nu, n, KAVG, FL_GT | FL_GA, p);
+    if (a.x != 0.0 || a.y != 0.0) pSp_adj(Fb, d, CH_A, m, nu, n, KAVG, FL_GP | FL_GT, a);
+    if (t.x != 0.0 || t.y != 0.0) pSp_adj(Fb, d, CH_T, m, nu, n, KAVG, FL_GP | FL_GA, t * 2.0);
+}
+
 // ---- K3 caches (k_build_cache), transposed: one thread per cache element of the listed blocks ----
 __global__ void k_adj_cache(VertBar Fb, Caches Cb, const int* blocks, int nblocks, Dims d) {
     const size_t bs = (size_t)d.N3n * d.N3n;
@@ -581,15 +722,6 @@ __global__ void k_adj_build_M(K3Args3 args, int mode, Ptr3 Mout, Dims d) {
 // as the forward K3 GEMM picks them, so that no block is padded beyond its size), 2 x 2 outputs per
 // thread, K chunks of 8, and the forward GEMM's three-multiplication complex product:
 // t1 = Σ ar br, t2 = Σ ai bi, t3 = Σ (ar + ai)(br + bi), C = (t1 - t2) + i (t3 - t1 - t2).
-struct GemmBatch {
-    const cplx* A[3];
-    const cplx* B[3];
-    cplx* C[3];
-    double alpha[3];
-    int accumulate;  // C += instead of C =
-    const int* blocks;
-    int nblocks;
-};
 template <int OPA, int OPB, int TILE>
 __global__ void __launch_bounds__((TILE / 2) * (TILE / 2)) k_adj_gemm(GemmBatch g, Dims d) {
     constexpr int TK = 8, H = TILE / 2, NT = H * H;
@@ -668,7 +800,8 @@ void launch_adj_gemm_tile(cudaStream_t s, const GemmBatch& g, const Dims& d) {
 }
 template <int OPA, int OPB>
 void launch_adj_gemm(cudaStream_t s, const GemmBatch& g, const Dims& d) {
-    if (d.N3n <= 16) launch_adj_gemm_tile<OPA, OPB, 16>(s, g, d);
+    if (g.digits) launch_adj_mma(s, OPA, g, d);
+    else if (d.N3n <= 16) launch_adj_gemm_tile<OPA, OPB, 16>(s, g, d);
     else if (d.N3n <= 24) launch_adj_gemm_tile<OPA, OPB, 24>(s, g, d);
     else launch_adj_gemm_tile<OPA, OPB, 32>(s, g, d);
 }
@@ -879,6 +1012,27 @@ cudaError_t launch_adj_K2(cudaStream_t s, const VertP& F, const FLP& FL, const B
     k_adj_K2<<<dim3(warp_grid3(cw, 3), 3), 128, 0, s>>>(F, FL, B, SX, Fb, FLb, Pbpp, Pbph, SXbar, rawbar, cw, n2, d);
     LCHK(); return cudaSuccess;
 }
+cudaError_t launch_adj_K2_tab(cudaStream_t s, const VertP& F, const FLP& FL, const BubbleP& B, const cplx* SX,
+                              const VertBar& Fb, const FLBar& FLb, const Ptr3& tb, cplx* Pbpp, cplx* Pbph, cplx* SXbar,
+                              const cplx* rawbar, const ChanWork& cw, size_t n2, const Dims& d) {
+    const int rows = std::max(1, std::max(cw.ngroups[0], std::max(cw.ngroups[1], cw.ngroups[2])));
+    const int threads = std::min(256, (2 * k2_table_half(d) + 31) / 32 * 32);
+    const size_t shm = (size_t)d.N2n * (sizeof(cplx) + sizeof(int));  // N2n < 2400 by the size limits of a state
+    k_adj_K2_rows<<<dim3(rows, 3), threads, shm, s>>>(F, FL, B, SX, Fb, FLb, tb, Pbpp, Pbph, SXbar, rawbar, cw, n2, d);
+    LCHK(); return cudaSuccess;
+}
+cudaError_t launch_adj_L_K2_tab(cudaStream_t s, const BubbleP& B, const Ptr3& tb, const cplx* rawbar,
+                                const ChanWork& cw, size_t n2, const Dims& d) {
+    k_adj_L_K2_tab<<<dim3(warp_grid3(cw, 3), 3), 128, 0, s>>>(B, tb, rawbar, cw, n2, d);
+    LCHK(); return cudaSuccess;
+}
+cudaError_t launch_adj_cache_tab(cudaStream_t s, const VertBar& Fb, const Ptr3& tb, const Caches& Cb, const int* blocks,
+                                 int nblocks, const int* oms, int noms, const Dims& d) {
+    k_adj_cache_tab<<<nb((size_t)nblocks * d.N3n * 32, 128), 128, 0, s>>>(Fb, tb, Cb, blocks, nblocks, d);
+    LCHK();
+    k_adj_gamma_table<<<dim3(nb((size_t)d.N2n * 2 * gamma_half(d), 256), noms), 256, 0, s>>>(Fb, tb, oms, d);
+    LCHK(); return cudaSuccess;
+}
 cudaError_t launch_adj_sx(cudaStream_t s, const cplx* Pipp, const cplx* Piph, const FLP& FL, const cplx* SXbar,
                           cplx* Pbpp, cplx* Pbph, cplx* SPibar, const FLBar& FLb, const Dims& d) {
     k_adj_sx<<<nb((size_t)3 * d.Nq * d.NPO * 32, 128), 128, 0, s>>>(Pipp, Piph, FL, SXbar, Pbpp, Pbph, SPibar, FLb, d);
@@ -899,7 +1053,7 @@ cudaError_t launch_adj_cache(cudaStream_t s, const VertBar& Fb, const Caches& Cb
 // distribution into Γ̄s (Gbar[slot]), Π̄ and γ̄L (FLbar, including the epilogue term)
 cudaError_t launch_adj_K3(cudaStream_t s, int mode, const K3Args3& a, const cplx* const Obar[3], cplx* const Abar[3],
                           cplx* const Gbar[3], cplx* const Mbuf[3], cplx* const Mbar[3], cplx* Pbpp, cplx* Pbph,
-                          cplx* const FLbar[3], const Dims& d) {
+                          cplx* const FLbar[3], const Dims& d, bool digits) {
     const int N = d.N3n;
     const size_t bs = (size_t)N * N;
     const Ptr3 mo{{Mbuf[0], Mbuf[1], Mbuf[2]}};  // slot pointers travel by value
@@ -917,6 +1071,7 @@ cudaError_t launch_adj_K3(cudaStream_t s, int mode, const K3Args3& a, const cplx
         g.alpha[i] = mode == 0 ? T * ((ch == CH_A) ? 1.0 : -1.0) : T;
     }
     g.accumulate = 1;
+    g.digits = digits;
     launch_adj_gemm<0, 1>(s, g, d);  // Ā += α ō Mᴴ
     LCHK();
     if (mode == 0) return cudaSuccess;
@@ -930,6 +1085,7 @@ cudaError_t launch_adj_K3(cudaStream_t s, int mode, const K3Args3& a, const cplx
         h.alpha[i] = T;
     }
     h.accumulate = 0;
+    h.digits = digits;
     launch_adj_gemm<1, 0>(s, h, d);  // M̄ = T Aᴴ ō
     LCHK();
     const Ptr3 mb{{Mbar[0], Mbar[1], Mbar[2]}};

@@ -618,6 +618,20 @@ __device__ __forceinline__ S fl_right(const S* FLK2p, const S* FLK2t, const S* F
 
 __device__ __forceinline__ int cross(int ch, int m, int n) { return ch == CH_P ? m - n - 1 : n; }
 
+// half width of the ω range that any window of the K2 BSE can reach, clipped to the stored bubble window
+__host__ __device__ __forceinline__ int k2_table_half(const Dims& d) {
+    const int W = d.xn2O + d.xn2n + d.xn1 + d.nRn + 2;  // (extents over F and a Vertex-valued F0)
+    return W < d.nPw ? W : d.nPw;
+}
+// first and last ω at which the vertex difference of the K2 BSE can differ from zero: the hull of its
+// windows (the K2 and RefVertex boxes and the K1 windows around ν, -(Ω+ν+1) and, p channel, Ω-ν-1),
+// clipped to the stored bubble window (solvers with a RefVertex)
+template <int CH>
+__device__ __forceinline__ void k2_hull(const Dims& d, int m, int nu, int& n0, int& n1) {
+    const int c2 = -(m + nu + 1), c3 = (CH == CH_P) ? m - nu - 1 : nu, hb = max(d.n2n, d.nRn), h1 = d.n1 - 1;
+    n0 = max(min(min(-hb, nu - h1), min(c2, c3) - h1), -d.nPw);
+    n1 = min(max(max(hb - 1, nu + h1), max(c2, c3) + h1), d.nPw - 1);
+}
 // half width of the Γ table: Γ(Ω, ν, ω) vanishes for |ω| beyond the K1 windows around ν, -(Ω+ν+1) and
 // Ω-ν-1, and every ω at which a cache or a left BSE reads it lies inside too
 __host__ __device__ __forceinline__ int gamma_half(const Dims& d) { return d.n2O + d.n2n + d.n1 + 2; }

@@ -83,12 +83,95 @@ __device__ __forceinline__ void store_digits(uint8_t* planes, int o, cplx v0, cp
     }
 }
 
+// One N x N complex product per CTA of NC·NC warps: av = two neighbouring k of row cl of the left operand,
+// mv = the same k of column cl of the right one; out(row, column, value, non-finite) is called by the lane
+// that holds an element.  fmax_ is zero on entry and a __syncthreads lies behind that.
+template <int NC, class OUT>
+__device__ __forceinline__ void digit_product(uint8_t* sm, int (*fmax_)[8 * NC], int N, int cl, int w0,
+                                              const cplx (&av)[2], const cplx (&mv)[2], OUT&& out) {
+    uint8_t* Mp = sm;
+    uint8_t* Ap = sm + 2 * S * PLANE<NC>;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    int em = max(cexpo(mv[0]), cexpo(mv[1])), ea = max(cexpo(av[0]), cexpo(av[1]));
+#pragma unroll
+    for (int o = 8; o <= 16; o <<= 1) {
+        em = max(em, __shfl_xor_sync(0xffffffffu, em, o));
+        ea = max(ea, __shfl_xor_sync(0xffffffffu, ea, o));
+    }
+    if (lane < 8) {
+        atomicMax(&fmax_[0][cl], ea);
+        atomicMax(&fmax_[1][cl], em);
+    }
+    __syncthreads();
+    const int so = cl * PITCH<NC> + 2 * w0;
+    store_digits<NC>(Ap, so, av[0], av[1], fmax_[0][cl]);
+    store_digits<NC>(Mp, so, mv[0], mv[1], fmax_[1][cl]);
+    __syncthreads();
+    // warp = (ν' chunk j, ν chunk nt): D rows 0-7 = Re, rows 8-15 = Im of the outputs ν' = 8j.., columns ν
+    const int j = warp % NC, nt = warp / NC;
+    float acc[S][4];
+#pragma unroll
+    for (int g = 0; g < S; ++g)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) acc[g][i] = 0.0f;
+    // lane l addresses row l % 8 of matrix l / 8: M re, M im, A re, A im of one digit
+    const uint32_t laddr = (uint32_t)__cvta_generic_to_shared(
+        (lane < 16 ? Mp + (8 * j + (lane & 7)) * PITCH<NC> : Ap + (8 * nt + (lane & 7)) * PITCH<NC>) +
+        ((lane >> 3) & 1) * PLANE<NC>);
+#pragma unroll 1
+    for (int c = 0; c < NC; ++c) {
+        uint32_t mr[S], mi[S], ar[S], ai[S];
+#pragma unroll
+        for (int s = 0; s < S; ++s)
+            asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+                         : "=r"(mr[s]), "=r"(mi[s]), "=r"(ar[s]), "=r"(ai[s])
+                         : "r"(laddr + (uint32_t)(2 * s * PLANE<NC> + 16 * c))
+                         : "memory");
+        // k = (ω chunk; Re A, Im A): rows Re: [Re M, -Im M], rows Im: [Im M, Re M]
+#pragma unroll
+        for (int s = 0; s < S; ++s)
+#pragma unroll
+            for (int t = 0; s + t < S; ++t)
+                asm volatile(
+                    "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
+                    "{%0,%1,%2,%3};"
+                    : "+f"(acc[s + t][0]), "+f"(acc[s + t][1]), "+f"(acc[s + t][2]), "+f"(acc[s + t][3])
+                    : "r"(mr[s]), "r"(mi[s]), "r"(mi[s] ^ 0x80008000u), "r"(mr[s]), "r"(ar[t]), "r"(ai[t]));
+    }
+    // D = 2^(F_A + F_M - 2044 - 124) Σ_g 256^(14-g) acc_g, joined as hi 256^11 + lo 256^7
+    const int col = 8 * j + (lane >> 2);
+    if (col >= N) return;
+    const int FM = fmax_[1][col];
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+        const int nu = 8 * nt + 2 * (lane & 3) + e;
+        if (nu >= N) continue;
+        const int FA = fmax_[0][nu], E = FA + FM - 2168;
+        if (FA == 0x7ff || FM == 0x7ff) {
+            const double qn = __longlong_as_double(0x7ff8000000000000ll);
+            out(nu, col, mk(qn, qn), true);
+            continue;
+        }
+        double p[2];
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            long long hi = 0, lo = 0;
+#pragma unroll
+            for (int g = 0; g < S; ++g) {
+                const long long v = (long long)__float2int_rn(acc[g][2 * q + e]);
+                if (g < 4) hi = hi * 256 + v;
+                else lo = lo * 256 + v;
+            }
+            p[q] = i2d_scaled(hi, E + 88) + i2d_scaled(lo, E + 56);
+        }
+        out(nu, col, mk(p[0], p[1]), false);
+    }
+}
+
 // MODE 0: L_K3, 1: K3 (and the dA·M part of the tangent), 3: the A·dM part of the tangent
 template <int MODE, int NC>
 __global__ void __launch_bounds__(32 * NC * NC) k_bse_K3_mma(K3Args3 args, Dims d) {
     extern __shared__ __align__(16) uint8_t sm[];
-    uint8_t* Mp = sm;
-    uint8_t* Ap = sm + 2 * S * PLANE<NC>;
     __shared__ cplx qf[8 * NC][2];  // the ω factors of M with their signs, as in k_bse_K3_oz
     __shared__ int fmax_[2][8 * NC];  // largest exponent fields: [0] rows ν of A, [1] columns ν' of M
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -157,7 +240,6 @@ __global__ void __launch_bounds__(32 * NC * NC) k_bse_K3_mma(K3Args3 args, Dims 
     }
     __syncthreads();
     cplx mv[2];
-    int em = 0, ea = 0;
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
         mv[i] = mk(0.0, 0.0);
@@ -165,82 +247,11 @@ __global__ void __launch_bounds__(32 * NC * NC) k_bse_K3_mma(K3Args3 args, Dims 
             const cplx* q = qf[w0 + i];
             mv[i] = full ? cfma(q[0], x0[i], q[1] * x1[i]) : q[0] * x0[i];
         }
-        em = max(em, cexpo(mv[i]));
-        ea = max(ea, cexpo(av[i]));
     }
-#pragma unroll
-    for (int o = 8; o <= 16; o <<= 1) {
-        em = max(em, __shfl_xor_sync(0xffffffffu, em, o));
-        ea = max(ea, __shfl_xor_sync(0xffffffffu, ea, o));
-    }
-    if (lane < 8) {
-        atomicMax(&fmax_[0][cl], ea);
-        atomicMax(&fmax_[1][cl], em);
-    }
-    __syncthreads();
-    const int so = cl * PITCH<NC> + 2 * w0;
-    store_digits<NC>(Ap, so, av[0], av[1], fmax_[0][cl]);
-    store_digits<NC>(Mp, so, mv[0], mv[1], fmax_[1][cl]);
-    __syncthreads();
-    // warp = (ν' chunk j, ν chunk nt): D rows 0-7 = Re, rows 8-15 = Im of the outputs ν' = 8j.., columns ν
-    const int j = warp % NC, nt = warp / NC;
-    float acc[S][4];
-#pragma unroll
-    for (int g = 0; g < S; ++g)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) acc[g][i] = 0.0f;
-    // lane l addresses row l % 8 of matrix l / 8: M re, M im, A re, A im of one digit
-    const uint32_t laddr = (uint32_t)__cvta_generic_to_shared(
-        (lane < 16 ? Mp + (8 * j + (lane & 7)) * PITCH<NC> : Ap + (8 * nt + (lane & 7)) * PITCH<NC>) +
-        ((lane >> 3) & 1) * PLANE<NC>);
-#pragma unroll 1
-    for (int c = 0; c < NC; ++c) {
-        uint32_t mr[S], mi[S], ar[S], ai[S];
-#pragma unroll
-        for (int s = 0; s < S; ++s)
-            asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
-                         : "=r"(mr[s]), "=r"(mi[s]), "=r"(ar[s]), "=r"(ai[s])
-                         : "r"(laddr + (uint32_t)(2 * s * PLANE<NC> + 16 * c))
-                         : "memory");
-        // k = (ω chunk; Re A, Im A): rows Re: [Re M, -Im M], rows Im: [Im M, Re M]
-#pragma unroll
-        for (int s = 0; s < S; ++s)
-#pragma unroll
-            for (int t = 0; s + t < S; ++t)
-                asm volatile(
-                    "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
-                    "{%0,%1,%2,%3};"
-                    : "+f"(acc[s + t][0]), "+f"(acc[s + t][1]), "+f"(acc[s + t][2]), "+f"(acc[s + t][3])
-                    : "r"(mr[s]), "r"(mi[s]), "r"(mi[s] ^ 0x80008000u), "r"(mr[s]), "r"(ar[t]), "r"(ai[t]));
-    }
-    // D = 2^(F_A + F_M - 2044 - 124) Σ_g 256^(14-g) acc_g, joined as hi 256^11 + lo 256^7
-    const int col = 8 * j + (lane >> 2);
-    if (col >= N) return;
-    const int FM = fmax_[1][col];
-#pragma unroll
-    for (int e = 0; e < 2; ++e) {
-        const int nu = 8 * nt + 2 * (lane & 3) + e;
-        if (nu >= N) continue;
-        const int FA = fmax_[0][nu], E = FA + FM - 2168;
+    digit_product<NC>(sm, fmax_, N, cl, w0, av, mv, [&](int nu, int col, cplx cv, bool bad) {
         const size_t io = base + (size_t)nu * N + col;
-        cplx o;
-        if (FA == 0x7ff || FM == 0x7ff) {
-            const double qn = __longlong_as_double(0x7ff8000000000000ll);
-            o = mk(qn, qn);
-        } else {
-            double p[2];
-#pragma unroll
-            for (int q = 0; q < 2; ++q) {
-                long long hi = 0, lo = 0;
-#pragma unroll
-                for (int g = 0; g < S; ++g) {
-                    const long long v = (long long)__float2int_rn(acc[g][2 * q + e]);
-                    if (g < 4) hi = hi * 256 + v;
-                    else lo = lo * 256 + v;
-                }
-                p[q] = i2d_scaled(hi, E + 88) + i2d_scaled(lo, E + 56);
-            }
-            const cplx cv = mk(p[0], p[1]);
+        cplx o = cv;
+        if (!bad) {
             if (MODE == 0) {
                 o = cv * (d.T * ((CH == CH_A) ? 1.0 : -1.0));
             } else if (a.flags & K3F_NOEPI) {
@@ -252,7 +263,46 @@ __global__ void __launch_bounds__(32 * NC * NC) k_bse_K3_mma(K3Args3 args, Dims 
             if (a.flags & K3F_ACC) o = a.out[io] + o;
         }
         a.out[io] = o;
+    });
+}
+
+// The products of the adjoint contraction: OPA = 0: C = α A Bᴴ, OPA = 1: C = α Aᴴ B (C += when
+// accumulating).  Adjoint GEMMs of Hubbard 8x8, nK3 = (8, 12) on GB300: 72 us each on the CUDA cores,
+// 23 us here.
+template <int OPA, int NC>
+__global__ void __launch_bounds__(32 * NC * NC) k_adj_mma(GemmBatch g, Dims d) {
+    extern __shared__ __align__(16) uint8_t sm[];
+    __shared__ int fmax_[2][8 * NC];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int N = d.N3n, slot = blockIdx.z;
+    const int blk = g.blocks ? g.blocks[blockIdx.x] : blockIdx.x;
+    const size_t base = (size_t)blk * N * N;
+    const cplx* A = (slot == 0 ? g.A[0] : slot == 1 ? g.A[1] : g.A[2]) + base;
+    const cplx* B = (slot == 0 ? g.B[0] : slot == 1 ? g.B[1] : g.B[2]) + base;
+    cplx* C = (slot == 0 ? g.C[0] : slot == 1 ? g.C[1] : g.C[2]) + base;
+    const double alpha = slot == 0 ? g.alpha[0] : slot == 1 ? g.alpha[1] : g.alpha[2];
+    if (tid < 8 * NC) fmax_[0][tid] = fmax_[1][tid] = 0;
+    const int cl = 8 * (warp % NC) + (lane & 7), w0 = 8 * (warp / NC) + 2 * (lane >> 3);
+    cplx av[2], mv[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const int w = w0 + i;
+        av[i] = mv[i] = mk(0.0, 0.0);
+        if (cl >= N || w >= N) continue;
+        if (OPA == 0) {
+            av[i] = ldg(A + (size_t)cl * N + w);
+            mv[i] = conjg(ldg(B + (size_t)cl * N + w));
+        } else {
+            av[i] = conjg(ldg(A + (size_t)w * N + cl));
+            mv[i] = ldg(B + (size_t)w * N + cl);
+        }
     }
+    __syncthreads();
+    digit_product<NC>(sm, fmax_, N, cl, w0, av, mv, [&](int r, int c, cplx cv, bool bad) {
+        cplx* o = C + (size_t)r * N + c;
+        const cplx v = bad ? cv : cv * alpha;
+        *o = g.accumulate ? *o + v : v;
+    });
 }
 
 template <int MODE, int NC>
@@ -272,15 +322,32 @@ cudaError_t run_mode(cudaStream_t s, const K3Args3& a, int nslots, const Dims& d
 
 }  // namespace
 
+template <int OPA>
+static cudaError_t run_adj(cudaStream_t s, const GemmBatch& g, const Dims& d) {
+    const dim3 grid((unsigned)g.nblocks, 1, 3);
+    switch ((d.N3n + 7) / 8) {
+        case 1: k_adj_mma<OPA, 1><<<grid, 32, SMEM<1>, s>>>(g, d); break;
+        case 2: k_adj_mma<OPA, 2><<<grid, 128, SMEM<2>, s>>>(g, d); break;
+        case 3: k_adj_mma<OPA, 3><<<grid, 288, SMEM<3>, s>>>(g, d); break;
+        default: k_adj_mma<OPA, 4><<<grid, 512, SMEM<4>, s>>>(g, d); break;
+    }
+    return cudaGetLastError();
+}
+cudaError_t launch_adj_mma(cudaStream_t s, int opa, const GemmBatch& g, const Dims& d) {
+    return opa ? run_adj<1>(s, g, d) : run_adj<0>(s, g, d);
+}
+
 bool k3_mma_supported(const Dims& d) { return d.N3n <= 32; }
 
 // raises the shared-memory limit of the four-chunk instantiations (82 KB); the others fit the default
 cudaError_t prepare_bse_K3_mma(const Dims& d) {
     if (d.N3n <= 24) return cudaSuccess;
-    static SmemRecord set0, set1, set3;
+    static SmemRecord set0, set1, set3, seta, setb;
     cudaError_t e = raise_smem_limit(k_bse_K3_mma<0, 4>, set0, SMEM<4>, 0);
     if (e == cudaSuccess) e = raise_smem_limit(k_bse_K3_mma<1, 4>, set1, SMEM<4>, 0);
     if (e == cudaSuccess) e = raise_smem_limit(k_bse_K3_mma<3, 4>, set3, SMEM<4>, 0);
+    if (e == cudaSuccess) e = raise_smem_limit(k_adj_mma<0, 4>, seta, SMEM<4>, 0);
+    if (e == cudaSuccess) e = raise_smem_limit(k_adj_mma<1, 4>, setb, SMEM<4>, 0);
     return e;
 }
 

@@ -901,10 +901,6 @@ __device__ __forceinline__ void bse_L_K2_body(const VertPT<S>& F, const cplx* Pi
 // (pSp_k2diff; the t channel's 2 pSp + xSp by crossing, xSp = -pSp in the a representation).
 // GB300's FP64 pipe bounds this kernel: both take FP64 work out of the per-term loop.
 // TAN: the tangent in one pass, as for K1 (tables X and dX).
-__host__ __device__ __forceinline__ int k2_table_half(const Dims& d) {
-    const int W = d.xn2O + d.xn2n + d.xn1 + d.nRn + 2;  // (extents over F and a Vertex-valued F0)
-    return W < d.nPw ? W : d.nPw;
-}
 // TAB: Γ from the table of the nonlocal solver (F.tab; T.F.tab for the tangent vertex), read along ω, so
 // that a term costs its product and the own K3 only.  The ω range is then the hull of the windows (Γ is
 // zero in their gaps).
@@ -950,9 +946,8 @@ __device__ __forceinline__ void bse_K2_row(const VertPT<S>& F, const FLPT<S>& FL
         if constexpr (TAN) tc = k2_c<CH>(T.F, d, m, nu, P);
         S acc{0, 0};
         if constexpr (TAB) {
-            const int c2 = -(m + nu + 1), c3 = (CH == CH_P) ? m - nu - 1 : nu, hb = max(d.n2n, d.nRn);
-            const int n0 = max(min(min(-hb, nu - h1), min(c2, c3) - h1), lo);
-            const int n1 = min(max(max(hb - 1, nu + h1), max(c2, c3) + h1), hi);
+            int n0, n1;
+            k2_hull<CH>(d, m, nu, n0, n1);
             const S* row = gamma_row(F.tab[CH], d, m, nu);
             const S* trow = TAN ? gamma_row(T.F.tab[CH], d, m, nu) : nullptr;
             const bool r3 = bin(m, d.n3O) && fin(nu, d.n3n);

@@ -160,6 +160,17 @@ struct ChanBarArrays {  // averages' cotangents (read) and the K arrays' cotange
 struct Ptr3 {
     cplx* p[3];
 };
+// batched N x N products of the adjoint K3 contraction (fdga_adjoint.cu, fdga_k3_mma.cu)
+struct GemmBatch {
+    const cplx* A[3];
+    const cplx* B[3];
+    cplx* C[3];
+    double alpha[3];
+    int accumulate;  // C += instead of C =
+    bool digits;     // by digit slicing (fdga_k3_mma.cu; Nν3 ≤ 32)
+    const int* blocks;
+    int nblocks;
+};
 struct Finalize3 {  // indexed by channel (p, t, a)
     const cplx* raw[3];
     cplx* out[3];
@@ -358,6 +369,8 @@ cudaError_t launch_scale(cudaStream_t s, cplx* out, const cplx* in, double sc, s
 // (fdga_k3_mma.cu), modes 0, 1 and 2
 bool k3_mma_supported(const Dims& d);
 cudaError_t prepare_bse_K3_mma(const Dims& d);
+// C = α A Bᴴ (conjugate transpose of A: C = α Aᴴ B) of the listed blocks, C += when accumulating
+cudaError_t launch_adj_mma(cudaStream_t s, int opa, const GemmBatch& g, const Dims& d);
 cudaError_t launch_bse_K3_mma(cudaStream_t s, int mode, const K3Args3& a, int nslots, const Dims& d);
 // FP64 K3 contractions on the tensor cores by exact BF16 digit slicing (fdga_k3_oz.cu), modes 0, 1
 // and 2 (the tangent); fa_scratch holds nslots x nblocks ints (per-block exponent bounds), adig the
@@ -459,7 +472,15 @@ cudaError_t launch_adj_cache(cudaStream_t s, const VertBar& Fb, const Caches& Cb
                              const Dims& d);
 cudaError_t launch_adj_K3(cudaStream_t s, int mode, const K3Args3& a, const cplx* const Obar[3], cplx* const Abar[3],
                           cplx* const Gbar[3], cplx* const Mbuf[3], cplx* const Mbar[3], cplx* Pbpp, cplx* Pbph,
-                          cplx* const FLbar[3], const Dims& d);
+                          cplx* const FLbar[3], const Dims& d, bool digits);
+// the stages of the adjoint that the Γ table shares (fdga_adjoint.cu); tb: the table's cotangent
+cudaError_t launch_adj_K2_tab(cudaStream_t s, const VertP& F, const FLP& FL, const BubbleP& B, const cplx* SX,
+                              const VertBar& Fb, const FLBar& FLb, const Ptr3& tb, cplx* Pbpp, cplx* Pbph, cplx* SXbar,
+                              const cplx* rawbar, const ChanWork& cw, size_t n2, const Dims& d);
+cudaError_t launch_adj_L_K2_tab(cudaStream_t s, const BubbleP& B, const Ptr3& tb, const cplx* rawbar,
+                                const ChanWork& cw, size_t n2, const Dims& d);
+cudaError_t launch_adj_cache_tab(cudaStream_t s, const VertBar& Fb, const Ptr3& tb, const Caches& Cb, const int* blocks,
+                                 int nblocks, const int* oms, int noms, const Dims& d);
 cudaError_t launch_adj_bubble(cudaStream_t s, const cplx* GR, cplx* Pbpp, cplx* Pbph, cplx* PbRpp, cplx* PbRph,
                               const cplx* SPibar, cplx* SRbar, cplx* GRbar, const cplx* twm, const Dims& d);
 cudaError_t launch_adj_qavg(cudaStream_t s, const ChanBarArrays& bar, const Dims& d);

@@ -182,6 +182,7 @@ struct fdga_handle {
         cplx *raw1 = nullptr, *raw2 = nullptr, *raw3 = nullptr, *M = nullptr, *Mb = nullptr;
         cplx *SigInb = nullptr, *SU2b = nullptr, *SigRb = nullptr, *u2Rb = nullptr, *u2Cb = nullptr;
         cplx *LRb = nullptr, *Lb = nullptr;
+        cplx* gtabb = nullptr;  // cotangent of the Γ table
         double* nbar = nullptr;
         Graph graphs[2][2][2];  // [strategy][update_sigma][hartree] (FP64)
     } adj;
@@ -1309,6 +1310,7 @@ int ensure_adjoint(fdga_handle* h) {
     AL(a.SigInb, h->nGk); AL(a.SU2b, h->nGk); AL(a.SigRb, h->nGk); AL(a.u2Rb, h->nGk);
     AL(a.u2Cb, (size_t)d.Nq * (2 * d.NG - 1));
     AL(a.LRb, 2 * h->n2); AL(a.Lb, 2 * h->n2);
+    if (h->gtab) AL(a.gtabb, gamma_table_len(d));
     AL(a.nbar, 1);
     return FDGA_OK;
 }
@@ -1328,7 +1330,13 @@ int enqueue_adjoint(fdga_handle* h, int strategy, bool update_sigma, bool hartre
     CK(Z(a.FLK2b, 3 * h->n2 * sizeof(cplx))); CK(Z(a.FLK3b, 3 * h->n3 * sizeof(cplx)));
     CK(Z(a.SigInb, h->nGk * sizeof(cplx))); CK(Z(a.SU2b, h->nGk * sizeof(cplx)));
     CK(Z(a.nbar, sizeof(double)));
+    const size_t nT = gamma_table_len(d) / 3;
+    const Ptr3 tb{{a.gtabb, a.gtabb ? a.gtabb + nT : nullptr, a.gtabb ? a.gtabb + 2 * nT : nullptr}};
+    if (a.gtabb) CK(Z(a.gtabb, 3 * nT * sizeof(cplx)));
+    // the adjoint GEMMs take the digit-sliced kernel where the map's contractions do (launch_k3_fp64)
+    const bool digits = h->k3_oz == 2 && k3_mma_supported(d);
     VertP F = vertex_view(h, h->xS), Fn = vertex_view(h, h->yS);
+    set_table(h, F, h->gtab);  // the value pass's
     // cotangent views: x̄ (with the averages' cotangents) and ȳ (SDE contributions to the new vertex)
     auto bar_view = [&](cplx* st, cplx* avg) {
         VertBar B{};
@@ -1360,6 +1368,7 @@ int enqueue_adjoint(fdga_handle* h, int strategy, bool update_sigma, bool hartre
             const Group& g = cls == 1 ? h->gK1 : k2group(h, ch);
             cw.items[ch] = g.trivial ? nullptr : g.d_items;
             cw.nitems[ch] = g.trivial ? (int)n : g.nitems;
+            if (cls == 2) k2_rows(h, g, cw, ch);
         }
         return cw;
     };
@@ -1438,13 +1447,16 @@ int enqueue_adjoint(fdga_handle* h, int strategy, bool update_sigma, bool hartre
         }
         a3.blocks = h->d_k3blocks;
         a3.nblocks = h->nk3blocks;
-        CK(launch_adj_K3(s, 1, a3, Ob, Ab, Gb, Mb, Mbb, a.Pbpp, a.Pbph, FL3b, d));
+        CK(launch_adj_K3(s, 1, a3, Ob, Ab, Gb, Mb, Mbb, a.Pbpp, a.Pbph, FL3b, d, digits));
     }
     {  // K2 outputs (with the FL epilogue) and K2 BSE transposed
         const cplx* ob[3] = {chanK(h, a.yb, CH_P, 2), chanK(h, a.yb, CH_T, 2), chanK(h, a.yb, CH_A, 2)};
         const Group* grp[3] = {&h->gK2pp, &h->gK2ph, &h->gK2ph};
         CK(fin_adj(ob, a.raw2, h->n2, grp, 1, 1, FL2b));
-        CK(launch_adj_K2(s, F, FL, B, h->SX, Xb, FLb, a.Pbpp, a.Pbph, a.SXb, a.raw2, work(2), h->n2, d));
+        if (a.gtabb)
+            CK(launch_adj_K2_tab(s, F, FL, B, h->SX, Xb, FLb, tb, a.Pbpp, a.Pbph, a.SXb, a.raw2, work(2), h->n2, d));
+        else
+            CK(launch_adj_K2(s, F, FL, B, h->SX, Xb, FLb, a.Pbpp, a.Pbph, a.SXb, a.raw2, work(2), h->n2, d));
     }
     {  // K1
         const cplx* ob[3] = {chanK(h, a.yb, CH_P, 1), chanK(h, a.yb, CH_T, 1), chanK(h, a.yb, CH_A, 1)};
@@ -1474,19 +1486,21 @@ int enqueue_adjoint(fdga_handle* h, int strategy, bool update_sigma, bool hartre
             }
             a3.blocks = h->d_k3blocks;
             a3.nblocks = h->nk3blocks;
-            CK(launch_adj_K3(s, 0, a3, Ob, Ab, nullptr, Mb, Mbb, nullptr, nullptr, nullptr, d));
+            CK(launch_adj_K3(s, 0, a3, Ob, Ab, nullptr, Mb, Mbb, nullptr, nullptr, nullptr, d, digits));
         }
         {  // FL.K2 = L_K2(F)
             const cplx* ob[3] = {FL2b[CH_P], FL2b[CH_T], FL2b[CH_A]};
             const Group* grp[3] = {&h->gK2pp, &h->gK2ph, &h->gK2ph};
             CK(fin_adj(ob, a.raw2, h->n2, grp, 0, 1, nullptr));
-            CK(launch_adj_L_K2(s, B, Xb, a.raw2, work(2), h->n2, d));
+            if (a.gtabb) CK(launch_adj_L_K2_tab(s, B, tb, a.raw2, work(2), h->n2, d));
+            else CK(launch_adj_L_K2(s, B, Xb, a.raw2, work(2), h->n2, d));
         }
     }
     {  // caches
         Caches Cb{};
         for (int i = 0; i < 10; ++i) Cb.c[i] = cb[i];
-        CK(launch_adj_cache(s, Xb, Cb, h->d_k3blocks, h->nk3blocks, d));
+        if (a.gtabb) CK(launch_adj_cache_tab(s, Xb, tb, Cb, h->d_k3blocks, h->nk3blocks, h->d_goms, h->ngoms, d));
+        else CK(launch_adj_cache(s, Xb, Cb, h->d_k3blocks, h->nk3blocks, d));
     }
     if (update_sigma) {  // bubbles and row sums -> Ḡ(R) -> Ḡ -> Σ̄ (Dyson)
         CK(launch_adj_bubble(s, h->GR, a.Pbpp, a.Pbph, a.PbRpp, a.PbRph, a.SPib, a.SRb, a.GRb, h->twm, d));

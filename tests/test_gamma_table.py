@@ -37,3 +37,25 @@ def test_map_matches_oracle(name, sym):
         assert blockwise_rel_err(cfg, gpu.fixed_point(x, strategy) + x, y) < 1e-10
         x = y
     gpu.close()
+
+
+@pytest.mark.parametrize("sym", [True, False], ids=["groups", "trivial"])
+@pytest.mark.parametrize("name", list(CASES))
+def test_adjoint_is_the_transpose_of_the_tangent(name, sym):
+    """<ȳ, J v> = <Jᵀ ȳ, v> to 1e-12 of |ȳ| |J v| (both sides are FP64 sums of the same terms)."""
+    from fdgasolver.models import hubbard_bare_Green
+    cfg = dict(CASES[name])
+    cfg["G0"] = hubbard_bare_Green(cfg["T"], cfg["nG"], cfg["L"], mu=0.0, t1=1.0)
+    gpu = make_gpu(cfg, sym)
+    rng = np.random.default_rng(10)
+    noise = lambda: rng.standard_normal(gpu.state_len) + 1j * rng.standard_normal(gpu.state_len)  # noqa: E731
+    for strategy in ("fdPA", "scPA"):
+        gpu.unflatten(gpu.fixed_point(0.05 * noise(), strategy))
+        x = gpu.flatten()
+        v, yb = noise(), noise()
+        jv = gpu.frule(v, strategy)[1]
+        gpu.unflatten(x)
+        xb = gpu.rrule(yb, strategy)[1]
+        a, b = np.vdot(yb, jv).real, np.vdot(xb, v).real
+        assert abs(a - b) < 1e-12 * np.linalg.norm(yb) * np.linalg.norm(jv)
+    gpu.close()
