@@ -1294,6 +1294,122 @@ __device__ __forceinline__ void sde_L_body(const VertPT<S>& F, const cplx* Pi, c
     }
 }
 
+// The same sums by (P, Ω) rows (solvers with a RefVertex).  In γ(Ω, ω̃, ν) - γ(Ω, ∞, ν) the K1 and K2(ν)
+// terms cancel, which leaves K2(ω̃) + K3(ω̃, ν): the K2 part of the sum is one number per row,
+//   L = T U [c SΠ + Σ_ω̃ Π K2(ω̃) + Σ_{K3 box} Π K3(ω̃, ν) + ref_scale Σ_r Π (F0 correction)],
+// and an item costs four FMAs (ph: and one addition) per K3 frequency.  A CTA does one row: one item per
+// lane, the frequencies split over the warps and joined through shared memory, so that no term passes
+// through a warp reduction.  The FP64 pipe bounded the item-wise form (k_sde_L_all, kept for a
+// Vertex-valued F0), which evaluated the channels per term and reduced every item over a warp.
+// SDE stage (this kernel, the class expansion, four transforms and the assembly) on GB300, item-wise -> by
+// rows, in us: Hubbard 8x8, nK3 = (8, 12) 94 -> 69; 5x5 without groups, nK3 = (5, 7) 119 -> 62; 8x8,
+// nK3 = (20, 40) 406 -> 166; SIAM, nK3 = (16, 16) 48 -> 39.
+constexpr int SDE_LANES = 32;
+template <int WHICH, class S, bool TAN>
+__device__ __forceinline__ void sde_L_row(const VertPT<S>& F, const cplx* Pi, const cplx* SPi, cplx* out,
+                                          const int* items, const int* gstart, int ngroups, int use_vertex,
+                                          double ref_scale, int accum, const Dims& d, const TanArgsT<S>& T, S* sm) {
+    using R = decltype(S::x);
+    const int g = blockIdx.x;
+    if (g >= ngroups) return;
+    const int i0 = gstart ? gstart[g] : g * d.N2n, i1 = gstart ? gstart[g + 1] : (g + 1) * d.N2n;
+    const int first = items ? items[i0] : i0;
+    const int m = (first / d.N2n) % d.N2O - (d.n2O - 1), P = first / (d.N2n * d.N2O);
+    const cplx* tPi = WHICH == 0 ? T.pp : T.ph;
+    const int hb = max(d.n2n, d.nRn), lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    S* pt = sm;                                // Π at ω̃, [2 hb]
+    S* tpt = pt + 2 * hb;                      // dΠ (TAN)
+    S* part = sm + (TAN ? 4 : 2) * hb;         // [nw][SDE_LANES] partial sums
+    S* rowv = part + nw * SDE_LANES;           // the row's K2 part
+    for (int j = threadIdx.x; j < 2 * hb; j += blockDim.x) {
+        const int nt = j - hb, n = WHICH == 0 ? m - nt - 1 : nt;
+        const bool in = fin(n, d.nPw);
+        pt[j] = in ? to_c<S>(ldg(Pi + ixPi(d, P, m, n))) : S{0, 0};
+        if constexpr (TAN) tpt[j] = in ? to_c<S>(ldg(tPi + ixPi(d, P, m, n))) : S{0, 0};
+    }
+    __syncthreads();
+    const bool vert = (use_vertex & 1) != 0;
+    auto k2sum = [&](const VertPT<S>& V, int n) -> S {  // K2(Ω, n) of the row's channels
+        if (WHICH == 0) return k2v(V.g[CH_P], d, m, n, P);
+        return k2v(V.g[CH_T], d, m, n, P) + k2v(V.g[CH_A], d, m, n, P);
+    };
+    auto k1sum = [&](const VertPT<S>& V) -> S {
+        if (WHICH == 0) return k1v(V.g[CH_P], d, m, P);
+        return k1v(V.g[CH_T], d, m, P) + k1v(V.g[CH_A], d, m, P);
+    };
+    if (warp == 0) {
+        S a{0, 0};
+        if (vert) {
+            for (int n = -d.n2n + lane; n < d.n2n; n += 32) {
+                if constexpr (!TAN) a = cfma(pt[n + hb], k2sum(F, n), a);
+                else a = cfma(tpt[n + hb], k2sum(F, n), cfma(pt[n + hb], k2sum(T.F, n), a));
+            }
+        }
+        a = warp_sum(a);
+        if (lane == 0) rowv[0] = a;
+    }
+    const bool r3 = vert && bin(m, d.n3O), rr = ref_scale != 0.0 && bin(m, d.nRO);
+    const size_t is = (size_t)P * d.NPO + (m + d.nPO - 1);
+    for (int j0 = i0; j0 < i1; j0 += SDE_LANES) {
+        const int it = j0 + lane;
+        const int idx = it < i1 ? (items ? items[it] : it) : -1;
+        const int nu = idx >= 0 ? idx % d.N2n - d.n2n : 0;
+        S acc{0, 0};
+        if (idx >= 0 && r3 && fin(nu, d.n3n)) {
+            for (int n = -d.n3n + warp; n < d.n3n; n += nw) {
+                S k, tk{0, 0};
+                if (WHICH == 0) {
+                    k = k3v(F.g[CH_P], d, m, n, nu, P);
+                    if constexpr (TAN) tk = k3v(T.F.g[CH_P], d, m, n, nu, P);
+                } else {
+                    k = k3v(F.g[CH_T], d, m, nu, n, P) + k3v(F.g[CH_A], d, m, nu, n, P);
+                    if constexpr (TAN) tk = k3v(T.F.g[CH_T], d, m, nu, n, P) + k3v(T.F.g[CH_A], d, m, nu, n, P);
+                }
+                if constexpr (!TAN) acc = cfma(pt[n + hb], k, acc);
+                else acc = cfma(tpt[n + hb], k, cfma(pt[n + hb], tk, acc));
+            }
+        }
+        if (idx >= 0 && rr && fin(nu, d.nRn)) {  // F0_p - U, or F0_a + F0_t - 2U; dΠ in the tangent
+            S ar{0, 0};
+            for (int r = -d.nRn + warp; r < d.nRn; r += nw) {
+                const S p = TAN ? tpt[r + hb] : pt[r + hb];
+                if (WHICH == 0) ar = cfma(p, ref_call(F.Fp_p, d, m, r, nu), ar);
+                else ar = cfma(p, ref_call(F.Ft_p, d, m, nu, r) - ref_call(F.Ft_x, d, m, r, nu), ar);
+            }
+            acc += ar * (R)ref_scale;
+        }
+        __syncthreads();  // (rowv, and the previous chunk's part)
+        part[warp * SDE_LANES + lane] = acc;
+        __syncthreads();
+        if (warp == 0 && idx >= 0) {
+            S s = rowv[0];
+            for (int w = 0; w < nw; ++w) s += part[w * SDE_LANES + lane];
+            if (vert) {
+                const S c = k1sum(F) + k2sum(F, nu), sp = to_c<S>(ldg(SPi + is));
+                if constexpr (!TAN) {
+                    s = cfma(c, sp, s);
+                } else {
+                    const S tc = k1sum(T.F) + k2sum(T.F, nu), tsp = to_c<S>(ldg((WHICH == 0 ? T.SPpp : T.SPph) + is));
+                    s = cfma(tc, sp, cfma(c, tsp, s));
+                }
+            }
+            const cplx v = to_d(s * (R)(d.T * d.U));
+            out[idx] = accum ? out[idx] + v : v;
+        }
+    }
+}
+template <class S, bool TAN>
+__global__ void __launch_bounds__(256) k_sde_L_rows(VertPT<S> F, BubbleP B, const cplx* SPpp, const cplx* SPph,
+                                                    ChanWork cw, int use_vertex, double ref_scale, Dims d,
+                                                    TanArgsT<S> T) {
+    extern __shared__ __align__(16) unsigned char sde_smem[];
+    S* sm = reinterpret_cast<S*>(sde_smem);
+    if (blockIdx.y == 0)
+        sde_L_row<0, S, TAN>(F, B.pp, SPpp, cw.out[0], cw.items[0], cw.gstart[0], cw.ngroups[0], use_vertex, ref_scale, cw.acc, d, T, sm);
+    else
+        sde_L_row<1, S, TAN>(F, B.ph, SPph, cw.out[1], cw.items[1], cw.gstart[1], cw.ngroups[1], use_vertex, ref_scale, cw.acc, d, T, sm);
+}
+
 // ---------------------------------------------------------------------------------------------
 // K1 and K2 of the :fdPA_new / :scPA_new strategies, local solver (src/BSEa/BSEa_K1.jl:57-100,
 // src/BSEa/BSEa_K2.jl:104-150), warp per item:
@@ -1930,6 +2046,20 @@ static unsigned warp_grid(const ChanWork& cw, int nch) {
     for (int c = 0; c < nch; ++c) mx = std::max(mx, cw.nitems[c]);
     return blocks_for((size_t)mx * 32, 128);
 }
+// rows of the SDE's L: eight warps split a row's K3 frequencies when the rows are few (the local solver),
+// else four
+template <class S, bool TAN>
+static cudaError_t sde_L_rows(cudaStream_t s, const VertPT<S>& F, const BubbleP& B, const cplx* SPpp, const cplx* SPph,
+                              const ChanWork& cw, int use_vertex, double ref_scale, const Dims& d,
+                              const TanArgsT<S>& T) {
+    const unsigned rows = row_grid(cw, 2);
+    const int threads = rows * 2 < 4 * 152 ? 256 : 128, hb = std::max(d.n2n, d.nRn);
+    const size_t smem = ((size_t)(TAN ? 4 : 2) * hb + threads / 32 * SDE_LANES + 1) * sizeof(S);
+    cudaError_t e = k2_smem_attr(k_sde_L_rows<S, TAN>, smem);
+    if (e != cudaSuccess) return e;
+    k_sde_L_rows<S, TAN><<<dim3(rows, 2), threads, smem, s>>>(F, B, SPpp, SPph, cw, use_vertex, ref_scale, d, T);
+    LAUNCH_CHECK(); return cudaSuccess;
+}
 // each vertex-evaluating kernel is launched in its V0 = F.has0 instantiation (see vert_spec)
 template <class K>
 static cudaError_t k2_launch_attr(K k_plain, K k_v0, K k_tab, bool v0, bool tab, size_t smem) {
@@ -1964,9 +2094,9 @@ static cudaError_t k2_launch_attr(K k_plain, K k_v0, K k_tab, bool v0, bool tab,
     }                                                                                                               \
     cudaError_t launch_sde_L_all(cudaStream_t s, const VT& F, const BubbleP& B, const cplx* SPpp, const cplx* SPph, \
                                  const ChanWork& cw, int use_vertex, double ref_scale, const Dims& d) {             \
+        if (!F.has0) return sde_L_rows<ST, false>(s, F, B, SPpp, SPph, cw, use_vertex, ref_scale, d, TT{});         \
         const dim3 g(warp_grid(cw, 2), 2);                                                                          \
-        if (F.has0) k_sde_L_all<ST, false, true><<<g, 128, 0, s>>>(F, B, SPpp, SPph, cw, use_vertex, ref_scale, d, TT{}); \
-        else k_sde_L_all<ST, false, false><<<g, 128, 0, s>>>(F, B, SPpp, SPph, cw, use_vertex, ref_scale, d, TT{});  \
+        k_sde_L_all<ST, false, true><<<g, 128, 0, s>>>(F, B, SPpp, SPph, cw, use_vertex, ref_scale, d, TT{});        \
         LAUNCH_CHECK(); return cudaSuccess;                                                                         \
     }                                                                                                               \
     cudaError_t launch_bse_K1_tan(cudaStream_t s, const VT& F, const FT& FL, const BubbleP& B, const cplx* SX,    \
@@ -1990,9 +2120,9 @@ static cudaError_t k2_launch_attr(K k_plain, K k_v0, K k_tab, bool v0, bool tab,
     }                                                                                                               \
     cudaError_t launch_sde_L_tan(cudaStream_t s, const VT& F, const BubbleP& B, const cplx* SPpp, const cplx* SPph, \
                                  const TT& T, const ChanWork& cw, double ref_scale, const Dims& d) {                \
+        if (!F.has0) return sde_L_rows<ST, true>(s, F, B, SPpp, SPph, cw, 1, ref_scale, d, T);                     \
         const dim3 g(warp_grid(cw, 2), 2);                                                                          \
-        if (F.has0) k_sde_L_all<ST, true, true><<<g, 128, 0, s>>>(F, B, SPpp, SPph, cw, 3, ref_scale, d, T);       \
-        else k_sde_L_all<ST, true, false><<<g, 128, 0, s>>>(F, B, SPpp, SPph, cw, 1, ref_scale, d, T);             \
+        k_sde_L_all<ST, true, true><<<g, 128, 0, s>>>(F, B, SPpp, SPph, cw, 3, ref_scale, d, T);                   \
         LAUNCH_CHECK(); return cudaSuccess;                                                                         \
     }
 #define FDGA_NEW_LAUNCHERS(VT, ST)                                                                                 \

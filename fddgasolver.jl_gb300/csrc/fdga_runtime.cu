@@ -597,6 +597,7 @@ cudaError_t sde_L_pair(fdga_handle* h, const V& F, const BubbleP& B, const cplx*
         cw.items[w] = g[w]->trivial ? nullptr : g[w]->d_items;
         cw.nitems[w] = g[w]->trivial ? (int)h->n2 : g[w]->nitems;
         cw.out[w] = h->raw2 + (size_t)w * h->n2;
+        k2_rows(h, *g[w], cw, w);
     }
     cudaError_t e = launch_sde_L_all(h->st, F, B, SPi, SPi + nS, cw, use_vertex, rs, d);
     if (e != cudaSuccess) return e;
@@ -1232,6 +1233,7 @@ int enqueue_tangent(fdga_handle* h, int strategy, bool update_sigma, bool hartre
             cw.items[w] = g[w]->trivial ? nullptr : g[w]->d_items;
             cw.nitems[w] = g[w]->trivial ? (int)h->n2 : g[w]->nitems;
             cw.out[w] = h->raw2 + (size_t)w * h->n2;
+            k2_rows(h, *g[w], cw, w);
         }
         // dL = L(dF; Π, SΠ) + L(F; dΠ, dSΠ) (+ the RefVertex part with dΠ), one pass
         if (mixed) {
