@@ -538,13 +538,14 @@ __global__ void k_adj_K2(VertP F, FLP FL, BubbleP B, const cplx* SX, VertBar Fb,
 
 // ---- S_X = (SΠ - SΠ0) U + Σ_t Π FL, transposed ----
 __global__ void k_adj_sx(const cplx* Pipp, const cplx* Piph, FLP FL, const cplx* SXbar, cplx* Pbpp, cplx* Pbph,
-                         cplx* SPibar, FLBar FLb, Dims d) {
+                         cplx* SPibar, FLBar FLb, Dims d, RowMask rm) {
     const size_t per = (size_t)d.Nq * d.NPO;
     const size_t i = (blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (i >= 3 * per) return;
     const int ch = (int)(i / per);
     const size_t r = i % per;
+    if (rm.row && !rm.row[r]) return;  // S̄_X is zero there, and Π not formed
     const int m = (int)(r % d.NPO) - (d.nPO - 1), P = (int)(r / d.NPO);
     const int w = (ch == CH_P) ? 0 : 1;
     const cplx* Pi = w ? Piph : Pipp;
@@ -1034,8 +1035,8 @@ cudaError_t launch_adj_cache_tab(cudaStream_t s, const VertBar& Fb, const Ptr3& 
     LCHK(); return cudaSuccess;
 }
 cudaError_t launch_adj_sx(cudaStream_t s, const cplx* Pipp, const cplx* Piph, const FLP& FL, const cplx* SXbar,
-                          cplx* Pbpp, cplx* Pbph, cplx* SPibar, const FLBar& FLb, const Dims& d) {
-    k_adj_sx<<<nb((size_t)3 * d.Nq * d.NPO * 32, 128), 128, 0, s>>>(Pipp, Piph, FL, SXbar, Pbpp, Pbph, SPibar, FLb, d);
+                          cplx* Pbpp, cplx* Pbph, cplx* SPibar, const FLBar& FLb, const Dims& d, const RowMask& rm) {
+    k_adj_sx<<<nb((size_t)3 * d.Nq * d.NPO * 32, 128), 128, 0, s>>>(Pipp, Piph, FL, SXbar, Pbpp, Pbph, SPibar, FLb, d, rm);
     LCHK(); return cudaSuccess;
 }
 cudaError_t launch_adj_L_K2(cudaStream_t s, const BubbleP& B, const VertBar& Fb, const cplx* rawbar, const ChanWork& cw,

@@ -94,9 +94,10 @@ __device__ __forceinline__ C prod2(C a, C da, C b, C db) {
 
 // TAN: the tangent bubbles dΠ from G and its tangent tG (product rule, the tails are constant)
 template <bool TAN>
-__global__ void k_bubble_local(const cplx* G, const cplx* tG, cplx* pp, cplx* ph, Dims d) {
+__global__ void k_bubble_local(const cplx* G, const cplx* tG, cplx* pp, cplx* ph, Dims d, RowMask rm) {
     size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
     if (i >= (size_t)d.NPO * d.NPw) return;
+    if (rm.row && !rm.row[i / d.NPw]) return;
     const int n = (int)(i % d.NPw) - d.nPw, m = (int)(i / d.NPw) - (d.nPO - 1);
     const cplx Gn = g_tail(G, d, 0, n);
     if (!TAN) {
@@ -117,14 +118,15 @@ __global__ void k_bubble_local(const cplx* G, const cplx* tG, cplx* pp, cplx* ph
 // C: arithmetic type (FP64, or FP32 for the mixed map's bubble from the FP32 copy of G(R)); G:
 // storage of G(R).  The twiddles are staged in shared memory in C.
 template <bool TAN, class C, class G>
-__global__ void k_bubble_nl(const G* GR, const G* tGR, cplx* pp, cplx* ph, const cplx* twp, Dims d, int TV) {
+__global__ void k_bubble_nl(const G* GR, const G* tGR, cplx* pp, cplx* ph, const cplx* twp, Dims d, int TV,
+                            RowMask rm) {
     extern __shared__ __align__(16) unsigned char sh_raw[];
     const int L = d.L, NR = L * L;
     C* A = reinterpret_cast<C*>(sh_raw);  // [2][TV][NR]   (pp, ph) in R
     C* B = A + 2 * (size_t)TV * NR;       // [2][TV][NR]  after the x transform
     C* tw = B + 2 * (size_t)TV * NR;      // [L]
     for (int j = threadIdx.x; j < L; j += blockDim.x) tw[j] = to_c<C>(twp[j]);
-    const int m = blockIdx.y - (d.nPO - 1);
+    const int iO = rm.oms ? rm.oms[blockIdx.y] : (int)blockIdx.y, m = iO - (d.nPO - 1);
     const int n0 = blockIdx.x * TV - d.nPw;
     for (int e = threadIdx.x; e < TV * NR; e += blockDim.x) {
         const int v = e / NR, R = e % NR;
@@ -172,7 +174,7 @@ __global__ void k_bubble_nl(const G* GR, const G* tGR, cplx* pp, cplx* ph, const
         const int P = rest % NR, which = rest / NR;
         const int Px = P % L, Py = P / L;
         const int n = n0 + v;
-        if (n >= d.nPw) continue;
+        if (n >= d.nPw || (rm.row && !rm.row[(size_t)P * d.NPO + iO])) continue;
         const C* b = B + (size_t)(which * TV + v) * NR;
         C s{0, 0};
         for (int y = 0; y < L; ++y) s = cfma(b[(size_t)y * L + Px], tw[(Py * y) % L], s);
@@ -268,12 +270,15 @@ __device__ __forceinline__ void fft_bwd_any(C (&v)[L]) {
     else fft_bwd_3m<L>(v);
 }
 
+// Bound by the FP64 pipe (about 60 operations per 8-point transform, 32 of them per (Ω, ν)).  rm leaves out the
+// Ω that no work item has and the stores of the momenta outside the irreducible wedge: Hubbard 8x8,
+// nK3 = (8, 12) on GB300 81 -> 50 us with the tile of bubble_fill; S_X (k_sx) 24 -> 11 us.
 template <int L, class C, class G, bool TAN>
-__global__ void k_bubble_fft(const G* GR, const G* tGR, cplx* pp, cplx* ph, Dims d, int TV) {
+__global__ void k_bubble_fft(const G* GR, const G* tGR, cplx* pp, cplx* ph, Dims d, int TV, RowMask rm) {
     extern __shared__ __align__(16) unsigned char sh_raw[];
     C* sh = reinterpret_cast<C*>(sh_raw);
     constexpr int NR = L * L, RS = L + 1, BS = L * (L + 1) + 1;
-    const int m = blockIdx.y - (d.nPO - 1);
+    const int iO = rm.oms ? rm.oms[blockIdx.y] : (int)blockIdx.y, m = iO - (d.nPO - 1);
     const int n0 = blockIdx.x * TV - d.nPw;
     for (int e = threadIdx.x; e < TV * NR; e += blockDim.x) {
         const int v = e / NR, R = e % NR;
@@ -329,7 +334,7 @@ __global__ void k_bubble_fft(const G* GR, const G* tGR, cplx* pp, cplx* ph, Dims
         const int rest = e / TV;
         const int P = rest % NR, which = rest / NR;
         const int n = n0 + v;
-        if (n >= d.nPw) continue;
+        if (n >= d.nPw || (rm.row && !rm.row[(size_t)P * d.NPO + iO])) continue;
         const C val = sh[(size_t)(which * TV + v) * BS + (P / L) * RS + (P % L)];
         (which ? ph : pp)[ixPi(d, P, m, n)] = to_d(val);
     }
@@ -596,11 +601,12 @@ __global__ void __launch_bounds__(256) k_build_cache_tab(VertPT<S> F, Caches C, 
 // ---------------------------------------------------------------------------------------------
 // Bubble row sums SΠ(P, Ω) = Σ_ν Π(P, Ω, ν) over the whole bubble mesh; blockIdx.y = array.
 // ---------------------------------------------------------------------------------------------
-__global__ void k_rowsum(const cplx* A0, const cplx* A1, cplx* S0, cplx* S1, int rowlen) {
+__global__ void k_rowsum(const cplx* A0, const cplx* A1, cplx* S0, cplx* S1, int rowlen, RowMask rm) {
     __shared__ double rx[256], ry[256];
     const cplx* A = blockIdx.y ? A1 : A0;
     cplx* S = blockIdx.y ? S1 : S0;
     const size_t row = blockIdx.x;
+    if (rm.row && !rm.row[row]) return;
     double sx = 0.0, sy = 0.0;
     for (int i = threadIdx.x; i < rowlen; i += blockDim.x) {
         const cplx v = A[row * rowlen + i];
@@ -638,7 +644,7 @@ __global__ void k_tail_const(cplx* T0, Dims d) {
 }
 // TAN: row sums of the tangent bubbles (product rule with tGR; the tails and T0 are constant)
 template <class C, class G, bool TAN>
-__global__ void k_pisum_R(const G* GR, const G* tGR, const cplx* T0, cplx* SR, Dims d) {
+__global__ void k_pisum_R(const G* GR, const G* tGR, const cplx* T0, cplx* SR, Dims d, RowMask rm) {
     const int NR = d.L * d.L;
     const size_t w = (blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
@@ -646,6 +652,7 @@ __global__ void k_pisum_R(const G* GR, const G* tGR, const cplx* T0, cplx* SR, D
     const int which = (int)(w / ((size_t)d.NPO * NR));
     const int rest = (int)(w % ((size_t)d.NPO * NR));
     const int R = rest / d.NPO, m = rest % d.NPO - (d.nPO - 1);  // SR[w][R][Ω]
+    if (rm.om && !rm.om[rest % d.NPO]) return;
     const int L = d.L, Rx = R % L, Ry = R / L;
     const int mR = ((L - Rx) % L) + L * ((L - Ry) % L);
     C acc{0, 0};
@@ -687,13 +694,14 @@ __global__ void k_pisum_R(const G* GR, const G* tGR, const cplx* T0, cplx* SR, D
 // A Vertex-valued F0 adds (Π-Π0)(Ω,ω) [F0(Ω,ω̃,∞) - U] = (SΠ - SΠ0) k0 + Σ_{ω̃ ∈ F0's K2 box}
 // (Π-Π0)(ω) [f0_right(ω̃) - k0], k0 = its own channel's K1 (f0_right at ω̃ = ∞).
 __global__ void k_sx(const cplx* Pipp, const cplx* Piph, const cplx* Pi0pp, const cplx* Pi0ph, const cplx* SPi,
-                     const cplx* SPi0, FLP FL, VertP F0v, cplx* SX, Dims d) {
+                     const cplx* SPi0, FLP FL, VertP F0v, cplx* SX, Dims d, RowMask rm) {
     const size_t per = (size_t)d.Nq * d.NPO;
     const size_t i = (blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5;  // warp per output
     const int lane = threadIdx.x & 31;
     if (i >= 3 * per) return;
     const int ch = (int)(i / per);
     const size_t r = i % per;
+    if (rm.row && !rm.row[r]) return;
     const int m = (int)(r % d.NPO) - (d.nPO - 1), P = (int)(r / d.NPO);
     const int w = (ch == CH_P) ? 0 : 1;
     const cplx* Pi = w ? Piph : Pipp;
@@ -729,13 +737,14 @@ __global__ void k_sx(const cplx* Pipp, const cplx* Piph, const cplx* Pi0pp, cons
 
 // Tangent of S_X: dS_X = dSΠ U + Σ_ω [dΠ FL(Ω,ω̃,∞) + Π dFL(Ω,ω̃,∞)]  (SΠ0 is constant).
 __global__ void k_sx_tan(const cplx* Pipp, const cplx* Piph, const cplx* tPipp, const cplx* tPiph, const cplx* tSPi,
-                         FLP FL, FLP tFL, VertP F0v, cplx* tSX, Dims d) {
+                         FLP FL, FLP tFL, VertP F0v, cplx* tSX, Dims d, RowMask rm) {
     const size_t per = (size_t)d.Nq * d.NPO;
     const size_t i = (blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (i >= 3 * per) return;
     const int ch = (int)(i / per);
     const size_t r = i % per;
+    if (rm.row && !rm.row[r]) return;
     const int m = (int)(r % d.NPO) - (d.nPO - 1), P = (int)(r / d.NPO);
     const int w = (ch == CH_P) ? 0 : 1;
     const cplx* Pi = w ? Piph : Pipp;
@@ -1565,8 +1574,9 @@ __global__ void k_sde_L_all(VertPT<S> Fin, BubbleP B, const cplx* SPpp, const cp
 // BSE_K2! (src/BSEa/BSEa_K2.jl:95-101), then the t-channel pSp recombination (γtd + γa)/2
 // (src/BSE_templates.jl:35-38).  Slots are indexed by channel; an absent slot has out = nullptr.
 __global__ void k_finalize3(Finalize3 f, int k2_epilogue, int t_recombine, size_t n) {
-    const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+    size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
     if (i >= n) return;
+    if (f.blocks) i = (size_t)f.blocks[i / f.bs] * f.bs + i % f.bs;
     cplx v[3];
     uint32_t e_prev = 0;
     const uint32_t* map_prev = nullptr;
@@ -1792,19 +1802,29 @@ cudaError_t launch_occupation(cudaStream_t s, const cplx* G, size_t n, double T,
 cudaError_t launch_g_realspace(cudaStream_t s, const cplx* G, cplx* GR, const cplx* tw, const Dims& d) {
     return launch_fft2(s, G, GR, d.NG, -1, 1.0 / (d.L * d.L), tw, d);
 }
+// The ν per CTA of a bubble launch: the largest power of two from the start value `tv` down that gives at
+// least four CTAs per SM of GB300 (the FFT passes of a CTA are short and separated by barriers; over all rows
+// Hubbard 8x8 takes 81 us at one CTA of 32 ν per SM and 68 at four); 8 ν keep the stores on whole 128-byte
+// lines.
+static int bubble_fill(int tv, const Dims& d, const RowMask& rm) {
+    const int nO = rm.oms ? rm.noms : d.NPO;
+    while (tv > 8 && (d.NPw + tv - 1) / tv * nO < 4 * 152) tv >>= 1;
+    return tv;
+}
 // DFT bubble (any L): TV fermion frequencies per CTA, (4 TV L² + L) values of shared memory
 template <bool TAN, class C, class G>
 static cudaError_t launch_bubble_dft(cudaStream_t s, const G* GR, const G* tGR, cplx* pp, cplx* ph, const cplx* twp,
-                                     const Dims& d) {
+                                     const Dims& d, const RowMask& rm) {
     const int NR = d.L * d.L;
     int tv = 32;
     while (tv > 1 && (size_t)(4 * tv * NR + d.L) * sizeof(C) > 160 * 1024) tv >>= 1;
+    tv = bubble_fill(tv, d, rm);
     const size_t shm = (size_t)(4 * tv * NR + d.L) * sizeof(C);
     static SmemRecord shm_set;  // raised once, outside graph capture (first call is from fdga_finalize)
     cudaError_t e = raise_smem_limit(k_bubble_nl<TAN, C, G>, shm_set, shm);
     if (e != cudaSuccess) return e;
-    dim3 grid((d.NPw + tv - 1) / tv, d.NPO);
-    k_bubble_nl<TAN, C, G><<<grid, 256, shm, s>>>(GR, tGR, pp, ph, twp, d, tv);
+    dim3 grid((d.NPw + tv - 1) / tv, rm.oms ? rm.noms : d.NPO);
+    k_bubble_nl<TAN, C, G><<<grid, 256, shm, s>>>(GR, tGR, pp, ph, twp, d, tv, rm);
     LAUNCH_CHECK(); return cudaSuccess;
 }
 int bubble_tile(const Dims& d) {
@@ -1815,53 +1835,56 @@ int bubble_tile(const Dims& d) {
 }
 template <int L, bool TAN>
 static cudaError_t launch_bubble_fft(cudaStream_t s, const cplx* GR, const cplx* tGR, cplx* pp, cplx* ph,
-                                     const Dims& d) {
+                                     const Dims& d, const RowMask& rm) {
     constexpr int BS = L * (L + 1) + 1;
     int tv = 32;
     while (tv > 1 && (size_t)2 * tv * BS * sizeof(cplx) > 80 * 1024) tv >>= 1;
+    tv = bubble_fill(tv, d, rm);
     const size_t shm = (size_t)2 * tv * BS * sizeof(cplx);
     static SmemRecord shm_set;  // raised once, outside graph capture (first call is from fdga_finalize)
     cudaError_t e = raise_smem_limit(k_bubble_fft<L, cplx, cplx, TAN>, shm_set, shm);
     if (e != cudaSuccess) return e;
-    dim3 grid((d.NPw + tv - 1) / tv, d.NPO);
-    k_bubble_fft<L, cplx, cplx, TAN><<<grid, 256, shm, s>>>(GR, tGR, pp, ph, d, tv);
+    dim3 grid((d.NPw + tv - 1) / tv, rm.oms ? rm.noms : d.NPO);
+    k_bubble_fft<L, cplx, cplx, TAN><<<grid, 256, shm, s>>>(GR, tGR, pp, ph, d, tv, rm);
     return cudaGetLastError();
 }
 // FP32 form (mixed map) from the FP32 copy of G(R); its tile fits the default 48 KB of shared memory
 template <int L, bool TAN>
 static cudaError_t launch_bubble_fft_f32(cudaStream_t s, const cplxf* GR, const cplxf* tGR, cplx* pp, cplx* ph,
-                                         const Dims& d) {
+                                         const Dims& d, const RowMask& rm) {
     constexpr int BS = L * (L + 1) + 1;
     int tv = 32;
     while (tv > 1 && (size_t)2 * tv * BS * sizeof(cplxf) > 48 * 1024) tv >>= 1;
+    tv = bubble_fill(tv, d, rm);
     const size_t shm = (size_t)2 * tv * BS * sizeof(cplxf);
-    dim3 grid((d.NPw + tv - 1) / tv, d.NPO);
-    k_bubble_fft<L, cplxf, cplxf, TAN><<<grid, 256, shm, s>>>(GR, tGR, pp, ph, d, tv);
+    dim3 grid((d.NPw + tv - 1) / tv, rm.oms ? rm.noms : d.NPO);
+    k_bubble_fft<L, cplxf, cplxf, TAN><<<grid, 256, shm, s>>>(GR, tGR, pp, ph, d, tv, rm);
     return cudaGetLastError();
 }
 bool bubble_f32_supported(const Dims& d) { return !d.local; }
 template <bool TAN>
 static cudaError_t bubble_f32_t(cudaStream_t s, const cplxf* GRf, const cplxf* tGRf, cplx* pp, cplx* ph,
-                                const cplx* twp, const Dims& d) {
+                                const cplx* twp, const Dims& d, const RowMask& rm) {
     switch (d.L) {
-        case 2: return launch_bubble_fft_f32<2, TAN>(s, GRf, tGRf, pp, ph, d);
-        case 4: return launch_bubble_fft_f32<4, TAN>(s, GRf, tGRf, pp, ph, d);
-        case 8: return launch_bubble_fft_f32<8, TAN>(s, GRf, tGRf, pp, ph, d);
-        case 16: return launch_bubble_fft_f32<16, TAN>(s, GRf, tGRf, pp, ph, d);
-        case 32: return launch_bubble_fft_f32<32, TAN>(s, GRf, tGRf, pp, ph, d);
-        case 3: return launch_bubble_fft_f32<3, TAN>(s, GRf, tGRf, pp, ph, d);
-        case 6: return launch_bubble_fft_f32<6, TAN>(s, GRf, tGRf, pp, ph, d);
-        case 12: return launch_bubble_fft_f32<12, TAN>(s, GRf, tGRf, pp, ph, d);
-        case 24: return launch_bubble_fft_f32<24, TAN>(s, GRf, tGRf, pp, ph, d);
-        default: return launch_bubble_dft<TAN, cplxf, cplxf>(s, GRf, tGRf, pp, ph, twp, d);
+        case 2: return launch_bubble_fft_f32<2, TAN>(s, GRf, tGRf, pp, ph, d, rm);
+        case 4: return launch_bubble_fft_f32<4, TAN>(s, GRf, tGRf, pp, ph, d, rm);
+        case 8: return launch_bubble_fft_f32<8, TAN>(s, GRf, tGRf, pp, ph, d, rm);
+        case 16: return launch_bubble_fft_f32<16, TAN>(s, GRf, tGRf, pp, ph, d, rm);
+        case 32: return launch_bubble_fft_f32<32, TAN>(s, GRf, tGRf, pp, ph, d, rm);
+        case 3: return launch_bubble_fft_f32<3, TAN>(s, GRf, tGRf, pp, ph, d, rm);
+        case 6: return launch_bubble_fft_f32<6, TAN>(s, GRf, tGRf, pp, ph, d, rm);
+        case 12: return launch_bubble_fft_f32<12, TAN>(s, GRf, tGRf, pp, ph, d, rm);
+        case 24: return launch_bubble_fft_f32<24, TAN>(s, GRf, tGRf, pp, ph, d, rm);
+        default: return launch_bubble_dft<TAN, cplxf, cplxf>(s, GRf, tGRf, pp, ph, twp, d, rm);
     }
 }
-cudaError_t launch_bubble_f32(cudaStream_t s, const cplxf* GRf, cplx* pp, cplx* ph, const cplx* twp, const Dims& d) {
-    return bubble_f32_t<false>(s, GRf, nullptr, pp, ph, twp, d);
+cudaError_t launch_bubble_f32(cudaStream_t s, const cplxf* GRf, cplx* pp, cplx* ph, const cplx* twp, const Dims& d,
+                              const RowMask& rm) {
+    return bubble_f32_t<false>(s, GRf, nullptr, pp, ph, twp, d, rm);
 }
 cudaError_t launch_bubble_f32_tan(cudaStream_t s, const cplxf* GRf, const cplxf* tGRf, cplx* tpp, cplx* tph,
-                                  const cplx* twp, const Dims& d) {
-    return bubble_f32_t<true>(s, GRf, tGRf, tpp, tph, twp, d);
+                                  const cplx* twp, const Dims& d, const RowMask& rm) {
+    return bubble_f32_t<true>(s, GRf, tGRf, tpp, tph, twp, d, rm);
 }
 
 cudaError_t set_fft_twiddles() {
@@ -1886,33 +1909,33 @@ cudaError_t set_fft_twiddles() {
 
 template <bool TAN>
 static cudaError_t bubble_t(cudaStream_t s, const cplx* G, const cplx* tG, const cplx* GR, const cplx* tGR, cplx* pp,
-                            cplx* ph, const cplx* twp, const Dims& d) {
+                            cplx* ph, const cplx* twp, const Dims& d, const RowMask& rm) {
     if (d.local) {
         const size_t n = (size_t)d.NPO * d.NPw;
-        k_bubble_local<TAN><<<blocks_for(n, 256), 256, 0, s>>>(G, tG, pp, ph, d);
+        k_bubble_local<TAN><<<blocks_for(n, 256), 256, 0, s>>>(G, tG, pp, ph, d, rm);
         LAUNCH_CHECK(); return cudaSuccess;
     }
     switch (d.L) {
-        case 2: return launch_bubble_fft<2, TAN>(s, GR, tGR, pp, ph, d);
-        case 4: return launch_bubble_fft<4, TAN>(s, GR, tGR, pp, ph, d);
-        case 8: return launch_bubble_fft<8, TAN>(s, GR, tGR, pp, ph, d);
-        case 16: return launch_bubble_fft<16, TAN>(s, GR, tGR, pp, ph, d);
-        case 32: return launch_bubble_fft<32, TAN>(s, GR, tGR, pp, ph, d);
-        case 3: return launch_bubble_fft<3, TAN>(s, GR, tGR, pp, ph, d);
-        case 6: return launch_bubble_fft<6, TAN>(s, GR, tGR, pp, ph, d);
-        case 12: return launch_bubble_fft<12, TAN>(s, GR, tGR, pp, ph, d);
-        case 24: return launch_bubble_fft<24, TAN>(s, GR, tGR, pp, ph, d);
+        case 2: return launch_bubble_fft<2, TAN>(s, GR, tGR, pp, ph, d, rm);
+        case 4: return launch_bubble_fft<4, TAN>(s, GR, tGR, pp, ph, d, rm);
+        case 8: return launch_bubble_fft<8, TAN>(s, GR, tGR, pp, ph, d, rm);
+        case 16: return launch_bubble_fft<16, TAN>(s, GR, tGR, pp, ph, d, rm);
+        case 32: return launch_bubble_fft<32, TAN>(s, GR, tGR, pp, ph, d, rm);
+        case 3: return launch_bubble_fft<3, TAN>(s, GR, tGR, pp, ph, d, rm);
+        case 6: return launch_bubble_fft<6, TAN>(s, GR, tGR, pp, ph, d, rm);
+        case 12: return launch_bubble_fft<12, TAN>(s, GR, tGR, pp, ph, d, rm);
+        case 24: return launch_bubble_fft<24, TAN>(s, GR, tGR, pp, ph, d, rm);
         default: break;
     }
-    return launch_bubble_dft<TAN, cplx, cplx>(s, GR, tGR, pp, ph, twp, d);
+    return launch_bubble_dft<TAN, cplx, cplx>(s, GR, tGR, pp, ph, twp, d, rm);
 }
 cudaError_t launch_bubble(cudaStream_t s, const cplx* G, const cplx* GR, cplx* pp, cplx* ph, const cplx* twp,
-                          const Dims& d) {
-    return bubble_t<false>(s, G, nullptr, GR, nullptr, pp, ph, twp, d);
+                          const Dims& d, const RowMask& rm) {
+    return bubble_t<false>(s, G, nullptr, GR, nullptr, pp, ph, twp, d, rm);
 }
 cudaError_t launch_bubble_tan(cudaStream_t s, const cplx* G, const cplx* tG, const cplx* GR, const cplx* tGR,
-                              cplx* tpp, cplx* tph, const cplx* twp, const Dims& d) {
-    return bubble_t<true>(s, G, tG, GR, tGR, tpp, tph, twp, d);
+                              cplx* tpp, cplx* tph, const cplx* twp, const Dims& d, const RowMask& rm) {
+    return bubble_t<true>(s, G, tG, GR, tGR, tpp, tph, twp, d, rm);
 }
 
 template <int L>
@@ -1958,16 +1981,17 @@ cudaError_t launch_tail_const(cudaStream_t s, cplx* T0, const Dims& d) {
     LAUNCH_CHECK(); return cudaSuccess;
 }
 cudaError_t launch_rowsum(cudaStream_t s, const cplx* A0, const cplx* A1, const cplx* GR, cplx* SRtmp, const cplx* twp,
-                          cplx* S0, cplx* S1, const Dims& d, const cplx* T0, const cplxf* GRf) {
+                          cplx* S0, cplx* S1, const Dims& d, const cplx* T0, const cplxf* GRf,
+                          const RowMask& rm) {
     if (d.nPw == d.nPn) {  // the full mesh is stored: sum the rows
         dim3 grid((unsigned)(d.Nq * d.NPO), 2);
-        k_rowsum<<<grid, 256, 0, s>>>(A0, A1, S0, S1, d.NPw);
+        k_rowsum<<<grid, 256, 0, s>>>(A0, A1, S0, S1, d.NPw, rm);
         LAUNCH_CHECK(); return cudaSuccess;
     }
     const int NR = d.L * d.L;
     const unsigned nb = blocks_for((size_t)2 * d.NPO * NR * 32, 128);
-    if (GRf) k_pisum_R<cplxf, cplxf, false><<<nb, 128, 0, s>>>(GRf, nullptr, T0, SRtmp, d);
-    else k_pisum_R<cplx, cplx, false><<<nb, 128, 0, s>>>(GR, nullptr, T0, SRtmp, d);
+    if (GRf) k_pisum_R<cplxf, cplxf, false><<<nb, 128, 0, s>>>(GRf, nullptr, T0, SRtmp, d, rm);
+    else k_pisum_R<cplx, cplx, false><<<nb, 128, 0, s>>>(GR, nullptr, T0, SRtmp, d, rm);
     LAUNCH_CHECK();
     // S^w[P][Ω] = Σ_R e^{+2πi P·R/L} SR[w][R][Ω]
     cudaError_t e = launch_fft2(s, SRtmp, S0, d.NPO, +1, 1.0, twp, d);
@@ -1977,9 +2001,9 @@ cudaError_t launch_rowsum(cudaStream_t s, const cplx* A0, const cplx* A1, const 
     return cudaSuccess;
 }
 cudaError_t launch_sx(cudaStream_t s, const BubbleP& B, const cplx* SPi, const cplx* SPi0, const FLP& FL,
-                      const VertP& F0v, cplx* SX, const Dims& d) {
+                      const VertP& F0v, cplx* SX, const Dims& d, const RowMask& rm) {
     const size_t n = (size_t)3 * d.Nq * d.NPO * 32;
-    k_sx<<<blocks_for(n, 128), 128, 0, s>>>(B.pp, B.ph, B.pp0, B.ph0, SPi, SPi0, FL, F0v, SX, d);
+    k_sx<<<blocks_for(n, 128), 128, 0, s>>>(B.pp, B.ph, B.pp0, B.ph0, SPi, SPi0, FL, F0v, SX, d, rm);
     LAUNCH_CHECK(); return cudaSuccess;
 }
 
@@ -2244,23 +2268,23 @@ cudaError_t launch_dyson_tan(cudaStream_t s, cplx* tG, const cplx* G, const cplx
 }
 cudaError_t launch_sx_tan(cudaStream_t s, const cplx* Pipp, const cplx* Piph, const cplx* tPipp, const cplx* tPiph,
                           const cplx* tSPi, const FLP& FL, const FLP& tFL, const VertP& F0v, cplx* tSX,
-                          const Dims& d) {
+                          const Dims& d, const RowMask& rm) {
     const size_t n = (size_t)3 * d.Nq * d.NPO * 32;
-    k_sx_tan<<<blocks_for(n, 128), 128, 0, s>>>(Pipp, Piph, tPipp, tPiph, tSPi, FL, tFL, F0v, tSX, d);
+    k_sx_tan<<<blocks_for(n, 128), 128, 0, s>>>(Pipp, Piph, tPipp, tPiph, tSPi, FL, tFL, F0v, tSX, d, rm);
     LAUNCH_CHECK(); return cudaSuccess;
 }
 cudaError_t launch_rowsum_tan(cudaStream_t s, const cplx* tA0, const cplx* tA1, const cplx* GR, const cplx* tGR,
                               cplx* SRtmp, const cplx* twp, cplx* tS0, cplx* tS1, const Dims& d, const cplxf* GRf,
-                              const cplxf* tGRf) {
+                              const cplxf* tGRf, const RowMask& rm) {
     if (d.nPw == d.nPn) {  // the full mesh is stored: the row sums are linear in Π
         dim3 grid((unsigned)(d.Nq * d.NPO), 2);
-        k_rowsum<<<grid, 256, 0, s>>>(tA0, tA1, tS0, tS1, d.NPw);
+        k_rowsum<<<grid, 256, 0, s>>>(tA0, tA1, tS0, tS1, d.NPw, rm);
         LAUNCH_CHECK(); return cudaSuccess;
     }
     const int NR = d.L * d.L;
     const unsigned nb = blocks_for((size_t)2 * d.NPO * NR * 32, 128);
-    if (GRf) k_pisum_R<cplxf, cplxf, true><<<nb, 128, 0, s>>>(GRf, tGRf, nullptr, SRtmp, d);
-    else k_pisum_R<cplx, cplx, true><<<nb, 128, 0, s>>>(GR, tGR, nullptr, SRtmp, d);
+    if (GRf) k_pisum_R<cplxf, cplxf, true><<<nb, 128, 0, s>>>(GRf, tGRf, nullptr, SRtmp, d, rm);
+    else k_pisum_R<cplx, cplx, true><<<nb, 128, 0, s>>>(GR, tGR, nullptr, SRtmp, d, rm);
     LAUNCH_CHECK();
     cudaError_t e = launch_fft2(s, SRtmp, tS0, d.NPO, +1, 1.0, twp, d);
     if (e != cudaSuccess) return e;

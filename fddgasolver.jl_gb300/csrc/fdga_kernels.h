@@ -35,6 +35,15 @@ inline cudaError_t raise_smem_limit(K kernel, SmemRecord& raised, size_t bytes, 
     return e;
 }
 
+// The (P, Ω) rows of the bubbles that any work item reads: with symmetry groups the K1, K2 and K3
+// representatives and blocks lie in an irreducible wedge of the momenta and one sign of Ω, so the other
+// rows are not formed.  row [P][iΩ], om [iΩ] (any P), oms the list of those iΩ; null: every row.
+struct RowMask {
+    const uint8_t* row = nullptr;
+    const uint8_t* om = nullptr;
+    const int* oms = nullptr;
+    int noms = 0;
+};
 struct ChanArrays {  // read-only K arrays of the three channels
     const cplx* K1[3];
     const cplx* K2[3];
@@ -177,6 +186,8 @@ struct Finalize3 {  // indexed by channel (p, t, a)
     const uint32_t* map[3];
     const cplx* FL[3];
     cplxf* outf[3];  // optional FP32 copies of out (FL.K3 of the mixed map)
+    const int* blocks;  // optional: only these blocks of bs elements are formed (n counts their elements)
+    unsigned bs;
 };
 
 constexpr int AA_MAX = 64;  // largest Anderson memory of the device solver
@@ -263,19 +274,19 @@ cudaError_t launch_finalize3(cudaStream_t s, const Finalize3& f, int k2_epilogue
 // T0: the tail·tail part of the R = 0 row sums (launch_tail_const, once per solver);
 // GRf (optional): FP32 copy of G(R) -> the real-space row sums run in FP32 (mixed map)
 cudaError_t launch_rowsum(cudaStream_t s, const cplx* A0, const cplx* A1, const cplx* GR, cplx* SRtmp, const cplx* twp,
-                          cplx* S0, cplx* S1, const Dims& d, const cplx* T0, const cplxf* GRf = nullptr);
+                          cplx* S0, cplx* S1, const Dims& d, const cplx* T0, const cplxf* GRf = nullptr, const RowMask& rm = RowMask());
 cudaError_t launch_tail_const(cudaStream_t s, cplx* T0, const Dims& d);
 bool bubble_f32_supported(const Dims& d);
-cudaError_t launch_bubble_f32(cudaStream_t s, const cplxf* GRf, cplx* pp, cplx* ph, const cplx* twp, const Dims& d);
+cudaError_t launch_bubble_f32(cudaStream_t s, const cplxf* GRf, cplx* pp, cplx* ph, const cplx* twp, const Dims& d, const RowMask& rm = RowMask());
 // F0v: the FP64 vertex view whose reference vertex enters F0(Ω, ω̃, ∞) (only has0/g0/b0 are read)
 cudaError_t launch_sx(cudaStream_t s, const BubbleP& B, const cplx* SPi, const cplx* SPi0, const FLP& FL,
-                      const VertP& F0v, cplx* SX, const Dims& d);
+                      const VertP& F0v, cplx* SX, const Dims& d, const RowMask& rm = RowMask());
 cudaError_t launch_dyson(cudaStream_t s, cplx* G, const cplx* Sig, const cplx* Gb, size_t n);
 cudaError_t launch_occupation(cudaStream_t s, const cplx* G, size_t n, double T, int Nk, double* out);
 cudaError_t launch_g_realspace(cudaStream_t s, const cplx* G, cplx* GR, const cplx* tw, const Dims& d);
 int bubble_tile(const Dims& d);
 cudaError_t launch_bubble(cudaStream_t s, const cplx* G, const cplx* GR, cplx* pp, cplx* ph, const cplx* twp,
-                          const Dims& d);
+                          const Dims& d, const RowMask& rm = RowMask());
 cudaError_t launch_qavg(cudaStream_t s, const ChanArrays& in, const ChanArraysW& out, const Dims& d);
 cudaError_t launch_build_cache(cudaStream_t s, const VertP& F, const Caches& C, const int* blocks, int nblocks,
                                const Dims& d);
@@ -429,15 +440,15 @@ cudaError_t launch_nonfinite(cudaStream_t s, const cplx* a, size_t n, unsigned i
 // Π, L(R), C of the U² term) of the same base point are inputs
 cudaError_t launch_dyson_tan(cudaStream_t s, cplx* tG, const cplx* G, const cplx* tSig, size_t n);
 cudaError_t launch_bubble_tan(cudaStream_t s, const cplx* G, const cplx* tG, const cplx* GR, const cplx* tGR,
-                              cplx* tpp, cplx* tph, const cplx* twp, const Dims& d);
+                              cplx* tpp, cplx* tph, const cplx* twp, const Dims& d, const RowMask& rm = RowMask());
 cudaError_t launch_bubble_f32_tan(cudaStream_t s, const cplxf* GRf, const cplxf* tGRf, cplx* tpp, cplx* tph,
-                                  const cplx* twp, const Dims& d);
+                                  const cplx* twp, const Dims& d, const RowMask& rm = RowMask());
 cudaError_t launch_rowsum_tan(cudaStream_t s, const cplx* tA0, const cplx* tA1, const cplx* GR, const cplx* tGR,
                               cplx* SRtmp, const cplx* twp, cplx* tS0, cplx* tS1, const Dims& d,
-                              const cplxf* GRf = nullptr, const cplxf* tGRf = nullptr);
+                              const cplxf* GRf = nullptr, const cplxf* tGRf = nullptr, const RowMask& rm = RowMask());
 cudaError_t launch_sx_tan(cudaStream_t s, const cplx* Pipp, const cplx* Piph, const cplx* tPipp, const cplx* tPiph,
                           const cplx* tSPi, const FLP& FL, const FLP& tFL, const VertP& F0v, cplx* tSX,
-                          const Dims& d);
+                          const Dims& d, const RowMask& rm = RowMask());
 cudaError_t launch_sde_sigma_tan(cudaStream_t s, const cplx* GR, const cplx* LR, const cplx* tGR, const cplx* tLpp,
                                  const cplx* tLph, cplx* tLR, cplx* tSR, cplx* tS, const cplx* twm, const cplx* twp,
                                  const Dims& d);
@@ -465,7 +476,7 @@ cudaError_t launch_adj_K2(cudaStream_t s, const VertP& F, const FLP& FL, const B
                           const VertBar& Fb, const FLBar& FLb, cplx* Pbpp, cplx* Pbph, cplx* SXbar, const cplx* rawbar,
                           const ChanWork& cw, size_t n2, const Dims& d);
 cudaError_t launch_adj_sx(cudaStream_t s, const cplx* Pipp, const cplx* Piph, const FLP& FL, const cplx* SXbar,
-                          cplx* Pbpp, cplx* Pbph, cplx* SPibar, const FLBar& FLb, const Dims& d);
+                          cplx* Pbpp, cplx* Pbph, cplx* SPibar, const FLBar& FLb, const Dims& d, const RowMask& rm = RowMask());
 cudaError_t launch_adj_L_K2(cudaStream_t s, const BubbleP& B, const VertBar& Fb, const cplx* rawbar, const ChanWork& cw,
                             size_t n2, const Dims& d);
 cudaError_t launch_adj_cache(cudaStream_t s, const VertBar& Fb, const Caches& Cb, const int* blocks, int nblocks,

@@ -108,6 +108,10 @@ struct fdga_handle {
     cplxf* gtabf = nullptr;
     int* d_goms = nullptr;
     int ngoms = 0;
+    // bubble rows that the work items read (set with the symmetry groups)
+    uint8_t *d_prow = nullptr, *d_pom = nullptr;
+    int* d_poms = nullptr;
+    RowMask rm;
     double* occ = nullptr;
     double n0 = 0.5;
     uint32_t* perm = nullptr;  // reference flatten index -> device index
@@ -584,6 +588,16 @@ void k2_rows(const fdga_handle* h, const Group& g, ChanWork& cw, int ch) {
         ++nl;                                                        \
     } while (0)
 
+// FL.K3 is read at the K3 blocks of the work items only (the contraction's γL terms), so its class expansion
+// covers those blocks (Hubbard 8x8, nK3 = (20, 40): 404 us over all blocks, 101 over these); sets the
+// list and returns the number of elements.  fdga_get_named expands the rest on demand.
+size_t fl3_blocks(const fdga_handle* h, Finalize3& f) {
+    if (!h->d_k3blocks) return h->n3;
+    f.blocks = h->d_k3blocks;
+    f.bs = (unsigned)(h->d.N3n * h->d.N3n);
+    return (size_t)h->nk3blocks * f.bs;
+}
+
 // L_pp and L_ph (vertex part and/or RefVertex part / 3) at the K2-group representatives, then the
 // SymmetryGroup broadcast into h->Lpp, h->Lph.
 template <class V>
@@ -690,13 +704,13 @@ int enqueue_iteration(fdga_handle* h, int strategy, bool update_sigma, bool hart
         if (h->precision == FDGA_MIXED && bubble_f32_supported(d)) {
             // mixed map: bubble and its full-mesh row sums in FP32 from an FP32 copy of G(R)
             LC(launch_to_f32(sB, h->GR, h->GRf, h->nGk));
-            LC(launch_bubble_f32(sB, h->GRf, h->Pipp, h->Piph, h->twp, d));
+            LC(launch_bubble_f32(sB, h->GRf, h->Pipp, h->Piph, h->twp, d, h->rm));
             LC(launch_rowsum(sB, h->Pipp, h->Piph, h->GR, h->SRtmp, h->twp, h->SPi, h->SPi + (size_t)d.Nq * d.NPO, d,
-                             h->T0tail, h->GRf));
+                             h->T0tail, h->GRf, h->rm));
         } else {
-            LC(launch_bubble(sB, h->G, h->GR, h->Pipp, h->Piph, h->twp, d));
+            LC(launch_bubble(sB, h->G, h->GR, h->Pipp, h->Piph, h->twp, d, h->rm));
             LC(launch_rowsum(sB, h->Pipp, h->Piph, h->GR, h->SRtmp, h->twp, h->SPi, h->SPi + (size_t)d.Nq * d.NPO, d,
-                             h->T0tail));
+                             h->T0tail, nullptr, h->rm));
         }
         // the SDE's U² term and the occupation need only G: also on branch B
         LC(launch_u2(sB, h->GR, h->u2C, h->u2R, h->SigU2, h->twp, d));
@@ -815,7 +829,7 @@ int enqueue_iteration(fdga_handle* h, int strategy, bool update_sigma, bool hart
             Finalize3 f3 = fin(3, h->raw3, out, grp);
             if (mixed)
                 for (int c = 0; c < 3; ++c) f3.outf[c] = h->FLK3f + (size_t)c * h->n3;
-            LC(launch_finalize3(s, f3, 0, 1, h->n3));
+            LC(launch_finalize3(s, f3, 0, 1, fl3_blocks(h, f3)));
         }
         stage("bse_L_K3_finalize");
     }
@@ -839,7 +853,7 @@ int enqueue_iteration(fdga_handle* h, int strategy, bool update_sigma, bool hart
         CK(cudaStreamWaitEvent(sD, h->evD, 0));
     }
     // ω-sums of the right BSE factor (needs FL.K2 of this iteration)
-    if (!is_new) LC(launch_sx(sD, B, h->SPi, h->SPi0, FLz, F, h->SX, d));
+    if (!is_new) LC(launch_sx(sD, B, h->SPi, h->SPi0, FLz, F, h->SX, d, h->rm));
     {  // K1
         ChanWork cw = work(1, h->raw1);
         if (is_new && mixed) LC(launch_bse_K1_new(sD, Ff, B, h->SPi, h->SPi0, cw, d));
@@ -1005,12 +1019,13 @@ int enqueue_tangent(fdga_handle* h, int strategy, bool update_sigma, bool hartre
         LC(launch_g_realspace(sB, t.G, t.GR, h->twm, d));
         if (mixed && bubble_f32_supported(d)) {
             LC(launch_to_f32(sB, t.GR, t.GRf, h->nGk));
-            LC(launch_bubble_f32_tan(sB, h->GRf, t.GRf, t.Pipp, t.Piph, h->twp, d));
+            LC(launch_bubble_f32_tan(sB, h->GRf, t.GRf, t.Pipp, t.Piph, h->twp, d, h->rm));
             LC(launch_rowsum_tan(sB, t.Pipp, t.Piph, h->GR, t.GR, h->SRtmp, h->twp, t.SPi, t.SPi + nS, d, h->GRf,
-                                 t.GRf));
+                                 t.GRf, h->rm));
         } else {
-            LC(launch_bubble_tan(sB, h->G, t.G, h->GR, t.GR, t.Pipp, t.Piph, h->twp, d));
-            LC(launch_rowsum_tan(sB, t.Pipp, t.Piph, h->GR, t.GR, h->SRtmp, h->twp, t.SPi, t.SPi + nS, d));
+            LC(launch_bubble_tan(sB, h->G, t.G, h->GR, t.GR, t.Pipp, t.Piph, h->twp, d, h->rm));
+            LC(launch_rowsum_tan(sB, t.Pipp, t.Piph, h->GR, t.GR, h->SRtmp, h->twp, t.SPi, t.SPi + nS, d, nullptr,
+                                 nullptr, h->rm));
         }
     } else {  // G and Π are held fixed
         LC(cudaMemsetAsync(t.Pipp, 0, h->nPi * sizeof(cplx), sB));
@@ -1142,7 +1157,7 @@ int enqueue_tangent(fdga_handle* h, int strategy, bool update_sigma, bool hartre
             Finalize3 f3 = fin(3, h->raw3, out, grp);
             if (mixed)
                 for (int c = 0; c < 3; ++c) f3.outf[c] = t.FLK3f + (size_t)c * h->n3;
-            LC(launch_finalize3(s, f3, 0, 1, h->n3));
+            LC(launch_finalize3(s, f3, 0, 1, fl3_blocks(h, f3)));
         }
         stage("bse_L_K3");
     } else {  // scPA: FL is not iterated
@@ -1163,7 +1178,7 @@ int enqueue_tangent(fdga_handle* h, int strategy, bool update_sigma, bool hartre
         CK(cudaEventRecord(h->evD, s));
         CK(cudaStreamWaitEvent(sD, h->evD, 0));
     }
-    LC(launch_sx_tan(sD, h->Pipp, h->Piph, t.Pipp, t.Piph, t.SPi, FL, tFL, F, t.SX, d));
+    LC(launch_sx_tan(sD, h->Pipp, h->Piph, t.Pipp, t.Piph, t.SPi, FL, tFL, F, t.SX, d, h->rm));
     stage("sx");
     // tangent factors of the fused K1/K2/SDE kernels
     const TanArgs T64{tF, tFL, t.Pipp, t.Piph, t.SX, t.SPi, t.SPi + nS};
@@ -1466,7 +1481,7 @@ int enqueue_adjoint(fdga_handle* h, int strategy, bool update_sigma, bool hartre
         CK(fin_adj(ob, a.raw1, h->n1, grp, 0, 1, nullptr));
         CK(launch_adj_K1(s, F, FL, B, h->SX, Xb, FLb, a.Pbpp, a.Pbph, a.SXb, a.raw1, work(1), h->n1, d));
     }
-    CK(launch_adj_sx(s, h->Pipp, h->Piph, FL, a.SXb, a.Pbpp, a.Pbph, a.SPib, FLb, d));
+    CK(launch_adj_sx(s, h->Pipp, h->Piph, FL, a.SXb, a.Pbpp, a.Pbph, a.SPib, FLb, d, h->rm));
     if (strategy == FDGA_FDPA) {  // FL is iterated only in fdPA
         {  // FL.K3 = L_K3(Γ caches)
             const cplx* ob[3] = {FL3b[CH_P], FL3b[CH_T], FL3b[CH_A]};
@@ -2073,6 +2088,27 @@ int fdga_init_sym_grp(fdga_handle* h) {
         CK(cudaMemcpyAsync(h->d_goms, oms.data(), oms.size() * sizeof(int), cudaMemcpyHostToDevice, h->st));
         CK(cudaStreamSynchronize(h->st));
         h->ngoms = (int)oms.size();
+        // bubble rows (P, Ω) of the K1 and K2 representatives and of the K3 blocks
+        const Dims& d = h->d;
+        std::vector<uint8_t> row((size_t)d.Nq * d.NPO, 0), pom(d.NPO, 0);
+        auto need = [&](int P, int m) { row[(size_t)P * d.NPO + (m + d.nPO - 1)] = pom[m + d.nPO - 1] = 1; };
+        for (int r : hg[1].items) need(r / d.N1, r % d.N1 - (d.n1 - 1));
+        for (int i = 2; i < 4; ++i)
+            for (int r : hg[i].items) need(r / (d.N2n * d.N2O), (r / d.N2n) % d.N2O - (d.n2O - 1));
+        for (int b : blocks) need(b / d.N3O, b % d.N3O - (d.n3O - 1));
+        std::vector<int> poms;
+        for (int i = 0; i < d.NPO; ++i)
+            if (pom[i]) poms.push_back(i);
+        if (!h->d_prow) {
+            AL(h->d_prow, row.size());
+            AL(h->d_pom, pom.size());
+            AL(h->d_poms, pom.size());
+        }
+        CK(cudaMemcpyAsync(h->d_prow, row.data(), row.size(), cudaMemcpyHostToDevice, h->st));
+        CK(cudaMemcpyAsync(h->d_pom, pom.data(), pom.size(), cudaMemcpyHostToDevice, h->st));
+        CK(cudaMemcpyAsync(h->d_poms, poms.data(), poms.size() * sizeof(int), cudaMemcpyHostToDevice, h->st));
+        CK(cudaStreamSynchronize(h->st));
+        h->rm = RowMask{h->d_prow, h->d_pom, h->d_poms, (int)poms.size()};
     }
     drop_graphs(h);
     h->c0_dirty = true;
@@ -3526,6 +3562,18 @@ int fdga_get_named(fdga_handle* h, const char* name, double* out, size_t n) {
         cplx* o = reinterpret_cast<cplx*>(out);
         for (size_t j = 0; j < len; ++j) o[j] = dev[dev_index(h->d, kind, j)];
         return FDGA_OK;
+    }
+    if (h->d_k3blocks && p >= h->FLK3 && p < h->FLK3 + 3 * h->n3) {
+        // the iteration expands FL.K3 over the work items' blocks; inspection fills the others
+        CK(cudaMemcpyAsync(h->tmpS, h->FLK3, 3 * h->n3 * sizeof(cplx), cudaMemcpyDeviceToDevice, h->st));
+        Finalize3 f{};
+        const Group* grp[3] = {&h->gK3ppL, &h->gK3phL, &h->gK3phL};
+        for (int c = 0; c < 3; ++c) {
+            f.raw[c] = h->tmpS + (size_t)c * h->n3;
+            f.out[c] = h->FLK3 + (size_t)c * h->n3;
+            f.map[c] = grp[c]->d_map;
+        }
+        CK(launch_finalize3(h->st, f, 0, 0, h->n3));
     }
     CK(cudaMemcpyAsync(dev.data(), p, len * sizeof(cplx), cudaMemcpyDeviceToHost, h->st));
     CK(cudaStreamSynchronize(h->st));
