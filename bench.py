@@ -229,8 +229,9 @@ def k3_gemm_roofline(S, stages, cfg_name):
     """Roofline of the fused K3 BSE GEMM (MODE 1): one complex Nν3 x Nν3 x Nν3 product per (channel,
     representative (P, Ω) block); complex MAC = 8 real flops.  On the FP64 CUDA-core kernel
     (k_bse_K3_gemm) the FP64 pipe bounds it; on the digit-sliced tensor-core kernel (k_bse_K3_oz,
-    the default from Nν3 = 32 on) the BF16 MMAs it issues are compared with the measured bf16 peak
-    and its FP64-equivalent rate with the FP64 pipe."""
+    the default above Nν3 = 32) the 16-bit MMA work is compared with the measured bf16 peak
+    and its FP64-equivalent rate with the FP64 pipe.  `flops_per_launch` counts the 36 pairs of an
+    8-digit product, the yardstick; the kernel issues 28 (seven digits), `issued_*`."""
     nb, N = S.query("k3_blocks"), S.query("k3_block_dim")
     ms = stages["bse_K3_gemm"]
     flops = 3 * nb * 8 * N ** 3
@@ -239,15 +240,16 @@ def k3_gemm_roofline(S, stages, cfg_name):
     peaks = measured_peaks()
     hbm = peaks.get("hbm_gbs", 6800.0)
     achieved = flops / (ms * 1e-3) / 1e12
-    if S.query("k3_fp64_tensor_cores") == 1:
-        # 36 BF16 MMAs (M = 128 rows, K = 16) per K chunk over all 2N real columns and 2N real K
+    if S.query("k3_fp64_tensor_cores") == 1 and N > 32:
+        # 36 16-bit MMAs (M = 128 rows, K = 16) per K chunk over all 2N real columns and 2N real K
         mma_flops = 3 * nb * 36 * 2 * 128 * (2 * N) * (2 * N)
         bf16 = peaks.get("bf16_tflops", 1900.0)
         tc = mma_flops / (ms * 1e-3) / 1e12
         return {"bound": "tensor", "kernel": "k_bse_K3_oz<1> (fused K3 BSE, FP64 by digit slicing on tcgen05)",
                 "achieved": tc, "peak": bf16, "unit": "TFLOP/s", "frac": tc / bf16,
                 "peak_source": "fallback" if peaks.get("fallback") else "measured (bf16_tflops)",
-                "flops_per_launch": mma_flops, "fp64_equivalent_tflops": achieved, "fp64_pipe_peak": fp64_peak,
+                "flops_per_launch": mma_flops, "issued_flops_per_launch": mma_flops * 28 // 36,
+                "issued_frac": tc * 28 / 36 / bf16, "fp64_equivalent_tflops": achieved, "fp64_pipe_peak": fp64_peak,
                 "fp64_equivalent_frac": achieved / fp64_peak,
                 "traffic": profile_traffic(f"k_bse_K3_oz_{cfg_name}.md"), "algorithmic_bytes": byts,
                 "hbm_achieved_gbs": byts / (ms * 1e-3) / 1e9, "hbm_peak_gbs": hbm,

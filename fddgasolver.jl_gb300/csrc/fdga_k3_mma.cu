@@ -49,32 +49,11 @@ template <int NC> constexpr int PLANE = 8 * NC * PITCH<NC>;
 // planes [A or M][digit][re, im]
 template <int NC> constexpr int SMEM = 2 * S * 2 * PLANE<NC>;
 
-// v 2^(62+1022-F) rounded to an integer (0 for zero and subnormal v); |v| < 2^(F-1022)
-__device__ __forceinline__ long long fixed62(double v, int F) {
-    const unsigned long long b = (unsigned long long)__double_as_longlong(v);
-    const int ev = (int)((b >> 52) & 0x7ffull);
-    const int rs = F - ev - 9;
-    if (ev == 0 || rs >= 55) return 0;
-    const unsigned long long mant = (b & 0xFFFFFFFFFFFFFull) | (1ull << 52);
-    const long long y = (long long)(rs < 0 ? mant << (-rs) : (rs == 0 ? mant : (mant + (1ull << (rs - 1))) >> rs));
-    return (long long)b < 0 ? -y : y;
-}
-// digit k (from the least significant) of two biased integers as a pair of FP16 numbers
-__device__ __forceinline__ uint32_t digit_pair(unsigned long long a, unsigned long long b, int k) {
-    const uint32_t x = k < 4 ? (uint32_t)a : (uint32_t)(a >> 32), y = k < 4 ? (uint32_t)b : (uint32_t)(b >> 32);
-    const uint32_t i = (uint32_t)(k & 3);
-    const uint32_t u = (__byte_perm(x, y, i | ((4u + i) << 8)) & 0x00ff00ffu) | 0x64006400u;
-    uint32_t r;
-    asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"(u), "r"(0x64806480u));  // 0x6480 = 1152
-    return r;
-}
-constexpr unsigned long long BIAS = 0x8080808080808080ull;
-
 // the digits of two neighbouring ω of one row, both parts, stored to the planes at byte offset o
 template <int NC>
 __device__ __forceinline__ void store_digits(uint8_t* planes, int o, cplx v0, cplx v1, int F) {
-    const unsigned long long r0 = (unsigned long long)fixed62(v0.x, F) + BIAS, i0 = (unsigned long long)fixed62(v0.y, F) + BIAS;
-    const unsigned long long r1 = (unsigned long long)fixed62(v1.x, F) + BIAS, i1 = (unsigned long long)fixed62(v1.y, F) + BIAS;
+    const unsigned long long r0 = (unsigned long long)fixed_digits<S>(v0.x, F) + DIGIT_BIAS, i0 = (unsigned long long)fixed_digits<S>(v0.y, F) + DIGIT_BIAS;
+    const unsigned long long r1 = (unsigned long long)fixed_digits<S>(v1.x, F) + DIGIT_BIAS, i1 = (unsigned long long)fixed_digits<S>(v1.y, F) + DIGIT_BIAS;
 #pragma unroll
     for (int s = 0; s < S; ++s) {
         uint8_t* p = planes + (2 * s) * PLANE<NC> + o;
@@ -138,7 +117,6 @@ __device__ __forceinline__ void digit_product(uint8_t* sm, int (*fmax_)[8 * NC],
                     : "+f"(acc[s + t][0]), "+f"(acc[s + t][1]), "+f"(acc[s + t][2]), "+f"(acc[s + t][3])
                     : "r"(mr[s]), "r"(mi[s]), "r"(mi[s] ^ 0x80008000u), "r"(mr[s]), "r"(ar[t]), "r"(ai[t]));
     }
-    // D = 2^(F_A + F_M - 2044 - 124) Σ_g 256^(14-g) acc_g, joined as hi 256^11 + lo 256^7
     const int col = 8 * j + (lane >> 2);
     if (col >= N) return;
     const int FM = fmax_[1][col];
@@ -146,7 +124,7 @@ __device__ __forceinline__ void digit_product(uint8_t* sm, int (*fmax_)[8 * NC],
     for (int e = 0; e < 2; ++e) {
         const int nu = 8 * nt + 2 * (lane & 3) + e;
         if (nu >= N) continue;
-        const int FA = fmax_[0][nu], E = FA + FM - 2168;
+        const int FA = fmax_[0][nu], E = FA + FM;
         if (FA == 0x7ff || FM == 0x7ff) {
             const double qn = __longlong_as_double(0x7ff8000000000000ll);
             out(nu, col, mk(qn, qn), true);
@@ -155,14 +133,9 @@ __device__ __forceinline__ void digit_product(uint8_t* sm, int (*fmax_)[8 * NC],
         double p[2];
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
-            long long hi = 0, lo = 0;
-#pragma unroll
-            for (int g = 0; g < S; ++g) {
-                const long long v = (long long)__float2int_rn(acc[g][2 * q + e]);
-                if (g < 4) hi = hi * 256 + v;
-                else lo = lo * 256 + v;
-            }
-            p[q] = i2d_scaled(hi, E + 88) + i2d_scaled(lo, E + 56);
+            const float a[8] = {acc[0][2 * q + e], acc[1][2 * q + e], acc[2][2 * q + e], acc[3][2 * q + e],
+                                acc[4][2 * q + e], acc[5][2 * q + e], acc[6][2 * q + e], acc[7][2 * q + e]};
+            p[q] = join_digits<S>(a, E);
         }
         out(nu, col, mk(p[0], p[1]), false);
     }

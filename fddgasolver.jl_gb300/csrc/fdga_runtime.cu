@@ -80,13 +80,13 @@ struct fdga_handle {
     int fdpa_single_hartree = 0;  // option: subtract the reference system's Hartree term once
     size_t navg = 0;
     int* d_err = nullptr;                        // device error flag of bounded in-kernel waits
-    int* oz_fa = nullptr;                        // per-block exponent bounds of the digit-sliced K3 (3 Nq NΩ3)
+    int* oz_fa = nullptr;                        // row bounds of the digit-sliced K3 (3 Nq NΩ3 blocks of Nν3 rows)
     uint8_t* oz_adig = nullptr;                  // A digit operands of oz_adig_blocks blocks (at most 512 MB)
     int oz_adig_blocks = 0;
     int k3_tc = 1;                               // mixed K3 contractions on the tensor cores when supported
     int k3_tma = 1;                              // ... in the TMA-fed warp-specialised kernel when it fits
-    // FP64 K3 contractions on the tensor cores (exact digit slicing): 0 never, 1 where supported, 2 from
-    // Nν3 = 32 on, 3 as 1 with the FP64 exponent bound of M in every tile (tests)
+    // FP64 K3 contractions on the tensor cores (exact digit slicing): 0 never, 1 (and 3) tcgen05 where
+    // supported, 2 tcgen05 from Nν3 = 32 on and the warp-level kernel below
     int k3_oz = 2;
     int jvp_tangent = 1;                         // GMRES Jacobian products by the tangent kernels (else differences)
     int newton_cycles = 1;                       // GMRES restart cycles per Newton step
@@ -261,13 +261,13 @@ int ensure_mixed(fdga_handle* h) {
     return FDGA_OK;
 }
 // a tensor-core wait that timed out inside a kernel (bounded polling) is reported here
-// scratch of the digit-sliced K3: per-block exponent bounds and a digit buffer for up to 512 MB of
+// scratch of the digit-sliced K3: the row bounds and a digit buffer for up to 512 MB of
 // blocks (larger launches run in groups)
 int ensure_k3_oz(fdga_handle* h) {
     const Dims& d = h->d;
     const size_t nblk = 3 * (size_t)d.Nq * d.N3O;
     if (!h->d_err) AL(h->d_err, 1);
-    if (!h->oz_fa) AL(h->oz_fa, nblk);
+    if (!h->oz_fa) AL(h->oz_fa, nblk * d.N3n);
     if (!h->oz_adig) {
         const size_t per = k3_oz_digit_bytes(d);
         const size_t cap = std::max<size_t>(1, std::min(nblk, ((size_t)512 << 20) / per));
@@ -642,7 +642,7 @@ cudaError_t launch_k3_tensor_cores(fdga_handle* h, cudaStream_t s, int mode, con
 }
 
 // The FP64 K3 contractions (modes 0, 1 and the tangent's mode 2) by exact digit slicing: on tcgen05
-// (fdga_k3_oz.cu) from Nν3 = 32 on, on warp-level products (fdga_k3_mma.cu) below, where a 128-row
+// (fdga_k3_oz.cu) above Nν3 = 32, on warp-level products (fdga_k3_mma.cu) up to there, where a 128-row
 // accumulator stands mostly empty (Nν3 = 24, Hubbard 8x8: 23 / 37 us against 79 / 97).  The FP64 CUDA-core
 // GEMM runs the rest: Nν3 above 32 that is no multiple of 8 or passes 128, the tangent of the one-loop
 // form, and everything when the option is off.
@@ -653,9 +653,10 @@ bool use_k3_oz(const fdga_handle* h) {
 cudaError_t launch_k3_fp64(fdga_handle* h, cudaStream_t s, int mode, const K3Args3& a3) {
     bool oneloop = false;
     for (int i = 0; i < 3; ++i) oneloop |= (a3.a[i].flags & K3F_1LOOP) != 0;
-    if (use_k3_oz(h) && (mode <= 1 || !oneloop)) return launch_bse_K3_oz(s, mode, a3, 3, h->d, h->d_err, h->oz_fa, h->oz_adig, h->oz_adig_blocks,
-                                                                h->k3_oz == 3);
-    if (h->k3_oz == 2 && k3_mma_supported(h->d) && (mode <= 1 || !oneloop)) return launch_bse_K3_mma(s, mode, a3, 3, h->d);
+    const bool digits = mode <= 1 || !oneloop;
+    if (digits && h->k3_oz == 2 && k3_mma_supported(h->d)) return launch_bse_K3_mma(s, mode, a3, 3, h->d);
+    if (digits && use_k3_oz(h))
+        return launch_bse_K3_oz(s, mode, a3, 3, h->d, h->d_err, h->oz_fa, h->oz_adig, h->oz_adig_blocks);
     return launch_bse_K3(s, mode, a3, 3, h->d, 0, h->k3_tile[FDGA_FP64][mode < 2 ? mode : 1]);
 }
 
@@ -1973,7 +1974,7 @@ int fdga_finalize(fdga_handle* h) {
     CK(launch_rowsum(s, h->Pipp, h->Piph, h->GR, h->SRtmp, h->twp, h->SPi, h->SPi + nS, d, h->T0tail));
     if (k3_oz_supported(d)) {
         if (int r = ensure_k3_oz(h)) return r;
-        CK(prepare_bse_K3_oz());
+        CK(prepare_bse_K3_oz(h->d));
     }
     if (k3_mma_supported(d)) CK(prepare_bse_K3_mma(d));
     CK(cudaStreamSynchronize(s));
@@ -3610,7 +3611,7 @@ int fdga_set_option(fdga_handle* h, const char* key, int value) {
         if (value < 0 || value > 3) return fail(h, FDGA_ERR_ARG, "k3_fp64_tensor_cores takes 0, 1, 2 or 3");
         if (value && k3_oz_supported(h->d)) {
             if (int r = ensure_k3_oz(h)) return r;
-            CK(prepare_bse_K3_oz());
+            CK(prepare_bse_K3_oz(h->d));
             CK(cudaStreamSynchronize(h->st));
         }
         h->k3_oz = value;
