@@ -320,12 +320,12 @@ cudaError_t launch_u2(cudaStream_t s, const cplx* GR, cplx* C, cplx* SR, cplx* o
 cudaError_t launch_sigma_assemble(cudaStream_t s, const cplx* Sin, const cplx* SU2, const uint32_t* map,
                                   const double* occ, const cplx* C0, const cplx* Sig0, cplx* Sig, double U, int hartree,
                                   int fdpa, double n0, size_t n);
-cudaError_t launch_gather(cudaStream_t s, cplx* dst, const cplx* src, const uint32_t* perm, size_t n);
-cudaError_t launch_scatter(cudaStream_t s, cplx* dst, const cplx* src, const uint32_t* perm, size_t n);
+cudaError_t launch_gather(cudaStream_t s, cplx* dst, const cplx* src, size_t n, const Dims& d);
+cudaError_t launch_scatter(cudaStream_t s, cplx* dst, const cplx* src, size_t n, const Dims& d);
 cudaError_t launch_residual(cudaStream_t s, const cplx* y, const cplx* x, cplx* fx, cplx* g, double beta, double* pmax,
                             int nblk, size_t n);
 cudaError_t launch_sub(cudaStream_t s, cplx* out, const cplx* a, const cplx* b, size_t n);
-cudaError_t launch_gather_sub(cudaStream_t s, cplx* out, const cplx* y, const cplx* x, const uint32_t* perm, size_t n);
+cudaError_t launch_gather_sub(cudaStream_t s, cplx* out, const cplx* y, const cplx* x, size_t n, const Dims& d);
 cudaError_t launch_aa_keys(cudaStream_t s, int nblk, const uint32_t* code, uint32_t* src, double* w, size_t n);
 cudaError_t launch_aa_check(cudaStream_t s, int nblk, const cplx* x, const uint32_t* code, const uint32_t* src,
                             unsigned int* count, size_t n);

@@ -114,7 +114,6 @@ struct fdga_handle {
     RowMask rm;
     double* occ = nullptr;
     double n0 = 0.5;
-    uint32_t* perm = nullptr;  // reference flatten index -> device index
     Group gSig, gK1, gK2pp, gK2ph, gK3pp, gK3ph, gK3ppL, gK3phL;
     Graph graphs[2][5][2][2];  // [precision][strategy][update_sigma][hartree]
     // fdga_residual on page-locked host buffers: one graph with the copies inside (see residual_graph)
@@ -1873,7 +1872,6 @@ int fdga_create(const fdga_config* c, fdga_handle** out) {
     if (d.Nq > 1 && !h->has0) ALC(h->gtab, gamma_table_len(d));
     h->ngoms = d.N2O;
     ALC(h->occ, 1);
-    ALC(h->perm, h->nstate);
     ALC(h->d_part, NBLK_RED);
     // the zero-fills of dalloc are queued on the (non-blocking) solver stream: finish them before
     // any upload, and keep the uploads on the same stream
@@ -1886,25 +1884,11 @@ int fdga_create(const fdga_config* c, fdga_handle** out) {
             tp[j] = mk(std::cos(a), std::sin(a));
         }
         if (cudaMemcpyAsync(h->twm, tm.data(), d.L * sizeof(cplx), cudaMemcpyHostToDevice, h->st) != cudaSuccess ||
-            cudaMemcpyAsync(h->twp, tp.data(), d.L * sizeof(cplx), cudaMemcpyHostToDevice, h->st) != cudaSuccess)
-            return fin_err(fail(h, FDGA_ERR_CUDA, "twiddle upload"));
-        // flatten permutation
-        std::vector<uint32_t> perm(h->nstate);
-        size_t j = 0;
-        for (int ch : {CH_P, CH_T, CH_A}) {
-            const size_t off = (size_t)ch * h->nchan;
-            for (size_t i = 0; i < h->n1; ++i) perm[j++] = (uint32_t)(off + dev_index(h->d, AK_K1, i));
-            for (size_t i = 0; i < h->n2; ++i) perm[j++] = (uint32_t)(off + h->n1 + dev_index(h->d, AK_K2, i));
-            for (size_t i = 0; i < h->n3; ++i) perm[j++] = (uint32_t)(off + h->n1 + h->n2 + dev_index(h->d, AK_K3, i));
-        }
-        for (size_t i = 0; i < h->nGk; ++i) perm[j++] = (uint32_t)(3 * h->nchan + i);
-        if (cudaMemcpyAsync(h->perm, perm.data(), h->nstate * sizeof(uint32_t), cudaMemcpyHostToDevice, h->st) !=
-                cudaSuccess ||
+            cudaMemcpyAsync(h->twp, tp.data(), d.L * sizeof(cplx), cudaMemcpyHostToDevice, h->st) != cudaSuccess ||
             cudaStreamSynchronize(h->st) != cudaSuccess)
-            return fin_err(fail(h, FDGA_ERR_CUDA, "permutation upload"));
+            return fin_err(fail(h, FDGA_ERR_CUDA, "twiddle upload"));
     }
 #undef ALC
-    if (cudaStreamSynchronize(h->st) != cudaSuccess) return fin_err(fail(h, FDGA_ERR_CUDA, "create sync"));
     if (c->precision == FDGA_MIXED) {
         if ((r = ensure_mixed(h))) return fin_err(r);
         h->precision = FDGA_MIXED;
@@ -2140,7 +2124,7 @@ int fdga_state_len(const fdga_handle* h, size_t* n) {
 int fdga_flatten(fdga_handle* h, double* x, size_t n) {
     if (!h || !x) return fail(h, FDGA_ERR_ARG, "null argument");
     if (n != h->nstate) return fail(h, FDGA_ERR_ARG, "state length mismatch");
-    CK(launch_gather(h->st, h->tmpS, h->xS, h->perm, n));
+    CK(launch_gather(h->st, h->tmpS, h->xS, n, h->d));
     CK(cudaMemcpyAsync(x, h->tmpS, n * sizeof(cplx), cudaMemcpyDeviceToHost, h->st));
     CK(cudaStreamSynchronize(h->st));
     return FDGA_OK;
@@ -2150,7 +2134,7 @@ int fdga_unflatten(fdga_handle* h, const double* x, size_t n) {
     if (!h || !x) return fail(h, FDGA_ERR_ARG, "null argument");
     if (n != h->nstate) return fail(h, FDGA_ERR_ARG, "state length mismatch");
     CK(cudaMemcpyAsync(h->tmpS, x, n * sizeof(cplx), cudaMemcpyHostToDevice, h->st));
-    CK(launch_scatter(h->st, h->xS, h->tmpS, h->perm, n));
+    CK(launch_scatter(h->st, h->xS, h->tmpS, n, h->d));
     CK(cudaStreamSynchronize(h->st));
     return FDGA_OK;
 }
@@ -2198,13 +2182,13 @@ int residual_graph(fdga_handle* h, int strategy, const double* x, double* R) {
         IterHooks hk;
         hk.after_fork = [&]() -> int {
             CK(cudaMemcpyAsync(h->tmpS, xh, nv * sizeof(cplx), cudaMemcpyHostToDevice, s));
-            CK(launch_scatter(s, h->xS, h->tmpS, h->perm, nv));
+            CK(launch_scatter(s, h->xS, h->tmpS, nv, h->d));
             return FDGA_OK;
         };
         hk.vertex_done = [&]() -> int {
             CK(cudaEventRecord(h->evR, s));
             CK(cudaStreamWaitEvent(sE, h->evR, 0));
-            CK(launch_gather_sub(sE, h->tmpS, h->yS, h->xS, h->perm, nv));
+            CK(launch_gather_sub(sE, h->tmpS, h->yS, h->xS, nv, h->d));
             CK(cudaMemcpyAsync(Rh, h->tmpS, nv * sizeof(cplx), cudaMemcpyDeviceToHost, sE));
             CK(cudaEventRecord(h->evR, sE));
             return FDGA_OK;
@@ -2251,13 +2235,13 @@ int fdga_residual(fdga_handle* h, int strategy, const double* x, double* R, size
     if (!h->finalized) return fail(h, FDGA_ERR_STATE, "fdga_finalize has not been called");
     if (h->fused_residual && page_locked(x) && page_locked(R)) return residual_graph(h, strategy, x, R);
     CK(cudaMemcpyAsync(h->tmpS, x, n * sizeof(cplx), cudaMemcpyHostToDevice, h->st));
-    CK(launch_scatter(h->st, h->xS, h->tmpS, h->perm, n));
+    CK(launch_scatter(h->st, h->xS, h->tmpS, n, h->d));
     int r = run_iteration(h, strategy, true, true);
     if (r) return r;
     // R = flatten(Φ(x)) - x, formed in device layout then permuted
     CK(launch_sub(h->st, h->tmpS, h->yS, h->xS, n));
     CK(cudaMemcpyAsync(h->xS, h->yS, n * sizeof(cplx), cudaMemcpyDeviceToDevice, h->st));
-    CK(launch_gather(h->st, h->yS, h->tmpS, h->perm, n));
+    CK(launch_gather(h->st, h->yS, h->tmpS, n, h->d));
     CK(cudaMemcpyAsync(R, h->yS, n * sizeof(cplx), cudaMemcpyDeviceToHost, h->st));
     CK(cudaStreamSynchronize(h->st));
     return check_device_error(h);
@@ -3240,7 +3224,7 @@ int fdga_jvp(fdga_handle* h, int strategy, const double* v, double* Jv, size_t n
     cplx *x = h->kr_x, *tmp = h->jv[0], *dir = h->jv[1], *yp = h->jv[2];
     CK(cudaMemcpyAsync(x, h->xS, n * sizeof(cplx), cudaMemcpyDeviceToDevice, h->st));
     CK(cudaMemcpyAsync(tmp, v, n * sizeof(cplx), cudaMemcpyHostToDevice, h->st));
-    CK(launch_scatter(h->st, dir, tmp, h->perm, n));  // reference layout -> device layout
+    CK(launch_scatter(h->st, dir, tmp, n, h->d));  // reference layout -> device layout
     // full-space central difference (v need not be symmetric): Jv = (Φ(x + εv) − Φ(x − εv))/(2ε)
     if (!h->kr_part) {
         r = dalloc(h, &h->kr_part, (size_t)(KR_MAX + 2) * NBLK_RED);
@@ -3267,7 +3251,7 @@ int fdga_jvp(fdga_handle* h, int strategy, const double* v, double* Jv, size_t n
     if ((r = run_iteration(h, strategy, true, true))) return r;
     CK(launch_kr_resid(h->st, NBLK_RED, nullptr, nullptr, 0.0, yp, h->yS, 0.5 / eps, tmp, n));
     CK(cudaMemcpyAsync(h->xS, x, n * sizeof(cplx), cudaMemcpyDeviceToDevice, h->st));
-    CK(launch_gather(h->st, h->yS, tmp, h->perm, n));
+    CK(launch_gather(h->st, h->yS, tmp, n, h->d));
     CK(cudaMemcpyAsync(Jv, h->yS, n * sizeof(cplx), cudaMemcpyDeviceToHost, h->st));
     CK(cudaStreamSynchronize(h->st));
     return FDGA_OK;
@@ -3285,14 +3269,14 @@ int fdga_frule(fdga_handle* h, int strategy, int update_sigma, int compute_hartr
     // value pass at x (leaves the intermediates of the base point in the handle), then the tangent
     if ((r = run_iteration(h, strategy, update_sigma != 0, compute_hartree != 0))) return r;
     CK(cudaMemcpyAsync(h->tmpS, v, n * sizeof(cplx), cudaMemcpyHostToDevice, h->st));
-    CK(launch_scatter(h->st, h->tan.x, h->tmpS, h->perm, n));  // reference layout -> device layout
+    CK(launch_scatter(h->st, h->tan.x, h->tmpS, n, h->d));  // reference layout -> device layout
     if ((r = run_tangent(h, strategy, update_sigma != 0, compute_hartree != 0))) return r;
     if ((r = check_device_error(h))) return r;
-    CK(launch_gather(h->st, h->tmpS, h->tan.y, h->perm, n));
+    CK(launch_gather(h->st, h->tmpS, h->tan.y, n, h->d));
     CK(cudaMemcpyAsync(Jv, h->tmpS, n * sizeof(cplx), cudaMemcpyDeviceToHost, h->st));
     CK(cudaStreamSynchronize(h->st));
     if (y) {
-        CK(launch_gather(h->st, h->tmpS, h->yS, h->perm, n));
+        CK(launch_gather(h->st, h->tmpS, h->yS, n, h->d));
         CK(cudaMemcpyAsync(y, h->tmpS, n * sizeof(cplx), cudaMemcpyDeviceToHost, h->st));
         CK(cudaStreamSynchronize(h->st));
     }
@@ -3316,13 +3300,13 @@ int fdga_rrule(fdga_handle* h, int strategy, int update_sigma, int compute_hartr
     h->precision = prec0;
     if (r) return r;
     CK(cudaMemcpyAsync(h->tmpS, ybar, n * sizeof(cplx), cudaMemcpyHostToDevice, h->st));
-    CK(launch_scatter(h->st, h->adj.yb, h->tmpS, h->perm, n));  // reference layout -> device layout
+    CK(launch_scatter(h->st, h->adj.yb, h->tmpS, n, h->d));  // reference layout -> device layout
     if ((r = run_adjoint(h, strategy, update_sigma != 0, compute_hartree != 0))) return r;
-    CK(launch_gather(h->st, h->tmpS, h->adj.xb, h->perm, n));
+    CK(launch_gather(h->st, h->tmpS, h->adj.xb, n, h->d));
     CK(cudaMemcpyAsync(xbar, h->tmpS, n * sizeof(cplx), cudaMemcpyDeviceToHost, h->st));
     CK(cudaStreamSynchronize(h->st));
     if (y) {
-        CK(launch_gather(h->st, h->tmpS, h->yS, h->perm, n));
+        CK(launch_gather(h->st, h->tmpS, h->yS, n, h->d));
         CK(cudaMemcpyAsync(y, h->tmpS, n * sizeof(cplx), cudaMemcpyDeviceToHost, h->st));
         CK(cudaStreamSynchronize(h->st));
     }
@@ -4076,12 +4060,12 @@ int fdga_mfrg_apply(fdga_handle* h, int strategy, const double* x, double* y, si
     if (n != nv) return fail(h, FDGA_ERR_ARG, "the mfRG map acts on the vertex part of the state (length(S.F))");
     cudaStream_t s = h->st;
     CK(cudaMemcpyAsync(h->tmpS, x, nv * sizeof(cplx), cudaMemcpyHostToDevice, s));
-    CK(launch_scatter(s, h->mf.u, h->tmpS, h->perm, nv));
+    CK(launch_scatter(s, h->mf.u, h->tmpS, nv, h->d));
     CK(launch_scale(s, h->mf.x, h->mf.u, kMfrgFactor, nv));
     if ((r = mfrg_prepare(h))) return r;
     if ((r = run_mfrg(h))) return r;
     CK(launch_kr_axpby(s, NBLK_RED, h->mf.u, h->mf.u, -1.0 / kMfrgFactor, h->mf.y, nv));
-    CK(launch_gather(s, h->tmpS, h->mf.u, h->perm, nv));
+    CK(launch_gather(s, h->tmpS, h->mf.u, nv, h->d));
     CK(cudaMemcpyAsync(y, h->tmpS, nv * sizeof(cplx), cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
     return check_device_error(h);
@@ -4103,7 +4087,7 @@ int fdga_residual_mfrg(fdga_handle* h, int strategy, const double* x, double* R,
     // x (unsymmetrised) in mf.u; the solver symmetrised from it in xS
     CK(cudaMemcpyAsync(h->tmpS, x, n * sizeof(cplx), cudaMemcpyHostToDevice, s));
     if (!update_sigma) CK(cudaMemcpyAsync(h->mf.u + nv, sigmaOf(h, h->xS), nS * sizeof(cplx), cudaMemcpyDeviceToDevice, s));
-    CK(launch_scatter(s, h->mf.u, h->tmpS, h->perm, n));
+    CK(launch_scatter(s, h->mf.u, h->tmpS, n, h->d));
     CK(cudaMemcpyAsync(h->xS, h->mf.u, h->nstate * sizeof(cplx), cudaMemcpyDeviceToDevice, s));
     if ((r = symmetrize_state(h))) return r;
     if ((r = run_iteration(h, strategy, update_sigma != 0, true))) return r;
@@ -4114,7 +4098,7 @@ int fdga_residual_mfrg(fdga_handle* h, int strategy, const double* x, double* R,
     CK(cudaMemsetAsync(h->mf.x, 0, nv * sizeof(cplx), s));
     CK(launch_kc_axpy(s, NBLK_RED, h->mf.x, h->kr64[2], h->kc_code, 1.0, h->mf.x, nv));
     if (update_sigma) CK(launch_sub(s, h->mf.x + nv, sigmaOf(h, h->yS), h->mf.u + nv, nS));
-    CK(launch_gather(s, h->tmpS, h->mf.x, h->perm, n));
+    CK(launch_gather(s, h->tmpS, h->mf.x, n, h->d));
     CK(cudaMemcpyAsync(R, h->tmpS, n * sizeof(cplx), cudaMemcpyDeviceToHost, s));
     CK(cudaMemcpyAsync(h->xS, h->yS, h->nstate * sizeof(cplx), cudaMemcpyDeviceToDevice, s));
     CK(cudaStreamSynchronize(s));
