@@ -947,7 +947,7 @@ __device__ __forceinline__ void bse_K2_row(const VertPT<S>& F, const FLPT<S>& FL
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
     const int lo = -d.nPw, hi = d.nPw - 1, h1 = d.xn1 - 1;
     const size_t is = (size_t)CH * d.Nq * d.NPO + (size_t)P * d.NPO + (m + d.nPO - 1);
-    for (int it = i0 + warp; it < i1; it += nwarps) {
+    for (int it = i0 + warp + nwarps * blockIdx.z; it < i1; it += nwarps * gridDim.z) {
         const int idx = items ? items[it] : it;
         const int nu = idx % d.N2n - d.n2n;
         const S c = k2_c<CH>(F, d, m, nu, P);
@@ -2119,9 +2119,16 @@ static unsigned row_grid(const ChanWork& cw, int nch) {
     for (int c = 0; c < nch; ++c) mx = std::max(mx, cw.ngroups[c]);
     return (unsigned)std::max(mx, 1);
 }
-// 4 warps per row; 16 when the launch has fewer than four rows per SM of GB300 (the local solver,
-// whose rows are only the NΩ2 bosonic frequencies)
-static unsigned row_threads(const ChanWork& cw, int nch) { return row_grid(cw, nch) * nch < 4 * 152 ? 512 : 128; }
+// K2: a CTA of 4 warps per row.  With fewer than four rows per SM of GB300 (the local solver, whose rows are only
+// the NΩ2 bosonic frequencies) 8 warps, and up to four CTAs share the items of a row, so that the FP64 work
+// spreads evenly over the SMs; each forms the row's factors anew, a small part.  One CTA of 16 warps per row
+// left some SMs with two rows and some with one: 69 us, now 43 us (SIAM, nK2 = (32, 32), nK3 = (16, 16)).
+static unsigned row_threads(const ChanWork& cw, int nch) { return row_grid(cw, nch) * nch < 4 * 152 ? 256 : 128; }
+static dim3 k2_grid(const ChanWork& cw, const Dims& d) {
+    const unsigned rows = row_grid(cw, 3), all = 3 * rows;
+    if (all >= 4 * 152) return dim3(rows, 3);
+    return dim3(rows, 3, std::min(std::min(4u, (8 * 152 + all - 1) / all), (unsigned)(d.N2n + 7) / 8));
+}
 template <class S, bool TAN>
 static size_t k2_row_smem(const Dims& d) {
     return (size_t)(TAN ? 2 : 1) * 2 * k2_table_half(d) * sizeof(S);
@@ -2177,7 +2184,7 @@ static cudaError_t k2_launch_attr(K k_plain, K k_v0, K k_tab, bool v0, bool tab,
         cudaError_t e = k2_launch_attr(k_bse_K2_all<ST, false, false, false>, k_bse_K2_all<ST, false, true, false>,     \
                                        k_bse_K2_all<ST, false, false, true>, F.has0, F.tab[0] != nullptr, smem); \
         if (e != cudaSuccess) return e;                                                                             \
-        const dim3 g(row_grid(cw, 3), 3);                                                                           \
+        const dim3 g = k2_grid(cw, d);                                                                              \
         if (F.tab[0]) k_bse_K2_all<ST, false, false, true><<<g, row_threads(cw, 3), smem, s>>>(F, FL, B, SX, cw, d, TT{}); \
         else if (F.has0) k_bse_K2_all<ST, false, true, false><<<g, row_threads(cw, 3), smem, s>>>(F, FL, B, SX, cw, d, TT{});    \
         else k_bse_K2_all<ST, false, false, false><<<g, row_threads(cw, 3), smem, s>>>(F, FL, B, SX, cw, d, TT{});         \
@@ -2203,7 +2210,7 @@ static cudaError_t k2_launch_attr(K k_plain, K k_v0, K k_tab, bool v0, bool tab,
         cudaError_t e = k2_launch_attr(k_bse_K2_all<ST, true, false, false>, k_bse_K2_all<ST, true, true, false>,     \
                                        k_bse_K2_all<ST, true, false, true>, F.has0, F.tab[0] != nullptr, smem);  \
         if (e != cudaSuccess) return e;                                                                             \
-        const dim3 g(row_grid(cw, 3), 3);                                                                           \
+        const dim3 g = k2_grid(cw, d);                                                                              \
         if (F.tab[0]) k_bse_K2_all<ST, true, false, true><<<g, row_threads(cw, 3), smem, s>>>(F, FL, B, SX, cw, d, T); \
         else if (F.has0) k_bse_K2_all<ST, true, true, false><<<g, row_threads(cw, 3), smem, s>>>(F, FL, B, SX, cw, d, T);        \
         else k_bse_K2_all<ST, true, false, false><<<g, row_threads(cw, 3), smem, s>>>(F, FL, B, SX, cw, d, T);             \
