@@ -26,30 +26,27 @@ __device__ __forceinline__ cplx cfnma(cplx a, cplx b, cplx c) {
     return mk(fma(-a.x, b.x, fma(a.y, b.y, c.x)), fma(-a.x, b.y, fma(-a.y, b.x, c.y)));
 }
 
-// Sum of part[0..np) in a fixed order, identical in every block; the result is valid in all threads.
-__device__ __forceinline__ cplx block_reduce_parts(const cplx* part, int np, cplx* sh) {
-    cplx s = mk(0.0, 0.0);
-    for (int i = threadIdx.x; i < np; i += RT) s += part[i];
-    sh[threadIdx.x] = s;
+// Block sum of per-thread values in a fixed order, valid in all threads: shuffles within the warps, then the
+// warps' sums in order.  One barrier; sh (one entry per warp) is used once per kernel.
+__device__ __forceinline__ cplx block_sum(cplx v, cplx (&sh)[RT / 32]) {
+    v = warp_sum(v);
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
     __syncthreads();
-    for (int o = RT / 2; o > 0; o >>= 1) {
-        if ((int)threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
-        __syncthreads();
-    }
-    const cplx r = sh[0];
-    __syncthreads();
+    cplx r = sh[0];
+#pragma unroll
+    for (int w = 1; w < RT / 32; ++w) r += sh[w];
     return r;
 }
-
+// Sum of part[0..np), identical in every block.
+__device__ __forceinline__ cplx block_reduce_parts(const cplx* part, int np, cplx (&sh)[RT / 32]) {
+    cplx s = mk(0.0, 0.0);
+    for (int i = threadIdx.x; i < np; i += RT) s += ld16(part + i);
+    return block_sum(s, sh);
+}
 // Block partial of a per-thread value, written to out[blockIdx.x].
-__device__ __forceinline__ void block_store_partial(cplx v, cplx* sh, cplx* out) {
-    sh[threadIdx.x] = v;
-    __syncthreads();
-    for (int o = RT / 2; o > 0; o >>= 1) {
-        if ((int)threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) out[blockIdx.x] = sh[0];
+__device__ __forceinline__ void block_store_partial(cplx v, cplx (&sh)[RT / 32], cplx* out) {
+    const cplx r = block_sum(v, sh);
+    if (threadIdx.x == 0) out[blockIdx.x] = r;
 }
 
 // Storage of the vectors.  Without symmetry groups every vector has one value per state element.
@@ -103,7 +100,7 @@ __global__ void __launch_bounds__(RT) k_aa_expand(cplx* x, const cplx* xr, const
 __global__ void __launch_bounds__(RT) k_aa_residual(const cplx* y, const cplx* xr, const uint32_t* code,
                                                     const uint32_t* src, cplx* fx, cplx* g, double beta, double* pmax,
                                                     size_t nr) {
-    __shared__ double red[RT];
+    __shared__ double red[RT / 32];
     double mx = 0.0;
     for (size_t k = blockIdx.x * (size_t)RT + threadIdx.x; k < nr; k += (size_t)gridDim.x * RT) {
         const cplx x = xr[k], f = key_value(y, code, src, k) - x;
@@ -111,13 +108,12 @@ __global__ void __launch_bounds__(RT) k_aa_residual(const cplx* y, const cplx* x
         g[k] = x + f * beta;
         mx = fmax(mx, f.x * f.x + f.y * f.y);
     }
-    red[threadIdx.x] = mx;
+    for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = mx;
     __syncthreads();
-    for (int o = RT / 2; o > 0; o >>= 1) {
-        if ((int)threadIdx.x < o) red[threadIdx.x] = fmax(red[threadIdx.x], red[threadIdx.x + o]);
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) pmax[blockIdx.x] = red[0];
+    if (threadIdx.x) return;
+    for (int w = 1; w < RT / 32; ++w) mx = fmax(mx, red[w]);
+    pmax[blockIdx.x] = mx;
 }
 
 // What bounds the step: at full length the FP64 pipe (about 200 FP64 instructions per element at
@@ -135,7 +131,7 @@ __global__ void __launch_bounds__(RT) k_aa_residual(const cplx* y, const cplx* x
 __global__ void __launch_bounds__(RT) k_aa_diff(cplx* dg, const cplx* g, const cplx* gold, cplx* df, const cplx* fx,
                                                 AAVecsW Q, int k, int nrot, const cplx* rot, const double* wgt,
                                                 cplx* part_out, size_t n) {
-    __shared__ cplx sh[RT];
+    __shared__ cplx sh[RT / 32];
     __shared__ cplx rs[2 * AA_MAX];
     for (int i = threadIdx.x; i < 2 * nrot; i += RT) rs[i] = rot[i];
     __syncthreads();
@@ -173,51 +169,73 @@ __global__ void __launch_bounds__(RT) k_aa_diff(cplx* dg, const cplx* g, const c
 __global__ void __launch_bounds__(RT) k_aa_mgs(cplx* df, const cplx* Qa, const cplx* part_in, int np, cplx* Rentry,
                                                const cplx* Qb, const cplx* fx, const double* wgt, cplx* part_out,
                                                cplx* pdot, size_t n) {
-    __shared__ cplx sh[RT];
-    const cplx r = block_reduce_parts(part_in, np, sh);
+    __shared__ cplx sh[3][RT / 32];
+    // (an element's loads are issued before the sum it waits for)
+    size_t i = blockIdx.x * (size_t)RT + threadIdx.x;
+    const size_t step = (size_t)gridDim.x * RT;
+    cplx a, v, wf, b;
+    double w = 1.0;
+    auto load = [&]() {
+        a = ld16(Qa + i); v = ld16(df + i); wf = ld16(fx + i);
+        if (Qb) b = ld16(Qb + i);
+        if (wgt) w = wgt[i];
+    };
+    if (i < n) load();
+    const cplx r = block_reduce_parts(part_in, np, sh[0]);
     if (blockIdx.x == 0 && threadIdx.x == 0) *Rentry = r;
     cplx s = mk(0.0, 0.0), q = mk(0.0, 0.0);
-    for (size_t i = blockIdx.x * (size_t)RT + threadIdx.x; i < n; i += (size_t)gridDim.x * RT) {
-        const cplx a = Qa[i];
-        const cplx v = cfnma(r, a, df[i]);
-        df[i] = v;
-        cplx wv = v, wf = fx[i];
-        if (wgt) { const double w = wgt[i]; wv = wv * w; wf = wf * w; }
+    while (i < n) {
+        v = cfnma(r, a, v);
+        st16(df + i, v);
+        cplx wv = v;
+        if (wgt) { wv = wv * w; wf = wf * w; }
         q = cfma_conj(a, wf, q);
-        if (Qb) s = cfma_conj(Qb[i], wv, s);
+        if (Qb) s = cfma_conj(b, wv, s);
         else s.x = fma(v.x, wv.x, fma(v.y, wv.y, s.x));
+        i += step;
+        if (i < n) load();
     }
-    block_store_partial(s, sh, part_out);
-    __syncthreads();
-    block_store_partial(q, sh, pdot);
+    block_store_partial(s, sh[1], part_out);
+    block_store_partial(q, sh[2], pdot);
 }
 
 // ‖Δf‖ = sqrt(Σ part_in), R(k,k) = ‖Δf‖, Q_k = Δf / ‖Δf‖, partial of <Q_k, fx>.
 __global__ void __launch_bounds__(RT) k_aa_qnew(cplx* Qk, const cplx* df, const cplx* part_in, int np, cplx* Rkk,
                                                 const cplx* fx, const double* wgt, cplx* pdot, size_t n) {
-    __shared__ cplx sh[RT];
-    const double nr = sqrt(fmax(0.0, block_reduce_parts(part_in, np, sh).x));
+    __shared__ cplx sh[2][RT / 32];
+    size_t i = blockIdx.x * (size_t)RT + threadIdx.x;
+    const size_t step = (size_t)gridDim.x * RT;
+    cplx v, wf;
+    double w = 1.0;
+    auto load = [&]() {
+        v = ld16(df + i); wf = ld16(fx + i);
+        if (wgt) w = wgt[i];
+    };
+    if (i < n) load();
+    const double nr = sqrt(fmax(0.0, block_reduce_parts(part_in, np, sh[0]).x));
     if (blockIdx.x == 0 && threadIdx.x == 0) *Rkk = mk(nr, 0.0);
     const double inv = 1.0 / nr;  // one division per block, not two per element
     cplx q = mk(0.0, 0.0);
-    for (size_t i = blockIdx.x * (size_t)RT + threadIdx.x; i < n; i += (size_t)gridDim.x * RT) {
-        const cplx v = df[i], u = mk(v.x * inv, v.y * inv);
-        Qk[i] = u;
-        cplx wf = fx[i];
-        if (wgt) wf = wf * wgt[i];
+    while (i < n) {
+        const cplx u = mk(v.x * inv, v.y * inv);
+        st16(Qk + i, u);
+        if (wgt) wf = wf * w;
         q = cfma_conj(u, wf, q);
+        i += step;
+        if (i < n) load();
     }
-    block_store_partial(q, sh, pdot);
+    block_store_partial(q, sh[1], pdot);
 }
 
 __device__ __forceinline__ double cabs_(cplx a) { return hypot(a.x, a.y); }
 // Deletion of the first column of the m x m QR factor by Givens rotations (NLsolve qrdelete!):
 // rotation i = 1..m-1 acts on rows (i-1, i) of R; the parameters go to rot[2(i-1)] = (c, -) and
 // rot[2(i-1)+1] = s; then the columns shift left by one.  One warp, a column of R per lane: the rotations
-// are a serial chain, the columns are not (one thread took 66 us at m = 8).
-__device__ __forceinline__ void givens_delete(cplx* R, int m, cplx* rot) {
+// are a serial chain, the columns are not (one thread took 66 us at m = 8).  Rs is the copy of R in shared
+// memory that the chain works on.
+__device__ __forceinline__ void givens_delete(cplx* Rs, cplx* R, int m, cplx* rot) {
     const int lane = threadIdx.x & 31;
-    auto Rr = [&](int i, int j) -> cplx& { return R[i + (size_t)m * j]; };
+    auto Rr = [&](int i, int j) -> cplx& { return Rs[i + (size_t)m * j]; };
     for (int i = 1; i < m; ++i) {
         const cplx f = Rr(i - 1, i), g = Rr(i, i);
         const double af = cabs_(f), ag = cabs_(g);
@@ -244,36 +262,68 @@ __device__ __forceinline__ void givens_delete(cplx* R, int m, cplx* rot) {
         }
         __syncwarp();
     }
-    for (int j = 0; j < m - 1; ++j) {
-        for (int i = lane; i < m - 1; i += 32) Rr(i, j) = Rr(i, j + 1);
-        __syncwarp();
+    for (int e = lane; e < m * m; e += 32) {
+        const int i = e % m, j = e / m;
+        R[e] = i < m - 1 && j < m - 1 ? Rr(i, j + 1) : Rr(i, j);
     }
 }
-__global__ void k_aa_givens(cplx* R, int m, cplx* rot) { givens_delete(R, m, rot); }
+__global__ void k_aa_givens(cplx* R, int m, cplx* rot) {
+    extern __shared__ __align__(16) unsigned char aa_sm[];
+    cplx* Rs = reinterpret_cast<cplx*>(aa_sm);
+    for (int e = threadIdx.x; e < m * m; e += 32) Rs[e] = R[e];
+    __syncwarp();
+    givens_delete(Rs, R, m, rot);
+}
 
-// γ = R⁻¹ (Σ_blocks part): one block; a warp per column of partials, then one warp back-substitutes
+// γ = R⁻¹ (Σ_blocks part): one block; a warp per column of partials, then warp 0 back-substitutes
 // (a row of R per lane).  R is column-major m x m.  del: the rotations of the next step's column
-// deletion follow in the same launch (R is not read by the update in between).
+// deletion in the same launch, on warp 1 and a second copy of R beside the rest (R is not read by the
+// update in between).  Serial chains of FP64 divisions bound it: R lies in shared memory and the parts of
+// the divisions by R_ii that do not wait for γ are done ahead for all rows at once.
 __global__ void __launch_bounds__(RT) k_aa_gamma(const cplx* part, int stride, int np, cplx* R, int m, int meff,
                                                  cplx* gam, int del, cplx* rot) {
+    extern __shared__ __align__(16) unsigned char aa_sm[];
     __shared__ cplx g[AA_MAX];
+    __shared__ cplx dv[AA_MAX];  // Smith's ratio and denominator of R_ii
+    cplx* Rs = reinterpret_cast<cplx*>(aa_sm);
+    cplx* Rg = Rs + (size_t)m * m;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int i = warp; i < meff; i += RT / 32) {
+    for (int e = threadIdx.x; e < m * m; e += RT) {
+        const cplx v = ld16(R + e);
+        Rs[e] = v;
+        if (del) Rg[e] = v;
+    }
+    __syncthreads();
+    if (warp == 1) {
+        if (del) givens_delete(Rg, R, m, rot);
+        return;
+    }
+    constexpr int NW = RT / 32 - 1;  // the other warps
+    for (int i = warp ? warp - 1 : 0; i < meff; i += NW) {
         cplx s = mk(0.0, 0.0);
-        for (int b = lane; b < np; b += 32) s += part[(size_t)i * stride + b];
+        for (int b = lane; b < np; b += 32) s += ld16(part + (size_t)i * stride + b);
         s = warp_sum(s);
         if (lane == 0) g[i] = s;
     }
-    __syncthreads();
+    if (warp == 0)
+        for (int i = lane; i < meff; i += 32) {
+            const cplx b = Rs[i + (size_t)m * i];
+            const bool big = fabs(b.x) >= fabs(b.y);
+            const double r = big ? b.y / b.x : b.x / b.y;
+            dv[i] = mk(r, big ? b.x + b.y * r : b.x * r + b.y);
+        }
+    asm volatile("bar.sync 1, %0;" ::"n"(32 * NW) : "memory");
     if (warp != 0) return;
     for (int i = meff - 1; i >= 0; --i) {
-        const cplx x = cdiv(g[i], R[i + (size_t)m * i]);
+        const cplx a = g[i], b = Rs[i + (size_t)m * i];
+        const double r = dv[i].x, den = dv[i].y;
+        const cplx x = fabs(b.x) >= fabs(b.y) ? mk((a.x + a.y * r) / den, (a.y - a.x * r) / den)
+                                              : mk((a.x * r + a.y) / den, (a.y * r - a.x) / den);
         __syncwarp();
-        if (lane == 0) { g[i] = x; gam[i] = x; }
-        for (int j = lane; j < i; j += 32) g[j] = cfnma(R[j + (size_t)m * i], x, g[j]);
+        if (lane == 0) gam[i] = x;
+        for (int j = lane; j < i; j += 32) g[j] = cfnma(Rs[j + (size_t)m * i], x, g[j]);
         __syncwarp();
     }
-    if (del) givens_delete(R, m, rot);
 }
 
 // x = g - Σ_i γ_i Δg_i (i in order) ; fxold = fx ; gold = g.
@@ -349,13 +399,21 @@ cudaError_t launch_aa_update(cudaStream_t s, int nblk, cplx* x, const cplx* g, c
 }
 cudaError_t launch_aa_givens(cudaStream_t s, cplx* R, int m, cplx* rot) {
     if (m < 2 || m > AA_MAX) return cudaErrorInvalidValue;
-    k_aa_givens<<<1, 32, 0, s>>>(R, m, rot);
+    const size_t smem = (size_t)m * m * sizeof(cplx);
+    static SmemRecord raised;
+    const cudaError_t e = raise_smem_limit(k_aa_givens, raised, smem);
+    if (e != cudaSuccess) return e;
+    k_aa_givens<<<1, 32, smem, s>>>(R, m, rot);
     AA_CHECK(); return cudaSuccess;
 }
 cudaError_t launch_aa_gamma(cudaStream_t s, const cplx* part, int stride, int np, cplx* R, int m, int meff, cplx* gam,
                             int del, cplx* rot) {
-    if (meff < 1 || meff > AA_MAX || (del && (m < 2 || meff != m))) return cudaErrorInvalidValue;
-    k_aa_gamma<<<1, RT, 0, s>>>(part, stride, np, R, m, meff, gam, del, rot);
+    if (meff < 1 || meff > m || m > AA_MAX || (del && (m < 2 || meff != m))) return cudaErrorInvalidValue;
+    const size_t smem = 2 * (size_t)m * m * sizeof(cplx);
+    static SmemRecord raised;
+    const cudaError_t e = raise_smem_limit(k_aa_gamma, raised, smem);
+    if (e != cudaSuccess) return e;
+    k_aa_gamma<<<1, RT, smem, s>>>(part, stride, np, R, m, meff, gam, del, rot);
     AA_CHECK(); return cudaSuccess;
 }
 
