@@ -131,7 +131,7 @@ struct fdga_handle {
     int last_launches = 0;
     cudaEvent_t ev[8] = {};
     cudaStream_t st2 = nullptr, st3 = nullptr;                         // branch streams of the iteration
-    cudaEvent_t evfork = nullptr, evA = nullptr, evB = nullptr, evC = nullptr, evD = nullptr, evE = nullptr,
+    cudaEvent_t evfork = nullptr, evA = nullptr, evB = nullptr, evC = nullptr, evD = nullptr, evE = nullptr, evK = nullptr, evF = nullptr,
                 evR = nullptr;
     // Anderson
     std::vector<cplx*> aa_buf;
@@ -675,8 +675,13 @@ int enqueue_iteration(fdga_handle* h, int strategy, bool update_sigma, bool hart
     VertP F = vertex_view(h, h->xS);
     VertP Fn = vertex_view(h, h->yS);  // Fbuff, i.e. the new F used by the SDE
     // Independent parts run as concurrent branches (graph capture and batches; sequential when the
-    // stages are timed): B = Dyson + bubbles + row sums, C = left K2 BSE, main = momentum averages,
-    // caches and left K3 BSE; both branches join the main stream before the right BSEs.
+    // stages are timed): B = Dyson + bubbles + row sums, then what the SDE needs of G alone; C = left K2 BSE
+    // (from the Γ table on); main = momentum averages, caches and left K3 BSE.  The row sums and the left K2
+    // join the main stream before the right BSEs.  Of those K1 runs behind branch B and K2 on branch D, beside
+    // the K3 contraction.  (With
+    // the left K2 behind the caches, K1 before K2 on one branch and the G part joined before the right BSEs the
+    // map took 83 / 162 / 345 / 219 us for SIAM nK3 = (4, 4) / (16, 16), Hubbard 8x8 (8, 12) / 4x4 (8, 16), so
+    // it takes 72 / 147 / 322 / 192.)
     const bool conc = !mark;
     cudaStream_t sB = conc ? h->st2 : s, sC = conc ? h->st3 : s;
     if (conc) {
@@ -712,13 +717,15 @@ int enqueue_iteration(fdga_handle* h, int strategy, bool update_sigma, bool hart
             LC(launch_rowsum(sB, h->Pipp, h->Piph, h->GR, h->SRtmp, h->twp, h->SPi, h->SPi + (size_t)d.Nq * d.NPO, d,
                              h->T0tail, nullptr, h->rm));
         }
-        // the SDE's U² term and the occupation need only G: also on branch B
+        if (conc) CK(cudaEventRecord(h->evB, sB));
+        // the SDE's U² term and the occupation need only G: also on branch B, joined by the SDE
         LC(launch_u2(sB, h->GR, h->u2C, h->u2R, h->SigU2, h->twp, d));
         nl += 2;
         LC(launch_occupation(sB, h->G, h->nGk, d.T, d.Nk, h->occ));
         stage("dyson_bubble");
+    } else if (conc) {
+        CK(cudaEventRecord(h->evB, sB));
     }
-    if (conc) CK(cudaEventRecord(h->evB, sB));
     // The mixed map evaluates vertices from an FP32 mirror of the state (converted once per
     // iteration) and keeps the caches, FL.K2 and FL.K3 in FP32: written once, read by the BSEs.
     const bool mixed = h->precision == FDGA_MIXED;
@@ -744,6 +751,7 @@ int enqueue_iteration(fdga_handle* h, int strategy, bool update_sigma, bool hart
         set_table(h, F, h->gtab);
         set_table(h, Ff, h->gtabf);
     }
+    if (conc) CK(cudaEventRecord(h->evA, s));  // branch C
     if (mixed) LC(launch_build_cache(s, Ff, C, h->d_k3blocks, h->nk3blocks, d));
     else LC(launch_build_cache(s, F, C, h->d_k3blocks, h->nk3blocks, d));
     // strategies that compute FL.K3 (:fdPA, :fdPA_new) write its FP32 copy in the finalize
@@ -785,10 +793,7 @@ int enqueue_iteration(fdga_handle* h, int strategy, bool update_sigma, bool hart
     // src/solve.jl:26-82: :fdPA computes FL.K2 and FL.K3, :fdPA_new FL.K3 only
     if (strategy == FDGA_FDPA) {
         {  // left K2 (FL.K2): branch C
-            if (conc) {
-                CK(cudaEventRecord(h->evA, s));
-                CK(cudaStreamWaitEvent(sC, h->evA, 0));
-            }
+            if (conc) CK(cudaStreamWaitEvent(sC, h->evA, 0));
             ChanWork cw = work(2, h->raw2);
             if (mixed) LC(launch_bse_L_K2_all(sC, Ff, B, cw, d));
             else LC(launch_bse_L_K2_all(sC, F, B, cw, d));
@@ -846,7 +851,7 @@ int enqueue_iteration(fdga_handle* h, int strategy, bool update_sigma, bool hart
             FLzf.K2[c] = h->FLzerof + (size_t)c * h->n2;
         }
     }
-    // K1 and K2 (branch D) run concurrently with the K3 contraction (main stream); the SDE joins
+    // K1 (branch B) and K2 (branch D) run concurrently with the K3 contraction (main stream); the SDE joins
     cudaStream_t sD = conc ? h->st3 : s;
     if (conc) {
         CK(cudaEventRecord(h->evD, s));
@@ -854,16 +859,21 @@ int enqueue_iteration(fdga_handle* h, int strategy, bool update_sigma, bool hart
     }
     // ω-sums of the right BSE factor (needs FL.K2 of this iteration)
     if (!is_new) LC(launch_sx(sD, B, h->SPi, h->SPi0, FLz, F, h->SX, d, h->rm));
+    if (conc) {
+        CK(cudaEventRecord(h->evK, sD));
+        CK(cudaStreamWaitEvent(sB, h->evK, 0));
+    }
     {  // K1
         ChanWork cw = work(1, h->raw1);
-        if (is_new && mixed) LC(launch_bse_K1_new(sD, Ff, B, h->SPi, h->SPi0, cw, d));
-        else if (is_new) LC(launch_bse_K1_new(sD, F, B, h->SPi, h->SPi0, cw, d));
-        else if (mixed) LC(launch_bse_K1_all(sD, Ff, FLzf, B, h->SX, cw, d));
-        else LC(launch_bse_K1_all(sD, F, FLz, B, h->SX, cw, d));
+        if (is_new && mixed) LC(launch_bse_K1_new(sB, Ff, B, h->SPi, h->SPi0, cw, d));
+        else if (is_new) LC(launch_bse_K1_new(sB, F, B, h->SPi, h->SPi0, cw, d));
+        else if (mixed) LC(launch_bse_K1_all(sB, Ff, FLzf, B, h->SX, cw, d));
+        else LC(launch_bse_K1_all(sB, F, FLz, B, h->SX, cw, d));
         cplx* out[3] = {chanK(h, h->yS, CH_P, 1), chanK(h, h->yS, CH_T, 1), chanK(h, h->yS, CH_A, 1)};
         const Group* grp[3] = {&h->gK1, &h->gK1, &h->gK1};
-        LC(launch_finalize3(sD, fin(1, h->raw1, out, grp), 0, 1, h->n1));
+        LC(launch_finalize3(sB, fin(1, h->raw1, out, grp), 0, 1, h->n1));
     }
+    if (conc) CK(cudaEventRecord(h->evF, sB));
     stage("bse_K1");
     {  // K2 (the _new form has no FL epilogue)
         ChanWork cw = work(2, h->raw2);
@@ -911,7 +921,10 @@ int enqueue_iteration(fdga_handle* h, int strategy, bool update_sigma, bool hart
         LC(launch_finalize3(s, fin(3, h->raw3, out, grp), 0, 1, h->n3));
     }
     stage("bse_K3_finalize");
-    if (conc) CK(cudaStreamWaitEvent(s, h->evE, 0));  // join: K1, K2 (D)
+    if (conc) {  // join: K2 (D), K1 and the SDE's part of G (B)
+        CK(cudaStreamWaitEvent(s, h->evE, 0));
+        CK(cudaStreamWaitEvent(s, h->evF, 0));
+    }
     if (hooks && hooks->vertex_done) {
         int r = hooks->vertex_done();
         if (r) return r;
@@ -1843,7 +1856,7 @@ int fdga_create(const fdga_config* c, fdga_handle** out) {
         fdga_destroy(h);
         return FDGA_ERR_CUDA;
     }
-    for (cudaEvent_t* e : {&h->evfork, &h->evA, &h->evB, &h->evC, &h->evD, &h->evE, &h->evR})
+    for (cudaEvent_t* e : {&h->evfork, &h->evA, &h->evB, &h->evC, &h->evD, &h->evE, &h->evK, &h->evF, &h->evR})
         cudaEventCreateWithFlags(e, cudaEventDisableTiming);
 #define ALC(ptr, n) do { r = dalloc(h, &(ptr), (n)); if (r) return fin_err(r); } while (0)
     ALC(h->Gbare, h->nGk); ALC(h->G0, h->nGk); ALC(h->Sig0, h->nGk); ALC(h->G, h->nGk);
@@ -1906,7 +1919,7 @@ void fdga_destroy(fdga_handle* h) {
     if (h->part_host) cudaFreeHost(h->part_host);
     for (void* p : h->allocs) cudaFree(p);
     for (auto& e : h->ev) if (e) cudaEventDestroy(e);
-    for (cudaEvent_t e : {h->evfork, h->evA, h->evB, h->evC, h->evD, h->evE, h->evR}) if (e) cudaEventDestroy(e);
+    for (cudaEvent_t e : {h->evfork, h->evA, h->evB, h->evC, h->evD, h->evE, h->evK, h->evF, h->evR}) if (e) cudaEventDestroy(e);
     for (cudaStream_t t : {h->st2, h->st3}) if (t) { cudaStreamSynchronize(t); cudaStreamDestroy(t); }
     if (h->st) cudaStreamDestroy(h->st);
     delete h;
