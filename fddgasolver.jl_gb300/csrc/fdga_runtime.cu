@@ -1009,8 +1009,8 @@ int enqueue_tangent(fdga_handle* h, int strategy, bool update_sigma, bool hartre
     VertP F = vertex_view(h, h->xS), Fn = vertex_view(h, h->yS);
     VertP tF = vertex_view_t<cplx>(h, t.x, t.avg, h->Fref), tFn = vertex_view_t<cplx>(h, t.y, t.avg, h->Fref);
     tF.noref = tFn.noref = 1;
-    // as in the value map, the Dyson/bubble tangents (branch B) and the left K2 tangent (branch C)
-    // run concurrently with the main stream's caches and left K3 when captured into a graph
+    // branches as in the value map: the Dyson/bubble tangents (B), the left K2 tangent from the Γ table on (C),
+    // then dK1 behind B and dK2 (D) beside the K3 contraction
     const bool conc = !mark;
     cudaStream_t sB = conc ? h->st2 : s, sC = conc ? h->st3 : s;
     if (conc) {
@@ -1045,13 +1045,13 @@ int enqueue_tangent(fdga_handle* h, int strategy, bool update_sigma, bool hartre
         LC(cudaMemsetAsync(t.Piph, 0, h->nPi * sizeof(cplx), sB));
         LC(cudaMemsetAsync(t.SPi, 0, 2 * nS * sizeof(cplx), sB));
     }
-    if (update_sigma) {  // the U² and occupation tangents need only dG: also on branch B
+    if (conc) CK(cudaEventRecord(h->evB, sB));
+    if (update_sigma) {  // the U² and occupation tangents need only dG: also on branch B, joined by the SDE
         LC(launch_u2_tan(sB, h->GR, h->u2C, t.GR, t.u2C, t.u2R, t.SigU2, h->twp, d));
         nl += 2;
         LC(launch_occupation(sB, t.G, h->nGk, d.T, d.Nk, t.occ));  // 1/2 + dn: the Hartree term reads dn
     }
     stage("dyson_bubble");
-    if (conc) CK(cudaEventRecord(h->evB, sB));
     // FP32 mirrors of the tangent vertex (mixed map); the value mirrors are the value pass's
     VertPF Ff{}, Fnf{}, tFf{}, tFnf{};
     FLPF FLf{}, tFLf{};
@@ -1085,6 +1085,7 @@ int enqueue_tangent(fdga_handle* h, int strategy, bool update_sigma, bool hartre
         set_table(h, tF, t.gtab);
         set_table(h, tFf, t.gtabf);
     }
+    if (conc) CK(cudaEventRecord(h->evA, s));  // branch C
     if (mixed) LC(launch_build_cache(s, tFf, tC, h->d_k3blocks, h->nk3blocks, d));
     else LC(launch_build_cache(s, tF, tC, h->d_k3blocks, h->nk3blocks, d));
     stage("k3_cache");
@@ -1132,10 +1133,7 @@ int enqueue_tangent(fdga_handle* h, int strategy, bool update_sigma, bool hartre
     };
     if (strategy == FDGA_FDPA) {
         {  // dFL.K2 = L_K2(dF)  (Π0 constant): branch C
-            if (conc) {
-                CK(cudaEventRecord(h->evA, s));
-                CK(cudaStreamWaitEvent(sC, h->evA, 0));
-            }
+            if (conc) CK(cudaStreamWaitEvent(sC, h->evA, 0));
             ChanWork cw = work(2, h->raw2, 0);
             if (mixed) LC(launch_bse_L_K2_all(sC, tFf, B, cw, d));
             else LC(launch_bse_L_K2_all(sC, tF, B, cw, d));
@@ -1185,7 +1183,7 @@ int enqueue_tangent(fdga_handle* h, int strategy, bool update_sigma, bool hartre
         CK(cudaStreamWaitEvent(s, h->evB, 0));
         if (strategy == FDGA_FDPA) CK(cudaStreamWaitEvent(s, h->evC, 0));
     }
-    // dK1 and dK2 (branch D) run concurrently with the K3 tangent (main stream)
+    // dK1 (branch B) and dK2 (branch D) run concurrently with the K3 tangent (main stream)
     cudaStream_t sD = conc ? h->st3 : s;
     if (conc) {
         CK(cudaEventRecord(h->evD, s));
@@ -1193,16 +1191,21 @@ int enqueue_tangent(fdga_handle* h, int strategy, bool update_sigma, bool hartre
     }
     LC(launch_sx_tan(sD, h->Pipp, h->Piph, t.Pipp, t.Piph, t.SPi, FL, tFL, F, t.SX, d, h->rm));
     stage("sx");
+    if (conc) {
+        CK(cudaEventRecord(h->evK, sD));
+        CK(cudaStreamWaitEvent(sB, h->evK, 0));
+    }
     // tangent factors of the fused K1/K2/SDE kernels
     const TanArgs T64{tF, tFL, t.Pipp, t.Piph, t.SX, t.SPi, t.SPi + nS};
     const TanArgsF T32{tFf, tFLf, t.Pipp, t.Piph, t.SX, t.SPi, t.SPi + nS};
     {  // dK1 = K1(dF; Π, FL, S_X) + K1(F; dΠ, dFL, dS_X), one pass
-        if (mixed) LC(launch_bse_K1_tan(sD, Ff, FLf, B, h->SX, T32, work(1, h->raw1, 0), d));
-        else LC(launch_bse_K1_tan(sD, F, FL, B, h->SX, T64, work(1, h->raw1, 0), d));
+        if (mixed) LC(launch_bse_K1_tan(sB, Ff, FLf, B, h->SX, T32, work(1, h->raw1, 0), d));
+        else LC(launch_bse_K1_tan(sB, F, FL, B, h->SX, T64, work(1, h->raw1, 0), d));
         cplx* out[3] = {chanK(h, t.y, CH_P, 1), chanK(h, t.y, CH_T, 1), chanK(h, t.y, CH_A, 1)};
         const Group* grp[3] = {&h->gK1, &h->gK1, &h->gK1};
-        LC(launch_finalize3(sD, fin(1, h->raw1, out, grp), 0, 1, h->n1));
+        LC(launch_finalize3(sB, fin(1, h->raw1, out, grp), 0, 1, h->n1));
     }
+    if (conc) CK(cudaEventRecord(h->evF, sB));
     stage("bse_K1");
     {  // dK2 likewise, then the FL epilogue with dFL.K2
         if (mixed) LC(launch_bse_K2_tan(sD, Ff, FLf, B, h->SX, T32, work(2, h->raw2, 0), d));
@@ -1251,7 +1254,10 @@ int enqueue_tangent(fdga_handle* h, int strategy, bool update_sigma, bool hartre
         LC(launch_finalize3(s, fin(3, h->raw3, out, grp), 0, 1, h->n3));
     }
     stage("bse_K3");
-    if (conc) CK(cudaStreamWaitEvent(s, h->evE, 0));  // join: dK1, dK2 (D)
+    if (conc) {  // join: dK2 (D), dK1 and the SDE's part of dG (B)
+        CK(cudaStreamWaitEvent(s, h->evE, 0));
+        CK(cudaStreamWaitEvent(s, h->evF, 0));
+    }
     cplx* tSig = sigmaOf(h, t.y);
     if (update_sigma) {
         const double rs = h->ref_nonzero ? 1.0 / 3.0 : 0.0;
