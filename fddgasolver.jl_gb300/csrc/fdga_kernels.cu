@@ -343,8 +343,11 @@ __global__ void k_bubble_fft(const G* GR, const G* tGR, cplx* pp, cplx* ph, Dims
 // Batched 2D transform over the L x L momentum grid: out[R][row] = scale Σ_P e^{sign 2πi P·R/L} in[P][row]
 // (momentum index x + L y outermost, `rows` contiguous values per momentum).  One CTA transforms TR
 // consecutive rows through shared memory (coalesced loads and stores along the rows).
+// blockIdx.y = 1: a second pair of arrays in the same launch (these launches are short: latency bounds them).
 template <int L>
-__global__ void k_fft2_rows(const cplx* in, cplx* out, int rows, int sign, double scale, int TR) {
+__global__ void k_fft2_rows(const cplx* in, cplx* out, const cplx* in2, cplx* out2, int rows, int sign, double scale,
+                            int TR) {
+    if (blockIdx.y) { in = in2; out = out2; }
     extern __shared__ cplx sh[];
     constexpr int NR = L * L, RS = L + 1, BS = L * (L + 1) + 1;
     const int r0 = blockIdx.x * TR;
@@ -2006,30 +2009,46 @@ cudaError_t launch_bubble_tan(cudaStream_t s, const cplx* G, const cplx* tG, con
 }
 
 template <int L>
-static cudaError_t launch_fft2_tpl(cudaStream_t s, const cplx* in, cplx* out, int rows, int sign, double scale) {
+static cudaError_t launch_fft2_tpl(cudaStream_t s, const cplx* in, cplx* out, const cplx* in2, cplx* out2, int rows,
+                                   int sign, double scale) {
     constexpr int BS = L * (L + 1) + 1, NR = L * L;
     // rows per CTA: enough CTAs to cover the GPU (two per SM for 152 SMs), within 48 KB of tile
     int tr = 1;
     while (tr < 32 && (size_t)(2 * tr) * BS * sizeof(cplx) <= 48 * 1024 && (rows + 2 * tr - 1) / (2 * tr) >= 304) tr *= 2;
     const size_t shm = (size_t)tr * BS * sizeof(cplx);
     const int threads = std::min(256, std::max(32, ((tr * NR + 31) / 32) * 32));
-    k_fft2_rows<L><<<(unsigned)((rows + tr - 1) / tr), threads, shm, s>>>(in, out, rows, sign, scale, tr);
+    k_fft2_rows<L><<<dim3((unsigned)((rows + tr - 1) / tr), in2 ? 2 : 1), threads, shm, s>>>(in, out, in2, out2, rows,
+                                                                                             sign, scale, tr);
     return cudaGetLastError();
+}
+// the lattices with register transforms: one launch for one pair of arrays or two
+static bool fft2_reg(const Dims& d) {
+    return d.L == 1 || d.L == 2 || d.L == 3 || d.L == 4 || d.L == 6 || d.L == 8 || d.L == 12 || d.L == 16 || d.L == 24;
+}
+static cudaError_t launch_fft2_reg(cudaStream_t s, const cplx* in, cplx* out, const cplx* in2, cplx* out2, int rows,
+                                   int sign, double scale, const Dims& d) {
+    switch (d.L) {
+        case 1: return launch_fft2_tpl<1>(s, in, out, in2, out2, rows, sign, scale);
+        case 2: return launch_fft2_tpl<2>(s, in, out, in2, out2, rows, sign, scale);
+        case 4: return launch_fft2_tpl<4>(s, in, out, in2, out2, rows, sign, scale);
+        case 8: return launch_fft2_tpl<8>(s, in, out, in2, out2, rows, sign, scale);
+        case 16: return launch_fft2_tpl<16>(s, in, out, in2, out2, rows, sign, scale);
+        case 3: return launch_fft2_tpl<3>(s, in, out, in2, out2, rows, sign, scale);
+        case 6: return launch_fft2_tpl<6>(s, in, out, in2, out2, rows, sign, scale);
+        case 12: return launch_fft2_tpl<12>(s, in, out, in2, out2, rows, sign, scale);
+        default: return launch_fft2_tpl<24>(s, in, out, in2, out2, rows, sign, scale);
+    }
+}
+// two arrays: Hubbard 8x8, nK3 = (8, 12): two launches of 8 us each otherwise
+static cudaError_t launch_fft2_pair(cudaStream_t s, const cplx* in, cplx* out, const cplx* in2, cplx* out2, int rows,
+                                    int sign, double scale, const cplx* tw_sign, const Dims& d) {
+    if (fft2_reg(d)) return launch_fft2_reg(s, in, out, in2, out2, rows, sign, scale, d);
+    const cudaError_t e = launch_fft2(s, in, out, rows, sign, scale, tw_sign, d);
+    return e == cudaSuccess ? launch_fft2(s, in2, out2, rows, sign, scale, tw_sign, d) : e;
 }
 cudaError_t launch_fft2(cudaStream_t s, const cplx* in, cplx* out, int rows, int sign, double scale,
                         const cplx* tw_sign, const Dims& d) {
-    switch (d.L) {
-        case 1: return launch_fft2_tpl<1>(s, in, out, rows, sign, scale);
-        case 2: return launch_fft2_tpl<2>(s, in, out, rows, sign, scale);
-        case 4: return launch_fft2_tpl<4>(s, in, out, rows, sign, scale);
-        case 8: return launch_fft2_tpl<8>(s, in, out, rows, sign, scale);
-        case 16: return launch_fft2_tpl<16>(s, in, out, rows, sign, scale);
-        case 3: return launch_fft2_tpl<3>(s, in, out, rows, sign, scale);
-        case 6: return launch_fft2_tpl<6>(s, in, out, rows, sign, scale);
-        case 12: return launch_fft2_tpl<12>(s, in, out, rows, sign, scale);
-        case 24: return launch_fft2_tpl<24>(s, in, out, rows, sign, scale);
-        default: break;
-    }
+    if (fft2_reg(d)) return launch_fft2_reg(s, in, out, nullptr, nullptr, rows, sign, scale, d);
     const int L = d.L, BS = L * (L + 1) + 1;
     int tr = 16;
     while (tr > 1 && (size_t)(2 * tr * BS + L) * sizeof(cplx) > 48 * 1024) tr >>= 1;
@@ -2061,11 +2080,7 @@ cudaError_t launch_rowsum(cudaStream_t s, const cplx* A0, const cplx* A1, const 
     else k_pisum_R<cplx, cplx, false><<<nb, 128, 0, s>>>(GR, nullptr, T0, SRtmp, d, rm);
     LAUNCH_CHECK();
     // S^w[P][Ω] = Σ_R e^{+2πi P·R/L} SR[w][R][Ω]
-    cudaError_t e = launch_fft2(s, SRtmp, S0, d.NPO, +1, 1.0, twp, d);
-    if (e != cudaSuccess) return e;
-    e = launch_fft2(s, SRtmp + (size_t)NR * d.NPO, S1, d.NPO, +1, 1.0, twp, d);
-    if (e != cudaSuccess) return e;
-    return cudaSuccess;
+    return launch_fft2_pair(s, SRtmp, S0, SRtmp + (size_t)NR * d.NPO, S1, d.NPO, +1, 1.0, twp, d);
 }
 cudaError_t launch_sx(cudaStream_t s, const BubbleP& B, const cplx* SPi, const cplx* SPi0, const FLP& FL,
                       const VertP& F0v, cplx* SX, const Dims& d, const RowMask& rm) {
@@ -2298,8 +2313,7 @@ cudaError_t launch_sde_sigma(cudaStream_t s, const cplx* GR, const cplx* Lpp, co
                              cplx* S, const cplx* twm, const cplx* twp, const Dims& d) {
     const int rows = d.N2O * d.N2n, NR = d.L * d.L;
     const double invN = 1.0 / NR;
-    cudaError_t e = launch_fft2(s, Lpp, LR, rows, -1, invN, twm, d);
-    if (e == cudaSuccess) e = launch_fft2(s, Lph, LR + (size_t)NR * rows, rows, -1, invN, twm, d);
+    cudaError_t e = launch_fft2_pair(s, Lpp, LR, Lph, LR + (size_t)NR * rows, rows, -1, invN, twm, d);
     if (e != cudaSuccess) return e;
     k_sde_sigma_R<false><<<blocks_for((size_t)NR * d.NG * 32, 128), 128, 0, s>>>(GR, LR, LR + (size_t)NR * rows, nullptr,
                                                                                  nullptr, nullptr, SR, d);
@@ -2311,8 +2325,7 @@ cudaError_t launch_sde_sigma_tan(cudaStream_t s, const cplx* GR, const cplx* LR,
                                  const Dims& d) {
     const int rows = d.N2O * d.N2n, NR = d.L * d.L;
     const double invN = 1.0 / NR;
-    cudaError_t e = launch_fft2(s, tLpp, tLR, rows, -1, invN, twm, d);
-    if (e == cudaSuccess) e = launch_fft2(s, tLph, tLR + (size_t)NR * rows, rows, -1, invN, twm, d);
+    cudaError_t e = launch_fft2_pair(s, tLpp, tLR, tLph, tLR + (size_t)NR * rows, rows, -1, invN, twm, d);
     if (e != cudaSuccess) return e;
     k_sde_sigma_R<true><<<blocks_for((size_t)NR * d.NG * 32, 128), 128, 0, s>>>(
         GR, LR, LR + (size_t)NR * rows, tGR, tLR, tLR + (size_t)NR * rows, tSR, d);
@@ -2360,9 +2373,7 @@ cudaError_t launch_rowsum_tan(cudaStream_t s, const cplx* tA0, const cplx* tA1, 
     if (GRf) k_pisum_R<cplxf, cplxf, true><<<nb, 128, 0, s>>>(GRf, tGRf, nullptr, SRtmp, d, rm);
     else k_pisum_R<cplx, cplx, true><<<nb, 128, 0, s>>>(GR, tGR, nullptr, SRtmp, d, rm);
     LAUNCH_CHECK();
-    cudaError_t e = launch_fft2(s, SRtmp, tS0, d.NPO, +1, 1.0, twp, d);
-    if (e != cudaSuccess) return e;
-    return launch_fft2(s, SRtmp + (size_t)NR * d.NPO, tS1, d.NPO, +1, 1.0, twp, d);
+    return launch_fft2_pair(s, SRtmp, tS0, SRtmp + (size_t)NR * d.NPO, tS1, d.NPO, +1, 1.0, twp, d);
 }
 cudaError_t launch_sigma_assemble(cudaStream_t s, const cplx* Sin, const cplx* SU2, const uint32_t* map,
                                   const double* occ, const cplx* C0, const cplx* Sig0, cplx* Sig, double U, int hartree,
