@@ -122,8 +122,8 @@ __global__ void __launch_bounds__(RT) k_aa_residual(const cplx* y, const cplx* x
 // projection run in one pass, every Gram-Schmidt pass also takes the partial of <Q_i, f> (no separate
 // pass of dot products), and γ and the next deletion's rotations come from one single-block kernel.
 // A step beside the map at m = 8 on GB300, on full vectors with separate passes -> now: Hubbard 8x8,
-// nK3 = (8, 12): 1.03 -> 0.22 ms; Hubbard 8x8, nK3 = (20, 40), 49 M elements: 22 -> 1.9 ms; SIAM,
-// nK3 = (16, 16), 0.1 M elements: 0.26 -> 0.19 ms.
+// nK3 = (8, 12): 1.03 -> 0.21 ms; Hubbard 8x8, nK3 = (20, 40), 49 M elements: 22 -> 1.8 ms; SIAM,
+// nK3 = (16, 16), 0.1 M elements: 0.26 -> 0.16 ms.
 
 // Column rotations (nrot > 0: the nrot = m - 1 rotations of a deletion, applied to Q in order), then
 // Δg = g - gold ; Δf = fx - fxold (in place in fxold) ; partial of <Q_0, Δf>, or of |Δf|² when Q has no
