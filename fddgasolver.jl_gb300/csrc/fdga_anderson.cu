@@ -96,7 +96,7 @@ __global__ void __launch_bounds__(RT) k_aa_expand(cplx* x, const cplx* xr, const
         st16(x + j, signed_(ld16(xr + key_of(c)), c & 1u));
     }
 }
-// fx = y - x ; g = x + beta fx ; block maxima of |fx|² (y full, x one value per key)
+// fx = y - x ; g = x + beta fx ; block maxima of |fx|², NaN kept (y full, x one value per key)
 __global__ void __launch_bounds__(RT) k_aa_residual(const cplx* y, const cplx* xr, const uint32_t* code,
                                                     const uint32_t* src, cplx* fx, cplx* g, double beta, double* pmax,
                                                     size_t nr) {
@@ -106,13 +106,13 @@ __global__ void __launch_bounds__(RT) k_aa_residual(const cplx* y, const cplx* x
         const cplx x = xr[k], f = key_value(y, code, src, k) - x;
         fx[k] = f;
         g[k] = x + f * beta;
-        mx = fmax(mx, f.x * f.x + f.y * f.y);
+        mx = max_mag(mx, f.x * f.x + f.y * f.y);
     }
-    for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    for (int o = 16; o > 0; o >>= 1) mx = max_mag(mx, __shfl_xor_sync(0xffffffffu, mx, o));
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = mx;
     __syncthreads();
     if (threadIdx.x) return;
-    for (int w = 1; w < RT / 32; ++w) mx = fmax(mx, red[w]);
+    for (int w = 1; w < RT / 32; ++w) mx = max_mag(mx, red[w]);
     pmax[blockIdx.x] = mx;
 }
 

@@ -56,7 +56,7 @@ struct Acc {
     __device__ __forceinline__ cplx total() const { return s64 + to_d(s32); }
 };
 
-// f = y (+ c) - x in FP64 ; f32 = f ; g = x + βf ; partial max|f|²
+// f = y (+ c) - x in FP64 ; f32 = f ; g = x + βf ; partial max|f|² (NaN kept)
 __global__ void __launch_bounds__(RT) k_ma_residual(const cplx* y, const cplx* c, const cplx* x, cplxf* f32, cplx* g,
                                                     double beta, double* pmax, size_t n) {
     __shared__ double red[RT];
@@ -66,12 +66,12 @@ __global__ void __launch_bounds__(RT) k_ma_residual(const cplx* y, const cplx* c
         if (c) f += c[i];
         f32[i] = tof(f);
         g[i] = x[i] + f * beta;
-        mx = fmax(mx, f.x * f.x + f.y * f.y);
+        mx = max_mag(mx, f.x * f.x + f.y * f.y);
     }
     red[threadIdx.x] = mx;
     __syncthreads();
     for (int o = RT / 2; o > 0; o >>= 1) {
-        if ((int)threadIdx.x < o) red[threadIdx.x] = fmax(red[threadIdx.x], red[threadIdx.x + o]);
+        if ((int)threadIdx.x < o) red[threadIdx.x] = max_mag(red[threadIdx.x], red[threadIdx.x + o]);
         __syncthreads();
     }
     if (threadIdx.x == 0) pmax[blockIdx.x] = red[0];

@@ -616,6 +616,13 @@ __device__ __forceinline__ S fl_right(const S* FLK2p, const S* FLK2t, const S* F
     return ldv(FLK2t + i) * (R)2 - ldv(FLK2a + i);  // dSp = 2 pSp + xSp, xSp(t) = -pSp(a)
 }
 
+// The larger of two magnitudes (values ≥ 0, infinity, NaN) that keeps a NaN, which fmax drops: with the sign bit
+// off, the bits order like the values and a NaN lies above infinity.  (Integer pipe; FP64 compares run at 1/64 rate.)
+__device__ __forceinline__ double max_mag(double a, double b) {
+    const long long m = 0x7fffffffffffffffll;
+    return __longlong_as_double(max(__double_as_longlong(a) & m, __double_as_longlong(b) & m));
+}
+
 __device__ __forceinline__ int cross(int ch, int m, int n) { return ch == CH_P ? m - n - 1 : n; }
 
 // half width of the ω range that any window of the K2 BSE can reach, clipped to the stored bubble window

@@ -1808,12 +1808,12 @@ __global__ void k_residual(const cplx* y, const cplx* x, cplx* fx, cplx* g, doub
         const cplx f = x ? y[i] - x[i] : y[i];
         if (fx) fx[i] = f;
         if (g && x) g[i] = x[i] + f * beta;
-        mx = fmax(mx, f.x * f.x + f.y * f.y);
+        mx = max_mag(mx, f.x * f.x + f.y * f.y);
     }
     red[threadIdx.x] = mx;
     __syncthreads();
     for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-        if ((int)threadIdx.x < o) red[threadIdx.x] = fmax(red[threadIdx.x], red[threadIdx.x + o]);
+        if ((int)threadIdx.x < o) red[threadIdx.x] = max_mag(red[threadIdx.x], red[threadIdx.x + o]);
         __syncthreads();
     }
     if (threadIdx.x == 0) pmax[blockIdx.x] = red[0];

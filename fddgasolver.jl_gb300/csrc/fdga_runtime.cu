@@ -1684,8 +1684,9 @@ double reduce_max(fdga_handle* h, int nblk, int& status) {
         e = cudaMemcpyAsync(h->part_host, h->d_part, nblk * sizeof(double), cudaMemcpyDeviceToHost, h->st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(h->st);
     if (e != cudaSuccess) { status = cuda_fail(h, e, "reduce_max"); return 0.0; }
-    double m = 0.0;  // the partials are squared magnitudes
-    for (int i = 0; i < nblk; ++i) m = std::max(m, h->part_host[i]);
+    double m = 0.0;  // the partials are squared magnitudes; a NaN stays
+    for (int i = 0; i < nblk; ++i)
+        if (!(h->part_host[i] <= m) && !std::isnan(m)) m = h->part_host[i];
     status = FDGA_OK;
     return std::sqrt(m);
 }
