@@ -794,17 +794,18 @@ __global__ void __launch_bounds__((TILE / 2) * (TILE / 2)) k_adj_gemm(GemmBatch 
         }
 }
 template <int OPA, int OPB, int TILE>
-void launch_adj_gemm_tile(cudaStream_t s, const GemmBatch& g, const Dims& d) {
+cudaError_t launch_adj_gemm_tile(cudaStream_t s, const GemmBatch& g, const Dims& d) {
     const int nt = (d.N3n + TILE - 1) / TILE;
     const dim3 grid((unsigned)(g.nblocks * nt * nt), 1, 3);
     k_adj_gemm<OPA, OPB, TILE><<<grid, (TILE / 2) * (TILE / 2), 0, s>>>(g, d);
+    return cudaGetLastError();
 }
 template <int OPA, int OPB>
-void launch_adj_gemm(cudaStream_t s, const GemmBatch& g, const Dims& d) {
-    if (g.digits) launch_adj_mma(s, OPA, g, d);
-    else if (d.N3n <= 16) launch_adj_gemm_tile<OPA, OPB, 16>(s, g, d);
-    else if (d.N3n <= 24) launch_adj_gemm_tile<OPA, OPB, 24>(s, g, d);
-    else launch_adj_gemm_tile<OPA, OPB, 32>(s, g, d);
+cudaError_t launch_adj_gemm(cudaStream_t s, const GemmBatch& g, const Dims& d) {
+    if (g.digits) return launch_adj_mma(s, OPA, g, d);
+    if (d.N3n <= 16) return launch_adj_gemm_tile<OPA, OPB, 16>(s, g, d);
+    if (d.N3n <= 24) return launch_adj_gemm_tile<OPA, OPB, 24>(s, g, d);
+    return launch_adj_gemm_tile<OPA, OPB, 32>(s, g, d);
 }
 // mode 1: M̄ -> Π̄ (row sums), Γ̄s, γ̄L (box) and the epilogue γ̄L(ν,ν') += ō; warp per (slot, block, ω)
 __global__ void k_adj_distribute_M(K3Args3 args, Ptr3 Mbar, Ptr3 Obar, Ptr3 Gbar, cplx* Pbpp, cplx* Pbph, cplx* FLb0,
@@ -1073,9 +1074,8 @@ cudaError_t launch_adj_K3(cudaStream_t s, int mode, const K3Args3& a, const cplx
     }
     g.accumulate = 1;
     g.digits = digits;
-    launch_adj_gemm<0, 1>(s, g, d);  // Ā += α ō Mᴴ
-    LCHK();
-    if (mode == 0) return cudaSuccess;
+    cudaError_t e = launch_adj_gemm<0, 1>(s, g, d);  // Ā += α ō Mᴴ
+    if (e != cudaSuccess || mode == 0) return e;
     GemmBatch h{};
     h.blocks = a.blocks;
     h.nblocks = a.nblocks;
@@ -1087,8 +1087,8 @@ cudaError_t launch_adj_K3(cudaStream_t s, int mode, const K3Args3& a, const cplx
     }
     h.accumulate = 0;
     h.digits = digits;
-    launch_adj_gemm<1, 0>(s, h, d);  // M̄ = T Aᴴ ō
-    LCHK();
+    e = launch_adj_gemm<1, 0>(s, h, d);  // M̄ = T Aᴴ ō
+    if (e != cudaSuccess) return e;
     const Ptr3 mb{{Mbar[0], Mbar[1], Mbar[2]}};
     const Ptr3 ob{{const_cast<cplx*>(Obar[0]), const_cast<cplx*>(Obar[1]), const_cast<cplx*>(Obar[2])}};
     const Ptr3 gb{{Gbar[0], Gbar[1], Gbar[2]}};
