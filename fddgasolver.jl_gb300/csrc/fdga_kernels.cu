@@ -2148,11 +2148,13 @@ template <class S, bool TAN>
 static size_t k2_row_smem(const Dims& d) {
     return (size_t)(TAN ? 2 : 1) * 2 * k2_table_half(d) * sizeof(S);
 }
-template <class K>
-static cudaError_t k2_smem_attr(K kernel, size_t smem) {
+// Limit of a row kernel.  The kernel is the template argument, so that each instantiation has a record of its own
+// (forms of one kernel share a function type).
+template <auto Kernel>
+static cudaError_t row_smem_limit(size_t smem) {
     if (smem > 227 * 1024) return cudaErrorInvalidValue;
-    static SmemRecord raised;  // one record per kernel instantiation
-    return raise_smem_limit(kernel, raised, smem);
+    static SmemRecord raised;
+    return raise_smem_limit(Kernel, raised, smem);
 }
 static unsigned warp_grid(const ChanWork& cw, int nch) {
     int mx = 0;
@@ -2168,15 +2170,17 @@ static cudaError_t sde_L_rows(cudaStream_t s, const VertPT<S>& F, const BubbleP&
     const unsigned rows = row_grid(cw, 2);
     const int threads = rows * 2 < 4 * 152 ? 256 : 128, hb = std::max(d.n2n, d.nRn);
     const size_t smem = ((size_t)(TAN ? 4 : 2) * hb + threads / 32 * SDE_LANES + 1) * sizeof(S);
-    cudaError_t e = k2_smem_attr(k_sde_L_rows<S, TAN>, smem);
+    cudaError_t e = row_smem_limit<k_sde_L_rows<S, TAN>>(smem);
     if (e != cudaSuccess) return e;
     k_sde_L_rows<S, TAN><<<dim3(rows, 2), threads, smem, s>>>(F, B, SPpp, SPph, cw, use_vertex, ref_scale, d, T);
     LAUNCH_CHECK(); return cudaSuccess;
 }
 // each vertex-evaluating kernel is launched in its V0 = F.has0 instantiation (see vert_spec)
-template <class K>
-static cudaError_t k2_launch_attr(K k_plain, K k_v0, K k_tab, bool v0, bool tab, size_t smem) {
-    return k2_smem_attr(tab ? k_tab : (v0 ? k_v0 : k_plain), smem);
+template <class S, bool TAN>
+static cudaError_t k2_smem_limit(bool v0, bool tab, size_t smem) {
+    if (tab) return row_smem_limit<k_bse_K2_all<S, TAN, false, true>>(smem);
+    if (v0) return row_smem_limit<k_bse_K2_all<S, TAN, true, false>>(smem);
+    return row_smem_limit<k_bse_K2_all<S, TAN, false, false>>(smem);
 }
 #define FDGA_VERTEX_LAUNCHERS(VT, FT, TT, ST)                                                                       \
     cudaError_t launch_bse_K1_all(cudaStream_t s, const VT& F, const FT& FL, const BubbleP& B, const cplx* SX,    \
@@ -2196,8 +2200,7 @@ static cudaError_t k2_launch_attr(K k_plain, K k_v0, K k_tab, bool v0, bool tab,
     cudaError_t launch_bse_K2_all(cudaStream_t s, const VT& F, const FT& FL, const BubbleP& B, const cplx* SX,    \
                                   const ChanWork& cw, const Dims& d) {                                             \
         const size_t smem = k2_row_smem<ST, false>(d);                                                             \
-        cudaError_t e = k2_launch_attr(k_bse_K2_all<ST, false, false, false>, k_bse_K2_all<ST, false, true, false>,     \
-                                       k_bse_K2_all<ST, false, false, true>, F.has0, F.tab[0] != nullptr, smem); \
+        cudaError_t e = k2_smem_limit<ST, false>(F.has0, F.tab[0] != nullptr, smem);                                   \
         if (e != cudaSuccess) return e;                                                                             \
         const dim3 g = k2_grid(cw, d);                                                                              \
         if (F.tab[0]) k_bse_K2_all<ST, false, false, true><<<g, row_threads(cw, 3), smem, s>>>(F, FL, B, SX, cw, d, TT{}); \
@@ -2222,8 +2225,7 @@ static cudaError_t k2_launch_attr(K k_plain, K k_v0, K k_tab, bool v0, bool tab,
     cudaError_t launch_bse_K2_tan(cudaStream_t s, const VT& F, const FT& FL, const BubbleP& B, const cplx* SX,    \
                                   const TT& T, const ChanWork& cw, const Dims& d) {                                \
         const size_t smem = k2_row_smem<ST, true>(d);                                                              \
-        cudaError_t e = k2_launch_attr(k_bse_K2_all<ST, true, false, false>, k_bse_K2_all<ST, true, true, false>,     \
-                                       k_bse_K2_all<ST, true, false, true>, F.has0, F.tab[0] != nullptr, smem);  \
+        cudaError_t e = k2_smem_limit<ST, true>(F.has0, F.tab[0] != nullptr, smem);                                   \
         if (e != cudaSuccess) return e;                                                                             \
         const dim3 g = k2_grid(cw, d);                                                                              \
         if (F.tab[0]) k_bse_K2_all<ST, true, false, true><<<g, row_threads(cw, 3), smem, s>>>(F, FL, B, SX, cw, d, T); \
