@@ -439,8 +439,8 @@ __device__ void adj_K2_body(const VertP& F, const FLP& FL, const cplx* Pi, const
     }
 }
 // The same with the Γ table (nonlocal solver with a RefVertex): one CTA per (P, Ω) row of representatives,
-// one ω per thread.  The cotangents of Π(ω) and FL(ω) are summed over the row's ν in registers and added
-// once; the cotangent of Γ(Ω, ν, ω) goes to one table element, shared by every P, instead of the up to
+// one ω per thread, the row's items in passes of `cap`.  The cotangents of Π(ω) and FL(ω) are summed over a
+// pass's ν in registers and added once; the cotangent of Γ(Ω, ν, ω) goes to one table element, shared by every P, instead of the up to
 // eight elements of the two other channels (k_adj_gamma_table carries the sum there).  The atomics bound
 // the evaluation in place.  Hubbard 8x8, nK3 = (8, 12) on GB300, in place -> with the table: K2 653 -> 56 us;
 // left K2 338 us and caches 311 us -> 25 (caches) + 32 us (k_adj_gamma_table) + the left K2's one atomic per
@@ -449,74 +449,77 @@ template <int CH>
 __device__ void adj_K2_row(const VertP& F, const FLP& FL, const cplx* Pi, const cplx* Pi0, const cplx* SX,
                            const VertBar& Fb, const FLBar& FLb, cplx* tabbar, cplx* Pibar, cplx* SXbar,
                            const cplx* rawbar, const int* items, const int* gstart, int ngroups, const Dims& d,
-                           cplx* ss, int* sn) {
+                           cplx* ss, int* sn, int cap) {
     const int g = blockIdx.x;
     if (g >= ngroups) return;
     const int i0 = gstart ? gstart[g] : g * d.N2n, i1 = gstart ? gstart[g + 1] : (g + 1) * d.N2n;
     const int first = items ? items[i0] : i0;
     const int m = (first / d.N2n) % d.N2O - (d.n2O - 1), P = first / (d.N2n * d.N2O);
     const size_t is = (size_t)CH * d.Nq * d.NPO + (size_t)P * d.NPO + (m + d.nPO - 1);
-    const int cnt = i1 - i0;
-    for (int j = threadIdx.x; j < cnt; j += blockDim.x) {
-        const int idx = items ? items[i0 + j] : i0 + j;
-        const int nu = idx % d.N2n - d.n2n;
-        const cplx s = rawbar[idx] * (d.T * (CH == CH_T ? -1.0 : 1.0));
-        ss[j] = s;
-        sn[j] = nu;
-        const cplx c = k2_c<CH>(F, d, m, nu, P);
-        aadd(SXbar + is, cmulc(c, s));
-        const cplx cb = cmulc(SX[is], s);
-        if (CH != CH_T) {
-            k2a(Fb.g[CH], d, m, nu, P, cb);
-        } else {
-            k2a(Fb.g[CH_T], d, m, nu, P, cb * 2.0);
-            k2a(Fb.g[CH_A], d, m, nu, P, cb * -1.0);
-        }
-    }
-    __syncthreads();
     const int half = k2_table_half(d), th = gamma_half(d);
-    for (int n = -half + (int)threadIdx.x; n < half; n += blockDim.x) {
-        const int wt = cross(CH, m, n);
-        const cplx FLr = fl_right(FL.K2[CH_P], FL.K2[CH_T], FL.K2[CH_A], d, CH, m, wt, P);
-        const size_t ip = ixPi(d, P, m, n);
-        const cplx pi = ldg(Pi + ip), pi0 = ldg(Pi0 + ip);
-        const cplx X = cfma(pi, FLr, (pi - pi0) * d.U);
-        cplx Xb = mk(0, 0);
-        const bool int_ = fin(n, th), n3 = bin(m, d.n3O) && fin(n, d.n3n), inr = fin(n, d.nRn);
-        for (int j = 0; j < cnt; ++j) {
-            const int nu = sn[j];
-            int n0, n1;
-            k2_hull<CH>(d, m, nu, n0, n1);
-            if (n < n0 || n > n1) continue;
-            const cplx s = ss[j];
-            const bool in3 = n3 && fin(nu, d.n3n);
-            cplx D = int_ ? ldg(gamma_row(F.tab[CH], d, m, nu) + n) : mk(0, 0);
-            if (in3 || inr) D += k2_own_diff<CH>(F, d, m, nu, n, P, in3);
-            Xb = cfmac(D, s, Xb);
-            const cplx Db = cmulc(X, s);
-            if (int_) aadd(const_cast<cplx*>(gamma_row<cplx>(tabbar, d, m, nu)) + n, Db);
-            if (in3) {
-                if (CH != CH_T) {
-                    k3a(Fb.g[CH], d, m, nu, n, P, Db);
-                } else {
-                    k3a(Fb.g[CH_T], d, m, nu, n, P, Db * 2.0);
-                    k3a(Fb.g[CH_A], d, m, nu, n, P, Db * -1.0);
-                }
+    for (int c0 = i0; c0 < i1; c0 += cap) {  // (one pass up to cap items)
+        const int cnt = min(cap, i1 - c0);
+        if (c0 > i0) __syncthreads();
+        for (int j = threadIdx.x; j < cnt; j += blockDim.x) {
+            const int idx = items ? items[c0 + j] : c0 + j;
+            const int nu = idx % d.N2n - d.n2n;
+            const cplx s = rawbar[idx] * (d.T * (CH == CH_T ? -1.0 : 1.0));
+            ss[j] = s;
+            sn[j] = nu;
+            const cplx c = k2_c<CH>(F, d, m, nu, P);
+            aadd(SXbar + is, cmulc(c, s));
+            const cplx cb = cmulc(SX[is], s);
+            if (CH != CH_T) {
+                k2a(Fb.g[CH], d, m, nu, P, cb);
+            } else {
+                k2a(Fb.g[CH_T], d, m, nu, P, cb * 2.0);
+                k2a(Fb.g[CH_A], d, m, nu, P, cb * -1.0);
             }
         }
-        aadd(Pibar + ip, cmulc(FLr + mk(d.U, 0), Xb));
-        fl_right_adj(FLb, d, CH, m, wt, P, cmulc(pi, Xb));
+        __syncthreads();
+        for (int n = -half + (int)threadIdx.x; n < half; n += blockDim.x) {
+            const int wt = cross(CH, m, n);
+            const cplx FLr = fl_right(FL.K2[CH_P], FL.K2[CH_T], FL.K2[CH_A], d, CH, m, wt, P);
+            const size_t ip = ixPi(d, P, m, n);
+            const cplx pi = ldg(Pi + ip), pi0 = ldg(Pi0 + ip);
+            const cplx X = cfma(pi, FLr, (pi - pi0) * d.U);
+            cplx Xb = mk(0, 0);
+            const bool int_ = fin(n, th), n3 = bin(m, d.n3O) && fin(n, d.n3n), inr = fin(n, d.nRn);
+            for (int j = 0; j < cnt; ++j) {
+                const int nu = sn[j];
+                int n0, n1;
+                k2_hull<CH>(d, m, nu, n0, n1);
+                if (n < n0 || n > n1) continue;
+                const cplx s = ss[j];
+                const bool in3 = n3 && fin(nu, d.n3n);
+                cplx D = int_ ? ldg(gamma_row(F.tab[CH], d, m, nu) + n) : mk(0, 0);
+                if (in3 || inr) D += k2_own_diff<CH>(F, d, m, nu, n, P, in3);
+                Xb = cfmac(D, s, Xb);
+                const cplx Db = cmulc(X, s);
+                if (int_) aadd(const_cast<cplx*>(gamma_row<cplx>(tabbar, d, m, nu)) + n, Db);
+                if (in3) {
+                    if (CH != CH_T) {
+                        k3a(Fb.g[CH], d, m, nu, n, P, Db);
+                    } else {
+                        k3a(Fb.g[CH_T], d, m, nu, n, P, Db * 2.0);
+                        k3a(Fb.g[CH_A], d, m, nu, n, P, Db * -1.0);
+                    }
+                }
+            }
+            aadd(Pibar + ip, cmulc(FLr + mk(d.U, 0), Xb));
+            fl_right_adj(FLb, d, CH, m, wt, P, cmulc(pi, Xb));
+        }
     }
 }
 __global__ void k_adj_K2_rows(VertP F, FLP FL, BubbleP B, const cplx* SX, VertBar Fb, FLBar FLb, Ptr3 tb, cplx* Pbpp,
-                              cplx* Pbph, cplx* SXbar, const cplx* rawbar, ChanWork cw, size_t n2, Dims d) {
+                              cplx* Pbph, cplx* SXbar, const cplx* rawbar, ChanWork cw, size_t n2, Dims d, int cap) {
     extern __shared__ __align__(16) unsigned char sh_rows[];
     cplx* ss = reinterpret_cast<cplx*>(sh_rows);
-    int* sn = reinterpret_cast<int*>(ss + d.N2n);
+    int* sn = reinterpret_cast<int*>(ss + cap);
     switch (blockIdx.y) {
-        case CH_P: adj_K2_row<CH_P>(F, FL, B.pp, B.pp0, SX, Fb, FLb, tb.p[CH_P], Pbpp, SXbar, rawbar, cw.items[CH_P], cw.gstart[CH_P], cw.ngroups[CH_P], d, ss, sn); break;
-        case CH_T: adj_K2_row<CH_T>(F, FL, B.ph, B.ph0, SX, Fb, FLb, tb.p[CH_T], Pbph, SXbar, rawbar + n2, cw.items[CH_T], cw.gstart[CH_T], cw.ngroups[CH_T], d, ss, sn); break;
-        default:   adj_K2_row<CH_A>(F, FL, B.ph, B.ph0, SX, Fb, FLb, tb.p[CH_A], Pbph, SXbar, rawbar + 2 * n2, cw.items[CH_A], cw.gstart[CH_A], cw.ngroups[CH_A], d, ss, sn); break;
+        case CH_P: adj_K2_row<CH_P>(F, FL, B.pp, B.pp0, SX, Fb, FLb, tb.p[CH_P], Pbpp, SXbar, rawbar, cw.items[CH_P], cw.gstart[CH_P], cw.ngroups[CH_P], d, ss, sn, cap); break;
+        case CH_T: adj_K2_row<CH_T>(F, FL, B.ph, B.ph0, SX, Fb, FLb, tb.p[CH_T], Pbph, SXbar, rawbar + n2, cw.items[CH_T], cw.gstart[CH_T], cw.ngroups[CH_T], d, ss, sn, cap); break;
+        default:   adj_K2_row<CH_A>(F, FL, B.ph, B.ph0, SX, Fb, FLb, tb.p[CH_A], Pbph, SXbar, rawbar + 2 * n2, cw.items[CH_A], cw.gstart[CH_A], cw.ngroups[CH_A], d, ss, sn, cap); break;
     }
 }
 __global__ void k_adj_K1(VertP F, FLP FL, BubbleP B, const cplx* SX, VertBar Fb, FLBar FLb, cplx* Pbpp, cplx* Pbph,
@@ -1019,8 +1022,9 @@ cudaError_t launch_adj_K2_tab(cudaStream_t s, const VertP& F, const FLP& FL, con
                               const cplx* rawbar, const ChanWork& cw, size_t n2, const Dims& d) {
     const int rows = std::max(1, std::max(cw.ngroups[0], std::max(cw.ngroups[1], cw.ngroups[2])));
     const int threads = std::min(256, (2 * k2_table_half(d) + 31) / 32 * 32);
-    const size_t shm = (size_t)d.N2n * (sizeof(cplx) + sizeof(int));  // N2n < 2400 by the size limits of a state
-    k_adj_K2_rows<<<dim3(rows, 3), threads, shm, s>>>(F, FL, B, SX, Fb, FLb, tb, Pbpp, Pbph, SXbar, rawbar, cw, n2, d);
+    const int cap = std::min(d.N2n, 2048);  // items of a row at once: 40 KB, within every launch's limit
+    const size_t shm = (size_t)cap * (sizeof(cplx) + sizeof(int));
+    k_adj_K2_rows<<<dim3(rows, 3), threads, shm, s>>>(F, FL, B, SX, Fb, FLb, tb, Pbpp, Pbph, SXbar, rawbar, cw, n2, d, cap);
     LCHK(); return cudaSuccess;
 }
 cudaError_t launch_adj_L_K2_tab(cudaStream_t s, const BubbleP& B, const Ptr3& tb, const cplx* rawbar,

@@ -1,6 +1,7 @@
 """Frequency boxes so wide that a row's tables pass the default shared-memory limit (48 KB) of a launch.
 
-Tolerance against the oracle: the plain path's 1e-10 per flatten block (FP64 sums in another order)."""
+Tolerance against the oracle: the plain path's 1e-10 per flatten block (FP64 sums in another order); rrule against
+frule: 1e-12 of |ȳ| |J v|, as for small boxes."""
 import numpy as np
 import pytest
 
@@ -25,6 +26,18 @@ def _matches_oracle(cfg, sym=True):
     err = blockwise_rel_err(cfg, S.fixed_point(x) + x, y)
     S.close()
     assert err < 1e-10
+
+
+def _transposed(cfg, sym=True):
+    S = make_gpu(cfg, sym)
+    x = S.fixed_point(_start(S, 2))
+    v, yb = _start(S, 3), _start(S, 4)
+    S.unflatten(x)
+    jv = S.frule(v)[1]
+    S.unflatten(x)
+    xb = S.rrule(yb)[1]
+    S.close()
+    assert abs(np.vdot(yb, jv).real - np.vdot(xb, v).real) < 1e-12 * np.linalg.norm(yb) * np.linalg.norm(jv)
 
 
 def test_each_form_of_k2_raises_its_own_limit():
@@ -55,3 +68,8 @@ def test_a_tangent_leaves_the_map_its_limit():
     S.frule(_start(S, 7))
     S.close()
     _matches_oracle(dict(SIAM, nK1=1700, nK2=(1, 1700)))
+
+
+def test_adjoint_of_wide_fermionic_rows():
+    """K2 rows of up to 2 nK2ν = 2560 items: past the 2458 whose values fit 48 KB (nonlocal, trivial groups)."""
+    _transposed(dict(HUB, nK1=1280, nK2=(1, 1280)), sym=False)
