@@ -566,6 +566,17 @@ VertPT<S> vertex_view_t(const fdga_handle* h, S* st, S* avg, S* const* fref) {
     return F;
 }
 VertP vertex_view(fdga_handle* h, cplx* S) { return vertex_view_t<cplx>(h, S, h->avg, h->Fref); }
+// Whether the handle keeps Γ tables (one of the map, one each of its tangent and its adjoint).  Nonlocal solvers
+// with a RefVertex share a table between the momenta; a Vertex-valued F0 has terms that depend on P.  A table
+// grows with the cube of the K2 box whatever the lattice, the state with its square: nK1 = 320,
+// nK2 = (160, 160) on 4 x 4 takes 6.3 GB for 78 MB of K2 arrays.  So it is kept up to 4 GiB (three are 5 % of the
+// device memory) or the state's own size, and larger boxes evaluate the vertex in place.  The line is memory, not
+// time: evaluating / tabulating, left K2 + K2 + caches at nK2 = (100, 100) (1.15 GB) take 2.1 / 1.4 ms on 2 x 2 and
+// 9.7 / 4.3 ms on 8 x 8 with groups.
+bool gamma_table_kept(const fdga_handle* h) {
+    if (h->d.Nq == 1 || h->has0) return false;
+    return gamma_table_len(h->d) * sizeof(cplx) <= std::max((size_t)4 << 30, h->nstate * sizeof(cplx));
+}
 // attaches a Γ table to a vertex view
 template <class S>
 void set_table(const fdga_handle* h, VertPT<S>& F, S* tab) {
@@ -1889,7 +1900,7 @@ int fdga_create(const fdga_config* c, fdga_handle** out) {
     ALC(h->LR, 2 * h->n2); ALC(h->SigR, h->nGk);
     ALC(h->raw1, 3 * h->n1); ALC(h->raw2, 3 * h->n2); ALC(h->raw3, 3 * h->n3);
     h->nk3blocks = d.Nq * d.N3O;
-    if (d.Nq > 1 && !h->has0) ALC(h->gtab, gamma_table_len(d));
+    if (gamma_table_kept(h)) ALC(h->gtab, gamma_table_len(d));
     h->ngoms = d.N2O;
     ALC(h->occ, 1);
     ALC(h->d_part, NBLK_RED);

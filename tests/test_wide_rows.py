@@ -1,4 +1,5 @@
-"""Frequency boxes so wide that a row's tables pass the default shared-memory limit (48 KB) of a launch.
+"""Frequency boxes so wide that a row's tables pass the default shared-memory limit (48 KB) of a launch, and K2
+boxes so large that a table of the irreducible vertex would dwarf the state.
 
 Tolerance against the oracle: the plain path's 1e-10 per flatten block (FP64 sums in another order); rrule against
 frule: 1e-12 of |ȳ| |J v|, as for small boxes."""
@@ -73,3 +74,22 @@ def test_a_tangent_leaves_the_map_its_limit():
 def test_adjoint_of_wide_fermionic_rows():
     """K2 rows of up to 2 nK2ν = 2560 items: past the 2458 whose values fit 48 KB (nonlocal, trivial groups)."""
     _transposed(dict(HUB, nK1=1280, nK2=(1, 1280)), sym=False)
+
+
+def test_large_k2_box_fits():
+    """nK2 = (170, 170) on 2 x 2: the K2 arrays take 22 MB, a table of the irreducible vertex 5.7 GB."""
+    import torch
+    cfg = dict(HUB, nK1=170, nK2=(170, 170), nK3=(2, 2), mPi_factor=2)
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    S = make_gpu(cfg, True)
+    x = S.fixed_point(_start(S, 8))
+    S.unflatten(x)
+    S.rrule(x)
+    S.unflatten(x)
+    S.frule(x)
+    used = free - torch.cuda.mem_get_info()[0]
+    S.close()
+    assert used < 2 << 30
+    _matches_oracle(cfg)
+    _transposed(cfg)
