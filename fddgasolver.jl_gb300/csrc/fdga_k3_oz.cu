@@ -43,6 +43,7 @@
 
 #include "fdga_digits.cuh"
 #include "fdga_kernels.h"
+#include "fdga_ring.h"
 
 namespace fdga {
 
@@ -158,6 +159,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 2)
     __shared__ uint64_t bfull_[NS];  // per stage: the workers have written the chunk's B digit operands
     __shared__ uint32_t tmem_base;
     __shared__ int abort_;
+    __shared__ int committed_;  // chunks whose MMAs were committed
     // the ω factors of M with their signs: [0] Π0 (mode 0), s1 (Π - Π0) (mode 1) or s1 dΠ (mode 3),
     // [1] s1 Π
     __shared__ cplx qf[128][2];
@@ -187,7 +189,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 2)
     const uint32_t arow = (uint32_t)N * 32u, stage = stage_bytes(N);
     // A: row ν, k = 2ω_l holds Re A, 2ω_l + 1 holds Im A; the S operands of a chunk arrive by one copy
     auto copy_A = [&](int c) {
-        const int st = c % NS;
+        const int st = ring_stage(c, NS);
         mbar_expect_tx(afull(st), (uint32_t)S * arow);
         bulk_g2s(smem_u32(sm + (size_t)st * stage), adig + ((size_t)(rest - r0) * nchunks + c) * S * arow,
                  (uint32_t)S * arow, afull(st));
@@ -281,10 +283,10 @@ __global__ void __launch_bounds__(OZ_THREADS, 2)
             // field, bits 0-13, takes the byte offsets of the other operands >> 4 without carry: all of the
             // shared memory lies below 2^18 bytes)
             const uint64_t dA0 = sdesc16(smem_u32(sm)), dB0 = sdesc16(smem_u32(sm) + S * arow);
-            int copied = min(nchunks, NS);
+            int copied = min(nchunks, NS), committed = 0;
             for (int c = 0; c < nchunks && ok; ++c) {
-                const int st = c % NS;
-                const uint32_t par = (c / NS) & 1;
+                const int st = ring_stage(c, NS);
+                const uint32_t par = ring_parity(c, NS);
                 ok = mbar_wait(afull(st), par, &abort_) && mbar_wait(bfull(st), par, &abort_);
                 if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -297,8 +299,9 @@ __global__ void __launch_bounds__(OZ_THREADS, 2)
                                 dB0 + so + (uint64_t)((t * B_DIG) >> 4), idesc, (c > 0 || s > 0) ? 1u : 0u);
                 asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(done(st))
                              : "memory");
+                committed = c + 1;
                 if (c >= 1 && c - 1 + NS < nchunks) {  // the stage of chunk c - 1 is free once that is done
-                    ok = mbar_wait(done((c - 1) % NS), ((c - 1) / NS) & 1, &abort_);
+                    ok = mbar_wait(done(ring_stage(c - 1, NS)), ring_parity(c - 1, NS), &abort_);
                     if (ok) {
                         copy_A(c - 1 + NS);
                         ++copied;
@@ -310,8 +313,10 @@ __global__ void __launch_bounds__(OZ_THREADS, 2)
                 // the MMAs in flight end before the tensor memory is released (below)
                 abort_ = 1;
                 atomicExch(err, 1);
-                for (int c = max(0, copied - NS); c < copied; ++c) mbar_wait(afull(c % NS), (c / NS) & 1, nullptr);
+                for (int c = max(0, copied - NS); c < copied; ++c)
+                    mbar_wait(afull(ring_stage(c, NS)), ring_parity(c, NS), nullptr);
             }
+            committed_ = committed;
         }
         __syncwarp();
     } else {
@@ -322,8 +327,8 @@ __global__ void __launch_bounds__(OZ_THREADS, 2)
 #pragma unroll
         for (int c = 0; c < MAXC; ++c) {
             if (c < nchunks && ok) {
-                const int st = c % NS;
-                if (c >= NS) ok = mbar_wait(done(st), ((c - NS) / NS) & 1, &abort_);
+                const int st = ring_stage(c, NS);
+                if (c >= NS) ok = mbar_wait(done(st), ring_parity(c - NS, NS), &abort_);
                 if (ok) {
                     if (have) {
                         const unsigned long long yr = (unsigned long long)fixed_digits<S>(mv[c].x, F) + DIGIT_BIAS;
@@ -342,10 +347,10 @@ __global__ void __launch_bounds__(OZ_THREADS, 2)
             }
         }
         // (commits complete in order: the last one is the end of all)
-        if (ok) ok = mbar_wait(done((nchunks - 1) % NS), ((nchunks - 1) / NS) & 1, &abort_);
-        if (!ok) {
+        if (ok) ok = mbar_wait(done(ring_stage(nchunks - 1, NS)), ring_parity(nchunks - 1, NS), &abort_);
+        if (!ok) {  // (any lane's: the control thread may have ended its part)
             abort_ = 1;
-            if (tid == 0) atomicExch(err, 1);
+            atomicExch(err, 1);
         }
     }
     ok = __all_sync(0xffffffffu, ok);  // (a wait may give up in some lanes only)
@@ -392,9 +397,10 @@ __global__ void __launch_bounds__(OZ_THREADS, 2)
     }
     __syncthreads();
     if (!worker) {
-        if (abort_) {  // the MMAs of the last chunks committed may still run: bounded waits before the release
-            for (int i = 0; i < NS; ++i) mbar_wait(done(i), 0, nullptr);
-        }
+        // after an abort the MMAs of the last chunks committed may still run: a bounded wait before the release for
+        // the last one (commits complete in order, and its stage's earlier uses were waited for before it)
+        if (abort_ && committed_ > 0)
+            mbar_wait(done(ring_stage(committed_ - 1, NS)), ring_parity(committed_ - 1, NS), nullptr);
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(*(volatile uint32_t*)&tmem_base), "n"(TCOLS));
         return;

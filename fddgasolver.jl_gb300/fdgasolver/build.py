@@ -14,7 +14,7 @@ CSRC = os.path.join(os.path.dirname(PKG), "csrc")
 OUT_DIR = os.path.join(PKG, "_lib")
 LIB = os.path.join(OUT_DIR, "libfdga.so")
 SOURCES = ["fdga_kernels.cu", "fdga_runtime.cu", "fdga_noalloc.cu", "fdga_anderson.cu", "fdga_anderson32.cu", "fdga_krylov.cu", "fdga_k3_tc.cu", "fdga_k3_tma.cu", "fdga_k3_oz.cu", "fdga_k3_mma.cu", "fdga_mfrg.cu", "fdga_adjoint.cu", "fdga_interp.cu"]
-HEADERS = ["fdga_device.cuh", "fdga_digits.cuh", "fdga_kernels.h"]
+HEADERS = ["fdga_device.cuh", "fdga_digits.cuh", "fdga_kernels.h", "fdga_ring.h"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 
 
