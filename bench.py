@@ -230,8 +230,8 @@ def k3_gemm_roofline(S, stages, cfg_name):
     representative (P, Ω) block); complex MAC = 8 real flops.  On the FP64 CUDA-core kernel
     (k_bse_K3_gemm) the FP64 pipe bounds it; on the digit-sliced tensor-core kernel (k_bse_K3_oz,
     the default above Nν3 = 32) the 16-bit MMA work is compared with the measured bf16 peak
-    and its FP64-equivalent rate with the FP64 pipe.  `flops_per_launch` counts the 36 pairs of an
-    8-digit product, the yardstick; the kernel issues 28 (seven digits), `issued_*`."""
+    and its FP64-equivalent rate with the FP64 pipe; `flops_per_launch` counts the 36 MMAs of an
+    8-digit product that the kernel issues."""
     nb, N = S.query("k3_blocks"), S.query("k3_block_dim")
     ms = stages["bse_K3_gemm"]
     flops = 3 * nb * 8 * N ** 3
@@ -248,8 +248,7 @@ def k3_gemm_roofline(S, stages, cfg_name):
         return {"bound": "tensor", "kernel": "k_bse_K3_oz<1> (fused K3 BSE, FP64 by digit slicing on tcgen05)",
                 "achieved": tc, "peak": bf16, "unit": "TFLOP/s", "frac": tc / bf16,
                 "peak_source": "fallback" if peaks.get("fallback") else "measured (bf16_tflops)",
-                "flops_per_launch": mma_flops, "issued_flops_per_launch": mma_flops * 28 // 36,
-                "issued_frac": tc * 28 / 36 / bf16, "fp64_equivalent_tflops": achieved, "fp64_pipe_peak": fp64_peak,
+                "flops_per_launch": mma_flops, "fp64_equivalent_tflops": achieved, "fp64_pipe_peak": fp64_peak,
                 "fp64_equivalent_frac": achieved / fp64_peak,
                 "traffic": profile_traffic(f"k_bse_K3_oz_{cfg_name}.md"), "algorithmic_bytes": byts,
                 "hbm_achieved_gbs": byts / (ms * 1e-3) / 1e9, "hbm_peak_gbs": hbm,

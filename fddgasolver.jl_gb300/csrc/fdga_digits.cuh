@@ -29,7 +29,7 @@ __device__ __forceinline__ double i2d_scaled(long long x, int e) {
 // An FP64 value as S balanced base-256 digits relative to a bound 2^(F-1022) > |v|: Y = v 2^(8S-2+1022-F)
 // rounded to an integer (0 for zero and subnormal v), |Y| ≤ 2^(8S-2); adding 0x80 to every byte of Y makes
 // byte k < S, less 128, the digit of weight 256^k, in [-128, 127].  S = 8: 62 fractional bits, exact for every
-// v within 2^9 of the bound; S = 7: 54, exact within 2.
+// v within 2^9 of the bound.
 template <int S>
 __device__ __forceinline__ long long fixed_digits(double v, int F) {
     const unsigned long long b = (unsigned long long)__double_as_longlong(v);

@@ -19,7 +19,7 @@
 // the digit).  The products of digit pairs (s, t) with s + t = g ≤ 7 share one FP32 accumulator:
 // products are at most 2^14 and at most 8·64 of them meet in one accumulator, so every partial sum is an
 // integer of at most 2^23 and exact.  The pairs with s + t ≥ 8 are dropped; with the rounding of Y they
-// leave below 2^-60 of (row bound)·(column bound) per product term, and the 36 digit products replace the
+// leave below 2^-58.9 of (row bound)·(column bound) per product term, and the 36 digit products replace the
 // FP64 operations (three real products per complex one, 64 issue slots each).  The epilogue joins the
 // eight integers exactly in two 64-bit integers and one FP64 addition, then applies T and γL as the
 // CUDA-core kernel does.  A row of A or a column of M that holds an infinity or NaN gives NaN in that row

@@ -7,38 +7,39 @@
 // column tiles of NT = 64 real columns.
 //
 // Exact slicing.  Row ν of A and column ν' of M each have a bound 2^(F-1022) from the largest exponent
-// field of their entries.  An entry becomes a 54-bit fixed-point integer relative to its bound and is cut
-// into S = 7 balanced base-256 digits, FP16 numbers exactly (fdga_digits.cuh).  The products of digit
-// pairs (s, t) with s + t = g share one FP32 accumulator in tensor memory (g = 0..6, 7 x 64 columns).  The
-// top digits are at most 64 and the others 128, so with K ≤ 256 the diagonals g ≤ 3 stay below 2^24 and are
-// exact; the last ones pass 2^24 only when nearly all digits of a row and a column have full size and
-// equal signs, and then round at one unit of a diagonal g ≥ 4 (2^-44 of the bounds).  The pairs with
-// s + t ≥ 7 are dropped; with the rounding of the entries they leave below 2^-52 of (row bound)·(column
-// bound) per product term, the size of an FP64 rounding.  The epilogue joins the diagonals exactly in two
-// 64-bit integers with one FP64 addition, then applies T and γL, as the FP64 kernel does.  A row of A or
-// column of M with an infinity or NaN gives NaN there, as the FP64 sums do.
+// field of their entries.  An entry becomes a 62-bit fixed-point integer relative to its bound and is cut
+// into S = 8 balanced base-256 digits, FP16 numbers exactly (fdga_digits.cuh).  The products of digit
+// pairs (s, t) with s + t = g share one FP32 accumulator in tensor memory (g = 0..7, 8 x 64 columns: all of
+// it).  The top digits are at most 64 and the others 128, so a diagonal of K products is at most g K 2^14: all
+// are exact for K ≤ 128 (Nν3 ≤ 64), and the diagonals g ≤ 4 for K ≤ 256; the others pass 2^24 there only when
+// nearly all digits of a row and a column have full size and equal signs, and then round by a unit of a
+// diagonal g ≥ 5 (2^-52 of the bounds).  The pairs with s + t ≥ 8 are dropped; with the rounding of the entries
+// they leave below 2^-58.9 of (row bound)·(column bound) per product term, which is less than an FP64 product's
+// rounding for terms within 2^5 of the bounds.  (Seven digits, 54 bits, left up to 2^-51.2, more than the 2^-53.2
+// of the 8 x 7-bit form before them, and took 302 / 442 us where eight take 331 / 496: 4x4, nK3 = (20, 40).)
+// The epilogue joins the diagonals exactly in two 64-bit integers with one FP64 addition, then applies T and γL,
+// as the FP64 kernel does.  A row of A or column of M with an infinity or NaN gives NaN there, as the FP64 sums do.
 //
 // Per launch and group of blocks: k_oz_adigits finds F of every row of every A block and writes its digit
 // operands to a global buffer, once per block, in the shared-memory operand layout; then the contraction
 // runs one CTA per (channel slot, block, column tile), two CTAs per SM: eight worker warps and a control
 // warp.  A worker forms N/8 entries of the tile of M in FP64 in registers, all their loads independent, and
 // the workers find the column bounds; then, K in chunks of 16 (8 ω, one entry per worker), they digitise
-// chunk after chunk into one of the stages (three for L_K3 up to Nν3 = 96, else two) while the control thread
-// keeps the A digits of the next chunks in flight (cp.async.bulk on an mbarrier) and issues the 28 MMAs of a
-// chunk when both have arrived (kind::f16, FP32 accumulation, committed to the stage's mbarrier).  The accumulators take the whole tensor memory of an
-// SM, so the CTA allocates it only once its M is formed and gives it back as soon as the accumulators are
-// joined into shared memory: the MMAs of one CTA run while its neighbour on the SM forms M or writes its
-// results.  The rows above N of the 128-row A operands are whatever lies behind them in shared memory: they
-// reach only rows of D that are not read.  Every wait on an mbarrier is bounded (a timeout sets *err and the
-// CTA's abort flag; the control thread still waits, bounded, for its copies and MMAs in flight before the
-// tensor memory is released).
+// chunk after chunk into one of the stages (three for L_K3 up to Nν3 = 80, else two) while the control thread
+// keeps the A digits of the next chunks in flight (cp.async.bulk on an mbarrier) and issues the 36 MMAs of a
+// chunk when both have arrived (kind::f16, FP32 accumulation, committed to the stage's mbarrier).  The
+// accumulators take the whole tensor memory of an SM, so the CTA allocates it only once its M is formed and
+// gives it back as soon as the accumulators are joined into shared memory: the MMAs of one CTA run while its
+// neighbour on the SM forms M or writes its results.  The rows above N of the 128-row A operands are whatever
+// lies behind them in their stage: they reach only rows of D that are not read.  Every wait on an mbarrier is
+// bounded (a timeout sets *err and the CTA's abort flag; the control thread still waits, bounded, for its copies
+// and MMAs in flight before the tensor memory is released).
 //
 // What bounds it: the MMAs, which cost about the same for 32 columns as for 64 (the 128-row A operand is
 // read for each), then the FP64 pipe (8 to 12 operations per entry of M and 2 to 6 per output).  The form
 // before had 32-column tiles, 36 BF16 MMAs of 7-bit digits, an FP32 bound pass over the operands of M, and M
 // formed and digitised per chunk between two CTA barriers.  L_K3 / K3 stage in us on GB300, that form -> this:
-// 4x4, nK3 = (20, 40) (Nν3 = 80, 702 blocks) 430 / 609 -> 302 / 443; 8x8, nK3 = (20, 40) 1030 / 1460 -> 713 / 1034;
-// the largest error of that map against its extended-precision restatement 2.0e-15 -> 0.5e-15.
+// 4x4, nK3 = (20, 40) (Nν3 = 80, 702 blocks) 429 / 607 -> 331 / 496; 8x8, nK3 = (20, 40) 1030 / 1460 -> 789 / 1160.
 #include <algorithm>
 
 #include "fdga_digits.cuh"
@@ -51,11 +52,11 @@ namespace {
 
 constexpr int WORKERS = 256;              // threads that form and digitise M
 constexpr int OZ_THREADS = WORKERS + 32;  // and the control warp
-constexpr int S = 7;                      // digits per operand
+constexpr int S = 8;                      // digits per operand
 constexpr int KC = 16;                    // real K per chunk (one FP16 MMA)
 constexpr int CW = KC / 2;                // ω per chunk
 constexpr int NT = 64;                    // real columns per tile
-constexpr int TCOLS = 512;                // tensor-memory columns (S·NT, rounded up to a power of two)
+constexpr int TCOLS = S * NT;             // tensor-memory columns (512: all of them)
 constexpr int B_DIG = NT * KC * 2;        // one B digit operand: 64 rows x 16 FP16 = 2 KB
 constexpr int CPITCH = NT / 2 + 1;        // complex values between rows of the results (one pad: 16-byte stores
                                           // of neighbouring rows fall on distinct banks)
@@ -153,16 +154,13 @@ template <int MODE, int MAXC, int NS>
 __global__ void __launch_bounds__(OZ_THREADS, 2)
     k_bse_K3_oz(K3Args3 args, Dims d, int ntile, const int* __restrict__ fa, const uint8_t* __restrict__ adig, int r0,
                 int* err) {
-    extern __shared__ __align__(1024) uint8_t sm[];  // NS stages; later the results
+    extern __shared__ __align__(128) uint8_t sm[];  // NS stages; later the results; behind them qf
     __shared__ uint64_t done_[NS];   // per stage: the chunk's MMAs are done (tcgen05.commit)
     __shared__ uint64_t afull_[NS];  // per stage: the chunk's A digit operands have arrived
     __shared__ uint64_t bfull_[NS];  // per stage: the workers have written the chunk's B digit operands
     __shared__ uint32_t tmem_base;
     __shared__ int abort_;
     __shared__ int committed_;  // chunks whose MMAs were committed
-    // the ω factors of M with their signs: [0] Π0 (mode 0), s1 (Π - Π0) (mode 1) or s1 dΠ (mode 3),
-    // [1] s1 Π
-    __shared__ cplx qf[128][2];
     __shared__ int cmax[NT / 2];  // largest exponent fields of the columns of M
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const bool worker = warp < WORKERS / 32;
@@ -187,6 +185,9 @@ __global__ void __launch_bounds__(OZ_THREADS, 2)
     auto afull = [&](int st) { return smem_u32(afull_ + st); };
     auto bfull = [&](int st) { return smem_u32(bfull_ + st); };
     const uint32_t arow = (uint32_t)N * 32u, stage = stage_bytes(N);
+    // the ω factors of M with their signs: [0] Π0 (mode 0), s1 (Π - Π0) (mode 1) or s1 dΠ (mode 3),
+    // [1] s1 Π
+    cplx(*qf)[2] = reinterpret_cast<cplx(*)[2]>(sm + max(NS * stage, (uint32_t)(N * CPITCH) * (uint32_t)sizeof(cplx)));
     // A: row ν, k = 2ω_l holds Re A, 2ω_l + 1 holds Im A; the S operands of a chunk arrive by one copy
     auto copy_A = [&](int c) {
         const int st = ring_stage(c, NS);
@@ -431,15 +432,16 @@ bool k3_oz_supported(const Dims& d) {
     return d.N3n >= 8 && d.N3n <= 128 && (d.N3n % 8) == 0;
 }
 
-// the stages (an A operand is read up to row 127, behind the last digit's N rows), or the results
+// the stages (an A operand is read up to row 127: behind the last digit's N rows into the stage's 16 KB of B), or
+// the results; then the ω factors
 static size_t k3_oz_smem(const Dims& d, int ns) {
     const size_t N = (size_t)d.N3n;
-    return std::max(ns * (size_t)stage_bytes(d.N3n) + (128 - N) * 32, N * CPITCH * sizeof(cplx));
+    return std::max(ns * (size_t)stage_bytes(d.N3n), N * CPITCH * sizeof(cplx)) + 2 * N * sizeof(cplx);
 }
 
 // NS: stages of mode 0, where the MMAs wait for the operands; modes 1 and 3 are bound by forming M, whose loads
-// want the L1 cache that a third stage takes (K3 contraction at 4x4, nK3 = (20, 40): 394 us with two stages, 407
-// with three; L_K3: 305 and 248)
+// want the L1 cache that a third stage takes (4x4, nK3 = (20, 40): K3 kernel, at seven digits, 394 us with two
+// stages, 407 with three; L_K3 stage 392 and 331).  Above Nν3 = 80 three stages leave room for one CTA on an SM only.
 template <int MAXC, int NS>
 static cudaError_t prepare_oz(const Dims& d) {
     static SmemRecord set0, set1, set3;
@@ -449,7 +451,9 @@ static cudaError_t prepare_oz(const Dims& d) {
     return e;
 }
 cudaError_t prepare_bse_K3_oz(const Dims& d) {
-    return d.N3n <= 64 ? prepare_oz<8, 3>(d) : (d.N3n <= 96 ? prepare_oz<12, 3>(d) : prepare_oz<16, 2>(d));
+    if (d.N3n <= 64) return prepare_oz<8, 3>(d);
+    if (d.N3n <= 80) return prepare_oz<12, 3>(d);
+    return d.N3n <= 96 ? prepare_oz<12, 2>(d) : prepare_oz<16, 2>(d);
 }
 
 // mode 0 (BSE_L_K3), 1 (BSE_K3), 2 (the tangent dK3 = T (dA·M + A·dM) + dγL): mode 2 runs as two
@@ -495,7 +499,8 @@ cudaError_t launch_bse_K3_oz(cudaStream_t s, int mode, const K3Args3& a, int nsl
     if (!k3_oz_supported(d) || mode < 0 || mode > 2 || !fa_scratch || !adig || adig_blocks < 1)
         return cudaErrorInvalidValue;
     if (d.N3n <= 64) return launch_oz<8, 3>(s, mode, a, nslots, d, err, fa_scratch, adig, adig_blocks);
-    if (d.N3n <= 96) return launch_oz<12, 3>(s, mode, a, nslots, d, err, fa_scratch, adig, adig_blocks);
+    if (d.N3n <= 80) return launch_oz<12, 3>(s, mode, a, nslots, d, err, fa_scratch, adig, adig_blocks);
+    if (d.N3n <= 96) return launch_oz<12, 2>(s, mode, a, nslots, d, err, fa_scratch, adig, adig_blocks);
     return launch_oz<16, 2>(s, mode, a, nslots, d, err, fa_scratch, adig, adig_blocks);
 }
 
