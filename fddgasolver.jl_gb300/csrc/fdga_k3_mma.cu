@@ -22,8 +22,18 @@
 // leave below 2^-58.9 of (row bound)·(column bound) per product term, and the 36 digit products replace the
 // FP64 operations (three real products per complex one, 64 issue slots each).  The epilogue joins the
 // eight integers exactly in two 64-bit integers and one FP64 addition, then applies T and γL as the
-// CUDA-core kernel does.  A row of A or a column of M that holds an infinity or NaN gives NaN in that row
-// or column, as the FP64 sums do.
+// CUDA-core kernel does.
+//
+// To what the accuracy is relative.  Where a row and a column have large entries at a common ω, the bounds are
+// about Σ_ω |A||M| and the digits beat an FP64 sum's rounding.  Operands graded against each other (A falls along
+// ω as M rises) have bounds far above it: entries 2^k below theirs keep 62 - k bits.  So one more product, of the
+// top digits in magnitude, sees whether any ω has a nonzero top digit on both sides, that is Σ |A||M| ≥ 2^-14 of
+// the bounds and an error below 2 Nν3 2^-45 of it; an output without one is summed again in FP64, one ω per lane
+// (A falling by 2^39 as M rises: error 1e-7 of Σ |A||M| -> 1e-16).  That is so in the adjoint and below Nν3 = 32,
+// where FP64 sums ran before; few outputs of the lattice workloads are (Hubbard 8x8, nK3 = (8, 12): K3 38 us with
+// and without; the residual call 584 -> 587 us).  At Nν3 = 32 the map's digits stand by themselves, as did the form before with bounds of whole blocks: a SIAM has outputs far from the
+// diagonal that would be summed again (K3 18 -> 43 us).  A row of A or a column of M that holds an infinity or NaN,
+// or products near the end of the normal range, are summed in FP64 everywhere.
 //
 // What bounds it: forming M (8 to 14 FP64 operations per entry) and the latency of one pass load ->
 // digits -> MMA -> store; a CTA of NC·NC warps (NC = ⌈Nν3/8⌉) does one block, each warp staging one 8 x 8
@@ -63,11 +73,13 @@ __device__ __forceinline__ void store_digits(uint8_t* planes, int o, cplx v0, cp
 }
 
 // One N x N complex product per CTA of NC·NC warps: av = two neighbouring k of row cl of the left operand,
-// mv = the same k of column cl of the right one; out(row, column, value, non-finite) is called by the lane
-// that holds an element.  fmax_ is zero on entry and a __syncthreads lies behind that.
-template <int NC, class OUT>
-__device__ __forceinline__ void digit_product(uint8_t* sm, int (*fmax_)[8 * NC], int N, int cl, int w0,
-                                              const cplx (&av)[2], const cplx (&mv)[2], OUT&& out) {
+// mv = the same k of column cl of the right one; out(row, column, value) is called by the lane that holds an
+// element, term(row, column, k) is the product of the two operands' elements at k in FP64, for outputs of operands
+// graded against each other (where `graded`) or not finite.  fmax_ is zero on entry and a __syncthreads lies behind
+// that.
+template <int NC, class TERM, class OUT>
+__device__ __forceinline__ void digit_product(uint8_t* sm, int (*fmax_)[8 * NC], int N, int cl, int w0, bool graded,
+                                              const cplx (&av)[2], const cplx (&mv)[2], TERM&& term, OUT&& out) {
     uint8_t* Mp = sm;
     uint8_t* Ap = sm + 2 * S * PLANE<NC>;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -93,6 +105,13 @@ __device__ __forceinline__ void digit_product(uint8_t* sm, int (*fmax_)[8 * NC],
     for (int g = 0; g < S; ++g)
 #pragma unroll
         for (int i = 0; i < 4; ++i) acc[g][i] = 0.0f;
+    float mag[4] = {0.0f, 0.0f, 0.0f, 0.0f};  // Σ of the top digits' products in magnitude
+    auto mma = [](float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+        asm volatile(
+            "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+            : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+            : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+    };
     // lane l addresses row l % 8 of matrix l / 8: M re, M im, A re, A im of one digit
     const uint32_t laddr = (uint32_t)__cvta_generic_to_shared(
         (lane < 16 ? Mp + (8 * j + (lane & 7)) * PITCH<NC> : Ap + (8 * nt + (lane & 7)) * PITCH<NC>) +
@@ -110,34 +129,39 @@ __device__ __forceinline__ void digit_product(uint8_t* sm, int (*fmax_)[8 * NC],
 #pragma unroll
         for (int s = 0; s < S; ++s)
 #pragma unroll
-            for (int t = 0; s + t < S; ++t)
-                asm volatile(
-                    "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
-                    "{%0,%1,%2,%3};"
-                    : "+f"(acc[s + t][0]), "+f"(acc[s + t][1]), "+f"(acc[s + t][2]), "+f"(acc[s + t][3])
-                    : "r"(mr[s]), "r"(mi[s]), "r"(mi[s] ^ 0x80008000u), "r"(mr[s]), "r"(ar[t]), "r"(ai[t]));
+            for (int t = 0; s + t < S; ++t) mma(acc[s + t], mr[s], mi[s], mi[s] ^ 0x80008000u, mr[s], ar[t], ai[t]);
+        const uint32_t pm = 0x7fff7fffu;
+        mma(mag, mr[0] & pm, mi[0] & pm, mi[0] & pm, mr[0] & pm, ar[0] & pm, ai[0] & pm);
     }
     const int col = 8 * j + (lane >> 2);
-    if (col >= N) return;
-    const int FM = fmax_[1][col];
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
         const int nu = 8 * nt + 2 * (lane & 3) + e;
-        if (nu >= N) continue;
-        const int FA = fmax_[0][nu], E = FA + FM;
-        if (FA == 0x7ff || FM == 0x7ff) {
-            const double qn = __longlong_as_double(0x7ff8000000000000ll);
-            out(nu, col, mk(qn, qn), true);
-            continue;
-        }
-        double p[2];
+        const bool in = col < N && nu < N;
+        cplx v = mk(0.0, 0.0);
+        bool weak = false;
+        if (in) {
+            const int FA = fmax_[0][nu], FM = fmax_[1][col], E = FA + FM;
+            double p[2];
 #pragma unroll
-        for (int q = 0; q < 2; ++q) {
-            const float a[8] = {acc[0][2 * q + e], acc[1][2 * q + e], acc[2][2 * q + e], acc[3][2 * q + e],
-                                acc[4][2 * q + e], acc[5][2 * q + e], acc[6][2 * q + e], acc[7][2 * q + e]};
-            p[q] = join_digits<S>(a, E);
+            for (int q = 0; q < 2; ++q) {
+                const float a[8] = {acc[0][2 * q + e], acc[1][2 * q + e], acc[2][2 * q + e], acc[3][2 * q + e],
+                                    acc[4][2 * q + e], acc[5][2 * q + e], acc[6][2 * q + e], acc[7][2 * q + e]};
+                p[q] = join_digits<S>(a, E);
+            }
+            v = mk(p[0], p[1]);
+            // (a row or column of zeros has F = 0: its sums are 0)
+            // (E below 1100: outputs near the end of the normal range, where the join flushes)
+            weak = FA != 0 && FM != 0 &&
+                   (FA == 0x7ff || FM == 0x7ff || E < 1100 || (graded && mag[e] == 0.0f && mag[2 + e] == 0.0f));
         }
-        out(nu, col, mk(p[0], p[1]), false);
+        for (unsigned todo = __ballot_sync(0xffffffffu, weak); todo; todo &= todo - 1) {  // one k per lane
+            const int src = __ffs(todo) - 1;
+            const int r = 8 * nt + 2 * (src & 3) + e, c = 8 * j + (src >> 2);
+            const cplx t = warp_sum(lane < N ? term(r, c, lane) : mk(0.0, 0.0));
+            if (lane == src) v = t;
+        }
+        if (in) out(nu, col, v);
     }
 }
 
@@ -179,6 +203,31 @@ __global__ void __launch_bounds__(32 * NC * NC) k_bse_K3_mma(K3Args3 args, Dims 
         qf[tid][0] = q0;
         qf[tid][1] = q1;
     }
+    // entry (ω, ν') of M: q[0] x0 + q[1] x1
+    auto load_M = [&](int w, int cl, cplx& x0, cplx& x1) {
+        x0 = ldg(a.B0 + base + (size_t)w * N + cl);
+        if (!full) return;
+        // s2 Π = ±s1 Π: the γL terms join the Γ terms before the products
+        const size_t ig = (CH == CH_P) ? base + (size_t)w * N + cl : base + (size_t)cl * N + w;
+        const int ot = cross(CH, m, w - d.n3n);
+        const bool hl = fin(ot, d.n3n);
+        const size_t il = base + (size_t)(ot + d.n3n) * N + cl;
+        cplx g = ldg(a.G + ig);
+        if (hl) {
+            const cplx l = gl_of(a.FLc, a.FLt, a.FLa, il);
+            g = (s1 == s2) ? g + l : g - l;
+        }
+        if (MODE == 3) {  // dM = s1 dΠ (F0 + Γ ± γL) + s1 Π (dΓ ± dγL)
+            x0 += g;
+            g = ldg(a.tG + ig);
+            if (hl) {
+                const cplx l = gl_of(a.tFLc, a.tFLt, a.tFLa, il);
+                g = (s1 == s2) ? g + l : g - l;
+            }
+        }
+        x1 = g;
+    };
+    auto form_M = [&](int w, cplx x0, cplx x1) { return full ? cfma(qf[w][0], x0, qf[w][1] * x1) : qf[w][0] * x0; };
     // staging: warp = (column chunk, ω chunk); a lane holds one column (row of A) and two neighbouring ω
     const int cl = 8 * (warp % NC) + (lane & 7), w0 = 8 * (warp / NC) + 2 * (lane >> 3);
     cplx av[2], x0[2], x1[2];
@@ -188,53 +237,29 @@ __global__ void __launch_bounds__(32 * NC * NC) k_bse_K3_mma(K3Args3 args, Dims 
         av[i] = x0[i] = x1[i] = mk(0.0, 0.0);
         if (cl >= N || w >= N) continue;
         av[i] = ldg(a.A + base + (size_t)cl * N + w);
-        x0[i] = ldg(a.B0 + base + (size_t)w * N + cl);
-        if (full) {
-            // s2 Π = ±s1 Π: the γL terms join the Γ terms before the products
-            const size_t ig = (CH == CH_P) ? base + (size_t)w * N + cl : base + (size_t)cl * N + w;
-            const int ot = cross(CH, m, w - d.n3n);
-            const bool hl = fin(ot, d.n3n);
-            const size_t il = base + (size_t)(ot + d.n3n) * N + cl;
-            cplx g = ldg(a.G + ig);
-            if (hl) {
-                const cplx l = gl_of(a.FLc, a.FLt, a.FLa, il);
-                g = (s1 == s2) ? g + l : g - l;
-            }
-            if (MODE == 3) {  // dM = s1 dΠ (F0 + Γ ± γL) + s1 Π (dΓ ± dγL)
-                x0[i] += g;
-                g = ldg(a.tG + ig);
-                if (hl) {
-                    const cplx l = gl_of(a.tFLc, a.tFLt, a.tFLa, il);
-                    g = (s1 == s2) ? g + l : g - l;
-                }
-            }
-            x1[i] = g;
-        }
+        load_M(w, cl, x0[i], x1[i]);
     }
     __syncthreads();
     cplx mv[2];
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
-        mv[i] = mk(0.0, 0.0);
-        if (cl < N && w0 + i < N) {
-            const cplx* q = qf[w0 + i];
-            mv[i] = full ? cfma(q[0], x0[i], q[1] * x1[i]) : q[0] * x0[i];
-        }
-    }
-    digit_product<NC>(sm, fmax_, N, cl, w0, av, mv, [&](int nu, int col, cplx cv, bool bad) {
+    for (int i = 0; i < 2; ++i) mv[i] = cl < N && w0 + i < N ? form_M(w0 + i, x0[i], x1[i]) : mk(0.0, 0.0);
+    auto term = [&](int nu, int col, int w) {
+        cplx y0, y1 = mk(0.0, 0.0);
+        load_M(w, col, y0, y1);
+        return ldg(a.A + base + (size_t)nu * N + w) * form_M(w, y0, y1);
+    };
+    digit_product<NC>(sm, fmax_, N, cl, w0, N < 32, av, mv, term, [&](int nu, int col, cplx cv) {
         const size_t io = base + (size_t)nu * N + col;
-        cplx o = cv;
-        if (!bad) {
-            if (MODE == 0) {
-                o = cv * (d.T * ((CH == CH_A) ? 1.0 : -1.0));
-            } else if (a.flags & K3F_NOEPI) {
-                o = cv * d.T;
-            } else {
-                const cplx g = (MODE == 3) ? gl_of(a.tFLc, a.tFLt, a.tFLa, io) : gl_of(a.FLc, a.FLt, a.FLa, io);
-                o = cplx{fma(cv.x, d.T, g.x), fma(cv.y, d.T, g.y)};
-            }
-            if (a.flags & K3F_ACC) o = a.out[io] + o;
+        cplx o;
+        if (MODE == 0) {
+            o = cv * (d.T * ((CH == CH_A) ? 1.0 : -1.0));
+        } else if (a.flags & K3F_NOEPI) {
+            o = cv * d.T;
+        } else {
+            const cplx g = (MODE == 3) ? gl_of(a.tFLc, a.tFLt, a.tFLa, io) : gl_of(a.FLc, a.FLt, a.FLa, io);
+            o = cplx{fma(cv.x, d.T, g.x), fma(cv.y, d.T, g.y)};
         }
+        if (a.flags & K3F_ACC) o = a.out[io] + o;
         a.out[io] = o;
     });
 }
@@ -255,27 +280,24 @@ __global__ void __launch_bounds__(32 * NC * NC) k_adj_mma(GemmBatch g, Dims d) {
     cplx* C = (slot == 0 ? g.C[0] : slot == 1 ? g.C[1] : g.C[2]) + base;
     const double alpha = slot == 0 ? g.alpha[0] : slot == 1 ? g.alpha[1] : g.alpha[2];
     if (tid < 8 * NC) fmax_[0][tid] = fmax_[1][tid] = 0;
+    auto left = [&](int r, int w) { return OPA == 0 ? ldg(A + (size_t)r * N + w) : conjg(ldg(A + (size_t)w * N + r)); };
+    auto right = [&](int c, int w) { return OPA == 0 ? conjg(ldg(B + (size_t)c * N + w)) : ldg(B + (size_t)w * N + c); };
     const int cl = 8 * (warp % NC) + (lane & 7), w0 = 8 * (warp / NC) + 2 * (lane >> 3);
     cplx av[2], mv[2];
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
         const int w = w0 + i;
-        av[i] = mv[i] = mk(0.0, 0.0);
-        if (cl >= N || w >= N) continue;
-        if (OPA == 0) {
-            av[i] = ldg(A + (size_t)cl * N + w);
-            mv[i] = conjg(ldg(B + (size_t)cl * N + w));
-        } else {
-            av[i] = conjg(ldg(A + (size_t)w * N + cl));
-            mv[i] = ldg(B + (size_t)w * N + cl);
-        }
+        const bool in = cl < N && w < N;
+        av[i] = in ? left(cl, w) : mk(0.0, 0.0);
+        mv[i] = in ? right(cl, w) : mk(0.0, 0.0);
     }
     __syncthreads();
-    digit_product<NC>(sm, fmax_, N, cl, w0, av, mv, [&](int r, int c, cplx cv, bool bad) {
-        cplx* o = C + (size_t)r * N + c;
-        const cplx v = bad ? cv : cv * alpha;
-        *o = g.accumulate ? *o + v : v;
-    });
+    digit_product<NC>(sm, fmax_, N, cl, w0, true, av, mv, [&](int r, int c, int w) { return left(r, w) * right(c, w); },
+                      [&](int r, int c, cplx cv) {
+                          cplx* o = C + (size_t)r * N + c;
+                          const cplx v = cv * alpha;
+                          *o = g.accumulate ? *o + v : v;
+                      });
 }
 
 template <int MODE, int NC>

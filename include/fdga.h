@@ -126,11 +126,14 @@ int fdga_set_precision(fdga_handle* h, int precision);
  * "fused_residual" (default 1): fdga_residual on page-locked x and R runs as one CUDA graph whose
  * host copies overlap the iteration; 0: copy, iterate and copy back in sequence.
  * "k3_fp64_tensor_cores" (default 2): the FP64 map's K3 contractions (BSE_L_K3 and BSE_K3) run on
- * the tensor cores by exact digit slicing of the FP64 operands (8 balanced 8-bit digits per row of A and
- * column of M, products summed by diagonal in FP32, joined exactly; FP64-level results): 2 on tcgen05 when
- * Nν3 is a multiple of 8 between 40 and 128 and on warp-level tensor-core products at every Nν3 up to 32,
- * 1 (or 3) on tcgen05 at every multiple of 8 between 8 and 128 (CUDA cores elsewhere), 0 never (FP64
- * CUDA-core GEMMs). */
+ * the tensor cores by exact digit slicing of the FP64 operands (8 balanced 8-bit digits per entry, 62 bits
+ * relative to the largest entry of its row of A or column of M; products summed by diagonal in FP32, joined
+ * exactly): 2 on tcgen05 when Nν3 is a multiple of 8 between 40 and 128 and on warp-level tensor-core products
+ * at every Nν3 up to 32, 1 (or 3, the same) on tcgen05 at every multiple of 8 between 8 and 128 (CUDA cores
+ * elsewhere), 0 never (FP64 CUDA-core GEMMs).  An output's error is below 2 Nν3 2^-58.9 of (largest of A's row)
+ * x (largest of M's column): that of an FP64 sum where the two are large at a common frequency.  Below Nν3 = 32,
+ * and up to it in fdga_rrule, outputs whose row and column are not (operands graded against each other) are
+ * summed in FP64; from 32 on in the map, use 0 for such operands. */
 int fdga_set_option(fdga_handle* h, const char* key, int value);
 
 /* fixed_point!(R, x, S) (src/solve.jl:119-157): unflatten x, iterate, R = flatten(S) - x.
