@@ -29,9 +29,11 @@
 // ω as M rises) have bounds far above it: entries 2^k below theirs keep 62 - k bits.  So one more product, of the
 // top digits in magnitude, sees whether any ω has a nonzero top digit on both sides, that is Σ |A||M| ≥ 2^-14 of
 // the bounds and an error below 2 Nν3 2^-45 of it; an output without one is summed again in FP64, one ω per lane
-// (A falling by 2^39 as M rises: error 1e-7 of Σ |A||M| -> 1e-16).  That is so in the adjoint and below Nν3 = 32,
-// where FP64 sums ran before; few outputs of the lattice workloads are (Hubbard 8x8, nK3 = (8, 12): K3 38 us with
-// and without; the residual call 584 -> 587 us).  At Nν3 = 32 the map's digits stand by themselves, as did the form before with bounds of whole blocks: a SIAM has outputs far from the
+// (A falling by 2^39 as M rises, Nν3 = 24: error 8e-9 of the largest output -> an FP64 sum's).  That is so in the
+// adjoint and below Nν3 = 32, where FP64 sums ran before.  Few outputs of the lattice workloads' maps are summed
+// again (Hubbard 8x8, nK3 = (8, 12): K3 38 us with and without; the residual call 584 -> 587 us), in the adjoint a
+// sixth of one product's, far from the diagonal (700 -> 733 us; one output at a time, each part by itself, 776).
+// At Nν3 = 32 the map's digits stand by themselves, as did the form before with bounds of whole blocks: a SIAM has outputs far from the
 // diagonal that would be summed again (K3 18 -> 43 us).  A row of A or a column of M that holds an infinity or NaN,
 // or products near the end of the normal range, are summed in FP64 everywhere.
 //
@@ -70,6 +72,22 @@ __device__ __forceinline__ void store_digits(uint8_t* planes, int o, cplx v0, cp
         *reinterpret_cast<uint32_t*>(p) = digit_pair(r0, r1, S - 1 - s);
         *reinterpret_cast<uint32_t*>(p + PLANE<NC>) = digit_pair(i0, i1, S - 1 - s);
     }
+}
+
+// Warp sums of eight values: that of x[i] in x[0] of the lanes 4i .. 4i + 3 (9 additions for the 40 of eight sums by
+// themselves: FP64 bounds an output summed again).
+__device__ __forceinline__ void sum8(double (&x)[8], int lane) {
+#pragma unroll
+    for (int h = 4; h >= 1; h >>= 1) {  // lanes 4h apart exchange halves
+        const bool up = (lane & (4 * h)) != 0;
+#pragma unroll
+        for (int i = 0; i < h; ++i) {
+            const double keep = up ? x[i + h] : x[i], send = up ? x[i] : x[i + h];
+            x[i] = keep + __shfl_xor_sync(0xffffffffu, send, 4 * h);
+        }
+    }
+    x[0] += __shfl_xor_sync(0xffffffffu, x[0], 2);
+    x[0] += __shfl_xor_sync(0xffffffffu, x[0], 1);
 }
 
 // One N x N complex product per CTA of NC·NC warps: av = two neighbouring k of row cl of the left operand,
@@ -155,11 +173,27 @@ __device__ __forceinline__ void digit_product(uint8_t* sm, int (*fmax_)[8 * NC],
             weak = FA != 0 && FM != 0 &&
                    (FA == 0x7ff || FM == 0x7ff || E < 1100 || (graded && mag[e] == 0.0f && mag[2 + e] == 0.0f));
         }
-        for (unsigned todo = __ballot_sync(0xffffffffu, weak); todo; todo &= todo - 1) {  // one k per lane
-            const int src = __ffs(todo) - 1;
-            const int r = 8 * nt + 2 * (src & 3) + e, c = 8 * j + (src >> 2);
-            const cplx t = warp_sum(lane < N ? term(r, c, lane) : mk(0.0, 0.0));
-            if (lane == src) v = t;
+        for (unsigned todo = __ballot_sync(0xffffffffu, weak); todo;) {  // four outputs at a time, one k per lane
+            int src[4];
+            double x[8];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                src[i] = todo ? __ffs(todo) - 1 : src[0];
+                todo &= todo - 1;
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                cplx t = mk(0.0, 0.0);
+                if (lane < N) t = term(8 * nt + 2 * (src[i] & 3) + e, 8 * j + (src[i] >> 2), lane);
+                x[2 * i] = t.x;
+                x[2 * i + 1] = t.y;
+            }
+            sum8(x, lane);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const cplx t = mk(__shfl_sync(0xffffffffu, x[0], 8 * i), __shfl_sync(0xffffffffu, x[0], 8 * i + 4));
+                if (lane == src[i]) v = t;
+            }
         }
         if (in) out(nu, col, v);
     }
