@@ -17,6 +17,7 @@ mΠν_factor=32, seeded synthetic RefVertex), init_sym_grp! symmetry groups.
 """
 import argparse
 import json
+import math
 import os
 import statistics
 import subprocess
@@ -228,7 +229,9 @@ def profile_traffic(name):
 def k3_gemm_roofline(S, stages, cfg_name):
     """Roofline of the fused K3 BSE GEMM (MODE 1): one complex Nν3 x Nν3 x Nν3 product per (channel,
     representative (P, Ω) block); complex MAC = 8 real flops.  On the FP64 CUDA-core kernel
-    (k_bse_K3_gemm) the FP64 pipe bounds it; on the digit-sliced tensor-core kernel (k_bse_K3_oz,
+    (k_bse_K3_gemm) the FP64 pipe bounds it; blocks up to Nν3 = 32 run on warp-level digit products
+    (k_bse_K3_mma), for which `frac` is a rate in FP64 terms over the FP64 FMA rate and `mma_frac` the
+    issued MMA work over the measured bf16 peak; on the digit-sliced tensor-core kernel (k_bse_K3_oz,
     the default above Nν3 = 32) the 16-bit MMA work is compared with the measured bf16 peak
     and its FP64-equivalent rate with the FP64 pipe; `flops_per_launch` counts the 36 MMAs of an
     8-digit product that the kernel issues."""
@@ -259,7 +262,11 @@ def k3_gemm_roofline(S, stages, cfg_name):
     # blocks of Nν3 ≤ 32: the warp-level digit-sliced kernel, whose FP64-equivalent rate may pass the FP64 pipe's
     kernel = ("k_bse_K3_mma<1> (fused K3 BSE, FP64 by digit slicing on mma.sync; FP64-equivalent rate)" if N <= 32
               else "k_bse_K3_gemm<1,32,cplx> (fused K3 BSE, FP64)")
+    # 37 MMAs of 16 x 8 x 16 (36 digit pairs, one of magnitudes) per 8 x 8 complex output tile and 8 ω
+    mma_flops = 3 * nb * 37 * (2 * 16 * 8 * 16) * math.ceil(N / 8) ** 3 if N <= 32 else 0
     return {"bound": "fp64", "kernel": kernel, "achieved": achieved,
+            "mma_flops_per_launch": mma_flops,
+            "mma_frac": mma_flops / (ms * 1e-3) / 1e12 / peaks.get("bf16_tflops", 1900.0),
             "peak": fp64_peak, "unit": "TFLOP/s", "frac": achieved / fp64_peak,
             "peak_source": "measured: the library's FP64 FMA calibration kernel on this GPU (fdga_query fp64_gflops)",
             "traffic": traffic, "algorithmic_bytes": byts, "hbm_achieved_gbs": byts / (ms * 1e-3) / 1e9,

@@ -30,12 +30,13 @@
 // top digits in magnitude, sees whether any ω has a nonzero top digit on both sides, that is Σ |A||M| ≥ 2^-14 of
 // the bounds and an error below 2 Nν3 2^-45 of it; an output without one is summed again in FP64, one ω per lane
 // (A falling by 2^39 as M rises, Nν3 = 24: error 8e-9 of the largest output -> an FP64 sum's).  That is so in the
-// adjoint and below Nν3 = 32, where FP64 sums ran before.  Few outputs of the lattice workloads' maps are summed
-// again (Hubbard 8x8, nK3 = (8, 12): K3 38 us with and without; the residual call 584 -> 587 us), in the adjoint a
-// sixth of one product's, far from the diagonal (700 -> 733 us; one output at a time, each part by itself, 776).
-// At Nν3 = 32 the map's digits stand by themselves, as did the form before with bounds of whole blocks: a SIAM has outputs far from the
-// diagonal that would be summed again (K3 18 -> 43 us).  A row of A or a column of M that holds an infinity or NaN,
-// or products near the end of the normal range, are summed in FP64 everywhere.
+// adjoint and below Nν3 = 32, where FP64 sums ran before.  Of the lattice workloads' maps 0.2 % of the outputs are
+// summed again (Hubbard 8x8, nK3 = (8, 12): K3 38 us with and without; the residual call 584 -> 587 us), of the
+// adjoint's 3.6 %, far from the diagonal of one product (700 -> 719 us; one output at a time, each part by itself,
+// 776).  At Nν3 = 32 the map's digits stand by themselves, as did the form before with bounds of whole blocks: a
+// SIAM has outputs far from the diagonal that would be summed again (K3 18 -> 43 us one at a time).  A row of A or a
+// column of M that holds an infinity or NaN, or products near the end of the normal range, are summed in FP64
+// everywhere.
 //
 // What bounds it: forming M (8 to 14 FP64 operations per entry) and the latency of one pass load ->
 // digits -> MMA -> store; a CTA of NC·NC warps (NC = ⌈Nν3/8⌉) does one block, each warp staging one 8 x 8

@@ -540,8 +540,9 @@ __global__ void k_build_cache(VertPT<S> Fin, Caches C, const int* blocks, int nb
 // Stage times on GB300 without -> with the table (its launch is in the cache stage), caches / left K2 /
 // K2 in us: Hubbard 8x8, nK3 = (8, 12) 45 / 48 / 112 -> 29 / 29 / 62; 8x8, nK3 = (20, 40) 915 / 386 / 829
 // -> 273 / 151 / 375; 5x5 without groups, nK3 = (5, 7) 23 / 69 / 141 -> 23 / 37 / 68.  The local solver
-// (one momentum) has nothing to share and evaluates in place, as does a Vertex-valued F0, whose own
-// channel depends on P.
+// has one momentum: its K2, left K2 and caches evaluate in place (the same Γ three times, not over every P).  So do
+// a Vertex-valued F0, whose own channel depends on P, and boxes whose table would outgrow the state
+// (gamma_table_kept).
 // ---------------------------------------------------------------------------------------------
 template <class S>
 __global__ void __launch_bounds__(256) k_gamma_table(VertPT<S> F, S* tp, S* tt, S* ta, const int* oms, Dims d) {
