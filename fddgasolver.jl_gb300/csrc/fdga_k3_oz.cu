@@ -444,10 +444,9 @@ static size_t k3_oz_smem(const Dims& d, int ns) {
 // stages, 407 with three; L_K3 stage 392 and 331).  Above Nν3 = 80 three stages leave room for one CTA on an SM only.
 template <int MAXC, int NS>
 static cudaError_t prepare_oz(const Dims& d) {
-    static SmemRecord set0, set1, set3;
-    cudaError_t e = raise_smem_limit(k_bse_K3_oz<0, MAXC, NS>, set0, k3_oz_smem(d, NS), 0);
-    if (e == cudaSuccess) e = raise_smem_limit(k_bse_K3_oz<1, MAXC, 2>, set1, k3_oz_smem(d, 2), 0);
-    if (e == cudaSuccess) e = raise_smem_limit(k_bse_K3_oz<3, MAXC, 2>, set3, k3_oz_smem(d, 2), 0);
+    cudaError_t e = raise_smem_limit_of<k_bse_K3_oz<0, MAXC, NS>>(k3_oz_smem(d, NS), 0);
+    if (e == cudaSuccess) e = raise_smem_limit_of<k_bse_K3_oz<1, MAXC, 2>>(k3_oz_smem(d, 2), 0);
+    if (e == cudaSuccess) e = raise_smem_limit_of<k_bse_K3_oz<3, MAXC, 2>>(k3_oz_smem(d, 2), 0);
     return e;
 }
 cudaError_t prepare_bse_K3_oz(const Dims& d) {

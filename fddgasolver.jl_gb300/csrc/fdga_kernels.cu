@@ -2149,13 +2149,9 @@ template <class S, bool TAN>
 static size_t k2_row_smem(const Dims& d) {
     return (size_t)(TAN ? 2 : 1) * 2 * k2_table_half(d) * sizeof(S);
 }
-// Limit of a row kernel.  The kernel is the template argument, so that each instantiation has a record of its own
-// (forms of one kernel share a function type).
 template <auto Kernel>
 static cudaError_t row_smem_limit(size_t smem) {
-    if (smem > 227 * 1024) return cudaErrorInvalidValue;
-    static SmemRecord raised;
-    return raise_smem_limit(Kernel, raised, smem);
+    return smem > 227 * 1024 ? cudaErrorInvalidValue : raise_smem_limit_of<Kernel>(smem);
 }
 static unsigned warp_grid(const ChanWork& cw, int nch) {
     int mx = 0;

@@ -34,6 +34,13 @@ inline cudaError_t raise_smem_limit(K kernel, SmemRecord& raised, size_t bytes, 
     if (e == cudaSuccess) raised.bytes[dev] = bytes;
     return e;
 }
+// The same with the record kept here, one per kernel: the kernel is the template argument, so that forms of one
+// kernel, which share a function type, and callers that prepare one kernel in several places have the right one.
+template <auto Kernel>
+inline cudaError_t raise_smem_limit_of(size_t bytes, size_t floor = 48 * 1024) {
+    static SmemRecord raised;
+    return raise_smem_limit(Kernel, raised, bytes, floor);
+}
 
 // The (P, Ω) rows of the bubbles that any work item reads: with symmetry groups the K1, K2 and K3
 // representatives and blocks lie in an irreducible wedge of the momenta and one sign of Ω, so the other

@@ -71,6 +71,21 @@ def test_a_tangent_leaves_the_map_its_limit():
     _matches_oracle(dict(SIAM, nK1=1700, nK2=(1, 1700)))
 
 
+def test_a_narrower_k3_box_leaves_a_wider_one_its_limit():
+    """K3 contractions at Nν3 = 96 after a handle with Nν3 = 72 was prepared: they share kernels."""
+    cfg = lambda n: dict(SIAM, nG=n + 4, nK1=n + 2, nK2=(3, n), nK3=(2, n), mPi_factor=2)  # noqa: E731
+    S = make_gpu(cfg(48), True)
+    x = _start(S, 9)
+    make_gpu(cfg(36), True).close()
+    y = S.fixed_point(x) + x
+    S.unflatten(x)
+    S.frule(x)
+    S.set_option("k3_fp64_tensor_cores", 0)
+    ref = S.fixed_point(x) + x
+    S.close()
+    assert blockwise_rel_err(cfg(48), y, ref) < 1e-12  # as test_k3_fp64_tensor_cores.py
+
+
 def test_adjoint_of_wide_fermionic_rows():
     """K2 rows of up to 2 nK2ν = 2560 items: past the 2458 whose values fit 48 KB (nonlocal, trivial groups)."""
     _transposed(dict(HUB, nK1=1280, nK2=(1, 1280)), sym=False)
