@@ -52,9 +52,10 @@ def test_nan_after_the_first_step(sym, L, mem):
 @pytest.mark.parametrize("solver", ["solve", "solve_mixed", "solve_newton"])
 def test_nan_in_the_start(sym, cfg, solver):
     S = make_gpu(cfg, sym)
-    for first in (0, -1):  # one element, and every element
-        x = S.flatten()
-        x[first:] = np.nan
-        S.unflatten(x if first == 0 else np.where(np.arange(x.size) == x.size // 2, np.nan, 0j))
+    every = np.full(S.state_len, np.nan + 0j)
+    one = np.zeros(S.state_len, dtype=complex)
+    one[S.state_len // 2] = np.nan
+    for x in (every, one):
+        S.unflatten(x)
         assert _rc(lambda: getattr(S, solver)(maxiter=4, tol=1e-4)) == NONFINITE
     S.close()
